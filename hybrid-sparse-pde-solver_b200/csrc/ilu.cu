@@ -2,27 +2,28 @@
 //
 // Setup, all on the device:
 //   1. level sets of the lower and upper triangles: level(i) = 1 + max level(j) over the
-//      strictly lower (upper) columns j of row i.  Computed by a frontier sweep (Kahn's
-//      order) inside ONE cooperative kernel, one grid barrier per level; the frontiers,
-//      laid end to end, are the rows grouped by level.
+//      strictly lower (upper) columns j of row i.  k_levels_chain takes the rows in index
+//      order, a block of them at a time, with a prefix scan for the dependence of each row
+//      on its neighbour; patterns it does not suit go to a frontier sweep (k_levels, Kahn's
+//      order, one grid barrier per level).
 //   2. the factorisation, level by level of the lower sets: each row runs the reference's
 //      IKJ elimination (same pivots, same update order, separate multiply and subtract),
-//      so the factor values equal the reference's lu_val_ bit for bit.
+//      so the factor values equal the reference's lu_val_ bit for bit.  Short rows run from
+//      an operation list worked out beforehand for all rows at once (k_ilu_factor_ops).
 //   3. level-ordered copies of L (strictly lower part) and U (diagonal + upper part), so
 //      the rows of one level are contiguous in memory.
-// Apply: forward then backward sweep, one level per barrier.  With at most a few
-// thousand rows per level (the natural-order 5-point grids here have <= n_side rows per
-// level) one thread block per sweep is fastest: a block barrier costs far less than a
-// grid barrier, and rows of the next level are prefetched while the current one waits.
-// The arithmetic per row is the reference's (ilu.cpp:230-237, :249-260), so z is
-// bit-identical to ILUPreconditioner::apply.
+// Apply: forward then backward sweep, each by the kernel its triangle's shape asks for
+// (TriMode below).  The arithmetic per row is the reference's (ilu.cpp:230-237, :249-260),
+// so z is bit-identical to ILUPreconditioner::apply.
 #include <cooperative_groups.h>
 
 #include <climits>
 #include <cmath>
+#include <tuple>
 #include <cstring>
 
 #include "ilu_row.cuh"
+#include "ilu_sweep.cuh"
 #include "krylov.cuh"
 #include "scan.cuh"
 
@@ -33,6 +34,7 @@ namespace hamlss {
 namespace {
 
 constexpr double kEps = 2.220446049250313e-16;
+constexpr int kIluLptrSmem = 4096;       // level pointers kept in shared memory by the one-block kernels
 
 // ---------------------------------------------------------------- pattern helpers
 // dpos[i] = position of a_ii in row i (-1 if absent); lcnt[i] = # columns < i;
@@ -63,30 +65,6 @@ __global__ void k_col_fill(int n, const int* __restrict__ rp, const int* __restr
                            int* fillpos, int* trow) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         for (int k = rp[i]; k < rp[i + 1]; ++k) trow[atomicAdd(&fillpos[ci[k]], 1)] = i;
-}
-
-// single-block exclusive scan of n+1 ints in place (setup only)
-__global__ void k_scan_inplace(int* a, int count) {
-    __shared__ int carry;
-    __shared__ int buf[1024];
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int base = 0; base < count; base += 1024) {
-        int i = base + threadIdx.x;
-        int v = i < count ? a[i] : 0;
-        buf[threadIdx.x] = v;
-        __syncthreads();
-        for (int o = 1; o < 1024; o <<= 1) {
-            int t = threadIdx.x >= o ? buf[threadIdx.x - o] : 0;
-            __syncthreads();
-            buf[threadIdx.x] += t;
-            __syncthreads();
-        }
-        if (i < count) a[i] = buf[threadIdx.x] - v + carry;   // exclusive
-        __syncthreads();
-        if (threadIdx.x == 1023) carry += buf[1023];
-        __syncthreads();
-    }
 }
 
 // Kahn frontier sweep over the dependency DAG of one triangle.
@@ -128,6 +106,346 @@ __global__ void k_levels(int n, const int* __restrict__ trp, const int* __restri
     }
 }
 
+// Level sets of a pattern in index order, one block per triangle (block 0 the lower one,
+// block 1 the upper one, whose rows are taken backwards).  kChainRows rows are decided at a
+// time: a row's dependencies in earlier rows are final and read from a shared-memory ring of
+// the last kChainRing levels (older ones from global memory), and its dependence on the row
+// just before it -- the west or east neighbour of a grid row -- is a max-plus recurrence
+// level[m] = max(level[m-1] + 1, c[m]) solved by a segmented prefix maximum.  Dependencies
+// inside the block of rows that are not that neighbour are met by repeating the pass until
+// nothing changes (levels only grow, so it ends): a natural-order grid takes a pass for each
+// grid row that the block spans.  The next block's pattern is loaded meanwhile.  A pattern
+// that needs many passes is given up (nlev[tri] = -1) and left to k_levels.
+// 512^2 grid, both triangles at once: 0.99 ms; 13.0 ms one after the other with one grid
+// barrier a level.
+constexpr int kChainRows = 1024;
+constexpr int kChainRing = 16384;
+constexpr int kChainPre = 6;             // dependencies of a row held in registers
+constexpr int kChainPasses = 24;         // passes a block allowed on average before giving up
+
+__global__ void __launch_bounds__(kChainRows)
+k_levels_chain(int n, const int* __restrict__ rp, const int* __restrict__ ci, int* levelL, int* levelU,
+               int* nlev) {
+    extern __shared__ int chain_ring[];
+    __shared__ int w_val[32];
+    __shared__ unsigned w_all;           // bit w: every row of warp w continues the chain
+    __shared__ int s_max;
+    const bool lower = blockIdx.x == 0;
+    int* level = lower ? levelL : levelU;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int chunks = (n + kChainRows - 1) / kChainRows;
+    if (tid == 0) s_max = 0;
+    // row m of the sweep is row i of the matrix
+    auto mirror = [&](int i) { return lower ? i : n - 1 - i; };
+    int rs1 = 0, re1 = 0;                // row bounds of the next block's row
+    int dep[kChainPre];                  // this block's row: its first dependencies (sweep index)
+    int rs = 0, re = 0;
+    auto bounds = [&](int c, int& s, int& e) {
+        const int m = c * kChainRows + tid;
+        s = e = 0;
+        if (c < chunks && m < n) {
+            const int i = mirror(m);
+            s = __ldg(&rp[i]);
+            e = __ldg(&rp[i + 1]);
+        }
+    };
+    auto deps = [&](int m, int s, int e, int (&d)[kChainPre]) {
+        int col[kChainPre];
+#pragma unroll
+        for (int k = 0; k < kChainPre; ++k) col[k] = s + k < e ? __ldg(&ci[s + k]) : -1;
+#pragma unroll
+        for (int k = 0; k < kChainPre; ++k) {
+            const int dm = s + k < e ? mirror(col[k]) : m;
+            d[k] = dm < m ? dm : -1;     // -1: the diagonal or the other triangle
+        }
+    };
+    bounds(0, rs, re);
+    deps(tid, rs, re, dep);
+    bounds(1, rs1, re1);
+    int sweeps = 0, top = -1;
+    for (int c = 0; c < chunks; ++c) {
+        const int m0 = c * kChainRows, m = m0 + tid;
+        int ndep[kChainPre];
+        deps(m + kChainRows, rs1, re1, ndep);           // next block, in flight meanwhile
+        int rs2, re2;
+        bounds(c + 2, rs2, re2);
+        // dependencies in earlier blocks: final; the neighbour: a chain link; others: `more`
+        int ext = 0;
+        bool chain = false, more = false;
+        auto take = [&](int dm) {
+            if (dm < 0) return;
+            if (dm >= m0) {
+                if (dm == m - 1) chain = true;
+                else more = true;
+            } else {
+                const int lv = m0 - dm <= kChainRing - kChainRows ? chain_ring[dm & (kChainRing - 1)]
+                                                                  : level[mirror(dm)];
+                ext = max(ext, lv + 1);
+            }
+        };
+        if (m < n) {
+#pragma unroll
+            for (int k = 0; k < kChainPre; ++k) take(dep[k]);
+            for (int k = rs + kChainPre; k < re; ++k) {
+                const int dm = mirror(__ldg(&ci[k]));
+                take(dm < m ? dm : -1);
+            }
+        }
+        // first row of a warp's chain ends at the warp boundary: carried across by the warps
+        const unsigned cont = __ballot_sync(0xffffffffu, chain);
+        int mine = -1;
+        bool again = false, first = true;
+        do {
+            int v = ext;
+            if (more && mine >= 0) {
+                auto inner = [&](int dm) {
+                    if (dm >= m0 && dm != m - 1) v = max(v, chain_ring[dm & (kChainRing - 1)] + 1);
+                };
+#pragma unroll
+                for (int k = 0; k < kChainPre; ++k) inner(dep[k]);
+                for (int k = rs + kChainPre; k < re; ++k) {
+                    const int dm = mirror(__ldg(&ci[k]));
+                    if (dm < m) inner(dm);
+                }
+            }
+            // segmented prefix maximum of v - lane over chain links, inside the warp
+            int u = v - lane;
+            const unsigned below = ~cont & (0xffffffffu >> (31 - lane));      // segment starts at or before lane
+            const int seg = below ? 31 - __clz(below) : 0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, u, o);
+                if (lane - o >= seg) u = max(u, t);
+            }
+            int lv = u + lane;
+            if (lane == 31) w_val[wid] = lv;
+            if (wid == 0 && lane == 0) w_all = 0;
+            __syncthreads();
+            // across warps: warp w's incoming value is the last level of warp w - 1
+            if (lane == 0 && cont == 0xffffffffu) atomicOr(&w_all, 1u << wid);
+            __syncthreads();
+            {
+                // value entering this warp: max over warps w' < wid reached through fully
+                // linked warps, of w_val[w'] + 32 (wid - 1 - w')
+                const unsigned full = w_all;
+                int in = -0x40000000;
+                if (lane < wid) {
+                    // every warp strictly between lane and wid is fully linked
+                    const unsigned need = (wid - lane > 1) ? (((1u << (wid - lane - 1)) - 1u) << (lane + 1)) : 0u;
+                    if ((full & need) == need) in = w_val[lane] + 32 * (wid - 1 - lane);
+                }
+                in = __reduce_max_sync(0xffffffffu, in);
+                // it reaches the lanes linked to the warp's first one
+                const bool linked = wid > 0 && (cont & (0xffffffffu >> (31 - lane))) == (0xffffffffu >> (31 - lane));
+                if (linked) lv = max(lv, in + 1 + lane);
+            }
+            const bool changed = lv != mine;
+            mine = lv;
+            if (m < n) chain_ring[m & (kChainRing - 1)] = lv;
+            // repeated only where some row has other dependencies inside the block
+            again = __syncthreads_or(first ? more : changed);
+            first = false;
+            ++sweeps;
+        } while (again && sweeps <= kChainPasses * (c + 16));
+        if (sweeps > kChainPasses * (c + 16)) {
+            if (tid == 0) nlev[blockIdx.x] = -1;
+            return;
+        }
+        if (m < n) {
+            level[mirror(m)] = mine;
+            top = max(top, mine);
+        }
+        rs = rs1; re = re1; rs1 = rs2; re1 = re2;
+#pragma unroll
+        for (int k = 0; k < kChainPre; ++k) dep[k] = ndep[k];
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (lane == 0) atomicMax(&s_max, top);
+    __syncthreads();
+    if (tid == 0) nlev[blockIdx.x] = s_max + 1;
+}
+
+__global__ void k_level_hist(int n, const int* __restrict__ level, int* cnt) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) atomicAdd(&cnt[level[i]], 1);
+}
+
+__global__ void k_level_place(int n, const int* __restrict__ level, int* fill, int* order) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        order[atomicAdd(&fill[level[i]], 1)] = i;
+}
+
+// Rows of each level by index (a level of at most kSortRows rows; wider ones keep the order
+// they were placed in, which no result depends on): neighbouring rows of a level then read
+// neighbouring entries.  *maxw receives the widest level.
+constexpr int kSortRows = 2048;
+__global__ void __launch_bounds__(256)
+k_level_sort(int nlev, const int* __restrict__ lptr, int* order, int* maxw) {
+    __shared__ int key[kSortRows];
+    for (int l = blockIdx.x; l < nlev; l += gridDim.x) {
+        const int b = lptr[l], w = lptr[l + 1] - b;
+        if (threadIdx.x == 0) atomicMax(maxw, w);
+        if (w <= 1 || w > kSortRows) continue;
+        int N = 2;
+        while (N < w) N <<= 1;
+        for (int t = threadIdx.x; t < N; t += blockDim.x) key[t] = t < w ? order[b + t] : INT_MAX;
+        __syncthreads();
+        for (int kk = 2; kk <= N; kk <<= 1)
+            for (int jj = kk >> 1; jj > 0; jj >>= 1) {
+                for (int t = threadIdx.x; t < N; t += blockDim.x) {
+                    const int p = t ^ jj;
+                    if (p > t) {
+                        const int x = key[t], y = key[p];
+                        if ((x > y) == ((t & kk) == 0)) { key[t] = y; key[p] = x; }
+                    }
+                }
+                __syncthreads();
+            }
+        for (int t = threadIdx.x; t < w; t += blockDim.x) order[b + t] = key[t];
+        __syncthreads();
+    }
+}
+
+__global__ void k_invert(int n, const int* __restrict__ order, int* pos) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) pos[order[t]] = t;
+}
+
+// out[t] = pos[order[t]]
+__global__ void k_compose(int n, const int* __restrict__ order, const int* __restrict__ pos, int* out) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) out[t] = pos[order[t]];
+}
+
+// Operation lists of the elimination (ilu_row) for rows of at most kOpsRow entries, in
+// position order of the lower levels: x = target entry of the row (+ kOpsDiv for the
+// division by pivot y), y = factor entry it reads (-1: the pivot is absent).
+constexpr int kOpsRow = 8;
+constexpr int kOpsDiv = 16;
+template <bool FILL>
+__global__ void k_ilu_ops(int n, const int* __restrict__ order, const int* __restrict__ rp,
+                          const int* __restrict__ ci, const int* __restrict__ dpos, int* optr, int2* ops,
+                          int4* info) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        const int i = order[t], s = rp[i], e = rp[i + 1];
+        int o = FILL ? optr[t] : 0;
+        for (int p = s; p < e; ++p) {
+            const int k = ci[p];
+            if (k >= i) break;
+            if (FILL) ops[o] = make_int2(kOpsDiv | (p - s), dpos[k]);
+            ++o;
+            int pi = p + 1;
+            for (int q = rp[k]; q < rp[k + 1]; ++q) {
+                const int j = ci[q];
+                if (j <= k) continue;
+                while (pi < e && ci[pi] < j) ++pi;
+                if (pi == e) break;
+                if (ci[pi] == j) {
+                    if (FILL) ops[o] = make_int2(pi - s, q);
+                    ++o;
+                }
+            }
+        }
+        if (FILL) info[t] = make_int4(s, e - s, optr[t], o - optr[t]);
+        else optr[t] = o;
+    }
+}
+
+// The elimination from operation lists, one block, a barrier per level.  A row's place and
+// lengths (info) are fetched two levels ahead, its values and first operations one level
+// ahead, so behind the barrier there is one round of loads -- the factor entries of earlier
+// rows that its operations read, all issued together -- and the row's arithmetic.  Walking
+// the pattern inside the level (k_ilu_factor_block) costs a chain of dependent loads
+// instead: 7.1 us a level on the 512^2 grid, 2.2 us here.
+constexpr int kOpsPre = 6;
+constexpr int kOpsThreads = 512;
+constexpr size_t kOpsSmem = (size_t)kOpsRow * kOpsThreads * sizeof(double);
+
+struct OpsRow {
+    int4 info;               // first entry, entries, first operation, operations; y = 0: no row
+    int2 op[kOpsPre];
+    double own[kOpsRow];
+};
+
+__global__ void __launch_bounds__(kOpsThreads, 1)
+k_ilu_factor_ops(int nlev, const int* __restrict__ lptr_g, const int4* __restrict__ info,
+                 const int* __restrict__ ci, const int2* __restrict__ ops, double* lu, int* status) {
+    extern __shared__ double ops_own[];                  // the current row's values, [entry][thread]
+    __shared__ int s_lptr[kIluLptrSmem];
+    const int tid = threadIdx.x;
+    constexpr int NT = kOpsThreads;
+    for (int l = tid; l <= nlev && l < kIluLptrSmem; l += NT) s_lptr[l] = lptr_g[l];
+    __syncthreads();
+    auto lptr = [&](int l) { return l < kIluLptrSmem ? s_lptr[l] : __ldg(&lptr_g[l]); };
+    auto own = [&](int k) -> double& { return ops_own[k * NT + tid]; };
+    auto where = [&](int l) {
+        if (l < nlev) {
+            const int t = lptr(l) + tid;
+            if (t < lptr(l + 1)) return __ldg(&info[t]);
+        }
+        return make_int4(0, 0, 0, 0);
+    };
+    auto fetch = [&](OpsRow& q, int4 in) {
+        q.info = in;
+#pragma unroll
+        for (int k = 0; k < kOpsRow; ++k)
+            if (k < in.y) q.own[k] = lu[in.x + k];       // changed only in the row's own level
+#pragma unroll
+        for (int k = 0; k < kOpsPre; ++k)
+            if (k < in.w) q.op[k] = __ldg(&ops[in.z + k]);
+    };
+    auto run = [&](const OpsRow& q) {
+        double val[kOpsPre];
+#pragma unroll
+        for (int k = 0; k < kOpsPre; ++k)
+            if (k < q.info.w) val[k] = q.op[k].y >= 0 ? lu[q.op[k].y] : 0.0;
+#pragma unroll
+        for (int k = 0; k < kOpsRow; ++k)
+            if (k < q.info.y) own(k) = q.own[k];
+        double lik = 0.0;
+        bool bad = false;
+        auto step = [&](int2 op, double x) {
+            const int a = op.x & (kOpsDiv - 1);
+            if (op.x & kOpsDiv) {
+                if (fabs(x) < kEps) {                    // the pivot of this entry's column
+                    atomicMin(status, ci[q.info.x + a]);
+                    bad = true;
+                    return;
+                }
+                lik = own(a) / x;
+                own(a) = lik;
+            } else {
+                own(a) = __dsub_rn(own(a), __dmul_rn(lik, x));
+            }
+        };
+#pragma unroll
+        for (int k = 0; k < kOpsPre; ++k)
+            if (k < q.info.w && !bad) step(q.op[k], val[k]);
+        for (int k = kOpsPre; k < q.info.w && !bad; ++k) {
+            const int2 op = __ldg(&ops[q.info.z + k]);
+            step(op, op.y >= 0 ? lu[op.y] : 0.0);
+        }
+        for (int k = 0; k < q.info.y; ++k) lu[q.info.x + k] = own(k);
+    };
+    OpsRow cur;
+    fetch(cur, where(0));
+    int4 in1 = where(1);
+    for (int l = 0; l < nlev; ++l) {
+        OpsRow nxt;
+        fetch(nxt, in1);                                 // level l + 1
+        const int4 in2 = where(l + 2);
+        if (cur.info.y > 0) {
+            run(cur);
+            const int e = lptr(l + 1);
+            for (int t = lptr(l) + tid + NT; t < e; t += NT) {   // rows beyond the block width
+                OpsRow more;
+                fetch(more, __ldg(&info[t]));
+                run(more);
+            }
+        }
+        __syncthreads();
+        cur = nxt;
+        in1 = in2;
+    }
+}
+
 __global__ void k_ilu_factor_block(int nlev, const int* __restrict__ order, const int* __restrict__ lptr,
                                    const int* __restrict__ rp, const int* __restrict__ ci,
                                    const int* __restrict__ dpos, double* lu, int* status) {
@@ -150,6 +468,36 @@ __global__ void k_ilu_factor_grid(int nlev, const int* __restrict__ order, const
     }
 }
 
+// facts[0..2] = the longest row's entries below, above the diagonal, and in all;
+// facts[5..6] = the entries below and above the diagonal
+__global__ void k_max_counts(int n, const int* __restrict__ lcnt, const int* __restrict__ ucnt,
+                             const int* __restrict__ rp, int* facts) {
+    int a = 0, b = 0, c = 0, nl = 0, nu = 0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        nl += lcnt[i];
+        nu += ucnt[i];
+        a = max(a, lcnt[i]);
+        b = max(b, ucnt[i]);
+        c = max(c, rp[i + 1] - rp[i]);
+    }
+    a = __reduce_max_sync(0xffffffffu, a);
+    b = __reduce_max_sync(0xffffffffu, b);
+    c = __reduce_max_sync(0xffffffffu, c);
+    nl = __reduce_add_sync(0xffffffffu, nl);
+    nu = __reduce_add_sync(0xffffffffu, nu);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&facts[5], nl);
+        atomicAdd(&facts[6], nu);
+        atomicMax(&facts[0], a);
+        atomicMax(&facts[1], b);
+        atomicMax(&facts[2], c);
+    }
+}
+
+__global__ void k_to_float(int n, const double* __restrict__ a, float* __restrict__ b) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) b[i] = (float)a[i];
+}
+
 // Level-ordered L / U copies.  Lrp/Urp are prefix sums of per-slot counts in order.
 __global__ void k_perm_counts(int n, const int* __restrict__ order, const int* __restrict__ cnt,
                               int* out) {
@@ -157,10 +505,9 @@ __global__ void k_perm_counts(int n, const int* __restrict__ order, const int* _
         out[t] = cnt[order[t]];
 }
 
-template <typename T>
 __global__ void k_fill_L(int n, const int* __restrict__ order, const int* __restrict__ rp,
                          const int* __restrict__ ci, const double* __restrict__ lu,
-                         const int* __restrict__ Lrp, int* Lci, T* Lv) {
+                         const int* __restrict__ Lrp, int* Lci, double* Lv) {
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         const int i = order[t];
         int o = Lrp[t];
@@ -168,7 +515,7 @@ __global__ void k_fill_L(int n, const int* __restrict__ order, const int* __rest
             const int j = ci[p];
             if (j >= i) break;
             Lci[o] = j;
-            Lv[o] = (T)lu[p];
+            Lv[o] = lu[p];
             ++o;
         }
     }
@@ -176,10 +523,9 @@ __global__ void k_fill_L(int n, const int* __restrict__ order, const int* __rest
 
 // U copy: the diagonal (1.0 if absent, as backward_sub assumes, ilu.cpp:251) then the
 // upper entries.  bad[0] receives the smallest row with |u_ii| < eps (ilu.cpp:257-259).
-template <typename T>
 __global__ void k_fill_U(int n, const int* __restrict__ order, const int* __restrict__ rp,
                          const int* __restrict__ ci, const double* __restrict__ lu,
-                         const int* __restrict__ Urp, int* Uci, T* Uv, T* Ud, int* bad) {
+                         const int* __restrict__ Urp, int* Uci, double* Uv, double* Ud, int* bad) {
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         const int i = order[t];
         int o = Urp[t];
@@ -187,42 +533,32 @@ __global__ void k_fill_U(int n, const int* __restrict__ order, const int* __rest
         for (int p = rp[i]; p < rp[i + 1]; ++p) {
             const int j = ci[p];
             if (j == i) { d = lu[p]; continue; }
-            if (j > i) { Uci[o] = j; Uv[o] = (T)lu[p]; ++o; }
+            if (j > i) {
+                Uci[o] = j;
+                Uv[o] = lu[p];
+                ++o;
+            }
         }
-        Ud[t] = (T)d;
-        if (bad && fabs(d) < kEps) atomicMin(bad, i);
+        Ud[t] = d;
+        if (fabs(d) < kEps) atomicMin(bad, i);
     }
 }
 
 // ------------------------------------------------------------------------ sweeps
+// A triangle in position order with the matrix's own columns and vectors in row order.
 template <typename T>
-struct IluLevels {
-    int n, nlevL, nlevU;
-    const int* ordL;
-    const int* lptrL;
-    const int* Lrp;
-    const int* Lci;
-    const T* Lv;
-    const int* ordU;
-    const int* lptrU;
-    const int* Urp;
-    const int* Uci;
-    const T* Uv;
-    const T* Ud;
+struct TriRows {
+    int n, nlev;
+    const int* ord;
+    const int* lptr;
+    const int* rp;
+    const int* ci;
+    const T* v;
+    const T* dg;
 };
 
-template <typename T>
-__device__ __forceinline__ T sub_mul(T s, T a, T b);
-template <>
-__device__ __forceinline__ double sub_mul<double>(double s, double a, double b) {
-    return __dsub_rn(s, __dmul_rn(a, b));
-}
-template <>
-__device__ __forceinline__ float sub_mul<float>(float s, float a, float b) {
-    return __fsub_rn(s, __fmul_rn(a, b));
-}
-
-// L y = r (unit lower, forward_sub) then U z = y (backward_sub); one block.
+// One sweep by one block for triangles with long rows (ilu_sweep.cuh's rings hold steps of
+// short rows).
 //
 // One level's critical path is a barrier plus the loads of the vector being solved for; the
 // rest of a row's inputs (its index, right-hand side, columns, values, diagonal) do not
@@ -234,7 +570,6 @@ __device__ __forceinline__ float sub_mul<float>(float s, float a, float b) {
 // back with ordinary loads after the barrier (block scope), and every row sums in its
 // stored (ascending column) order, so results are bit-identical to the plain loop.
 constexpr int kIluPre = 4;
-constexpr int kIluLptrSmem = 4096;
 
 template <typename T>
 struct IluStage2 {
@@ -245,12 +580,20 @@ struct IluStage2 {
 };
 
 template <typename T, bool DIV, int NT>
-__device__ __forceinline__ void ilu_sweep_block(int nlev, const int* __restrict__ lptr_g, const int* s_lptr,
-                                                const int* __restrict__ ord, const int* __restrict__ rp,
-                                                const int* __restrict__ ci, const T* __restrict__ v,
-                                                const T* __restrict__ dg, const T* rhs, T* out) {
-    auto lptr = [&](int l) { return l < kIluLptrSmem ? s_lptr[l] : __ldg(&lptr_g[l]); };
+__global__ void __launch_bounds__(NT)
+k_tri_block(TriRows<T> F, const T* rhs, T* out, const int* gate) {
+    __shared__ int s_lptr[kIluLptrSmem];
+    if (gate && *(volatile const int*)gate) return;
     const int tid = threadIdx.x;
+    for (int l = tid; l <= F.nlev && l < kIluLptrSmem; l += NT) s_lptr[l] = F.lptr[l];
+    __syncthreads();
+    const int nlev = F.nlev;
+    const int* __restrict__ ord = F.ord;
+    const int* __restrict__ rp = F.rp;
+    const int* __restrict__ ci = F.ci;
+    const T* __restrict__ v = F.v;
+    const T* __restrict__ dg = F.dg;
+    auto lptr = [&](int l) { return l < kIluLptrSmem ? s_lptr[l] : __ldg(&F.lptr[l]); };
     // stage 1 of a level: (t, i, o0, cnt) of this thread's first row, t = -1 if none
     auto stage1 = [&](int l, int& t, int& i, int& o0, int& cnt) {
         t = -1;
@@ -317,44 +660,21 @@ __device__ __forceinline__ void ilu_sweep_block(int nlev, const int* __restrict_
     }
 }
 
-template <typename T, int NT>
-__global__ void __launch_bounds__(NT)
-k_ilu_apply_block(IluLevels<T> F, const T* __restrict__ r, T* y, T* z, const int* gate) {
-    __shared__ int s_lptr[kIluLptrSmem];
-    if (gate && *(volatile const int*)gate) return;
-    for (int l = threadIdx.x; l <= F.nlevL && l < kIluLptrSmem; l += NT) s_lptr[l] = F.lptrL[l];
-    __syncthreads();
-    ilu_sweep_block<T, false, NT>(F.nlevL, F.lptrL, s_lptr, F.ordL, F.Lrp, F.Lci, F.Lv, nullptr, r, y);
-    for (int l = threadIdx.x; l <= F.nlevU && l < kIluLptrSmem; l += NT) s_lptr[l] = F.lptrU[l];
-    __syncthreads();
-    ilu_sweep_block<T, true, NT>(F.nlevU, F.lptrU, s_lptr, F.ordU, F.Urp, F.Uci, F.Uv, F.Ud, y, z);
-}
-
-// Same sweeps with the whole grid (cooperative launch) for matrices with wide levels.
-template <typename T>
-__global__ void k_ilu_apply_grid(IluLevels<T> F, const T* __restrict__ r, T* y, T* z, const int* gate) {
+// The same sweep with the whole grid (cooperative launch) for triangles with wide levels.
+template <typename T, bool DIV>
+__global__ void k_tri_grid(TriRows<T> F, const T* __restrict__ rhs, T* out, const int* gate) {
     if (gate && *(volatile const int*)gate) return;
     cg::grid_group grid = cg::this_grid();
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-    for (int l = 0; l < F.nlevL; ++l) {
-        const int b = F.lptrL[l], e = F.lptrL[l + 1];
+    for (int l = 0; l < F.nlev; ++l) {
+        const int b = F.lptr[l], e = F.lptr[l + 1];
         for (int t = b + tid; t < e; t += nth) {
-            const int i = F.ordL[t];
-            T s = r[i];
-            for (int o = F.Lrp[t]; o < F.Lrp[t + 1]; ++o) s = sub_mul<T>(s, F.Lv[o], __ldcg(&y[F.Lci[o]]));
-            y[i] = s;
+            const int i = F.ord[t];
+            T s = rhs[i];
+            for (int o = F.rp[t]; o < F.rp[t + 1]; ++o) s = sub_mul<T>(s, F.v[o], __ldcg(&out[F.ci[o]]));
+            out[i] = DIV ? s / F.dg[t] : s;
         }
-        grid.sync();
-    }
-    for (int l = 0; l < F.nlevU; ++l) {
-        const int b = F.lptrU[l], e = F.lptrU[l + 1];
-        for (int t = b + tid; t < e; t += nth) {
-            const int i = F.ordU[t];
-            T s = __ldcg(&y[i]);
-            for (int o = F.Urp[t]; o < F.Urp[t + 1]; ++o) s = sub_mul<T>(s, F.Uv[o], __ldcg(&z[F.Uci[o]]));
-            z[i] = s / F.Ud[t];
-        }
-        grid.sync();
+        if (l + 1 < F.nlev) grid.sync();
     }
 }
 
@@ -744,15 +1064,49 @@ int coop_blocks(Ctx& ctx, K kernel, int threads) {
 }
 
 template <typename K, typename... Args>
-void coop_launch(Ctx& ctx, K kernel, int blocks, int threads, Args... args) {
+void coop_launch(cudaStream_t s, K kernel, int blocks, int threads, Args... args) {
     void* ptrs[] = {(void*)&args...};
-    HAMLSS_CUDA(cudaLaunchCooperativeKernel((const void*)kernel, dim3(blocks), dim3(threads), ptrs, 0,
-                                            ctx.lane.stream));
+    HAMLSS_CUDA(cudaLaunchCooperativeKernel((const void*)kernel, dim3(blocks), dim3(threads), ptrs, 0, s));
 }
 
 }  // namespace
 
 // ---------------------------------------------------------------------- the object
+// Kernel of a triangle's sweep, by its shape:
+//   GRID   more than 4,096 rows a level on average: the whole grid, a grid barrier (~2 us) a
+//          level; one block would spend longer than that on a level's rows
+//   RING   otherwise, rows of at most 16 entries: one block, shared-memory rings
+//          (0.15 to 0.37 us a level)
+//   BLOCK  otherwise (a step of the ring kernel would hold too few rows): one block reading
+//          through the caches (~1.1 us a level)
+enum class TriMode { RING, BLOCK, GRID };
+constexpr int kTriMaxRow = 16;
+
+struct Triangle {
+    int nlev = 0, nnz = 0, max_row = 0, max_width = 0;
+    TriMode mode = TriMode::GRID;
+    DBuf<int> ord, lptr, level;
+    DBuf<int> code, code32, sptr;        // RING: entry codes, step bounds (ilu_sweep.cuh)
+    int nsteps = 0, step_rows = 0;
+    bool far = false;                    // RING: entries beyond the ring
+    DBuf<int> rp, ci;                    // the other modes: row bounds and columns
+    DBuf<double> v, dg;                  // in position order (RING: [row][place], with reciprocals)
+    DBuf<float> v32, dg32;
+};
+
+// (values, diagonals, codes) of a triangle by value type
+inline std::tuple<DBuf<double>&, DBuf<double>&, DBuf<int>&> tri_bufs(Triangle& t, double) { return {t.v, t.dg, t.code}; }
+inline std::tuple<DBuf<float>&, DBuf<float>&, DBuf<int>&> tri_bufs(Triangle& t, float) { return {t.v32, t.dg32, t.code32}; }
+
+// Calls f(std::integral_constant<int, K>) with the entry places a RING triangle's rows get.
+template <typename F>
+void tri_places(const Triangle& t, F&& f) {
+    if (t.max_row <= 2) f(std::integral_constant<int, 2>{});
+    else if (t.max_row <= 4) f(std::integral_constant<int, 4>{});
+    else if (t.max_row <= 8) f(std::integral_constant<int, 8>{});
+    else f(std::integral_constant<int, 16>{});
+}
+
 struct IluPrec : Prec {
     hamlss_mat* A = nullptr;
     // pattern of the factor: A's for ILU(0); the factor's own (frp, fci) for ILUT
@@ -760,25 +1114,14 @@ struct IluPrec : Prec {
     const int* pci = nullptr;
     int pnnz = 0;
     DBuf<int> frp, fci;
-    DBuf<int> dpos, lcnt, ucnt, trp, trow, indeg, cnt, levelL, levelU, nlev;
-    DBuf<int> ordL, lptrL, ordU, lptrU, Lrp, Lci, Urp, Uci;
-    DBuf<double> lu, Lv, Uv, Ud;
-    DBuf<float> Lv32, Uv32, Ud32;
-    DBuf<double> y;
-    DBuf<float> y32;
-    int nlevL = 0, nlevU = 0, nnzL = 0, nnzU = 0;
+    DBuf<int> dpos;
+    DBuf<double> lu;
+    Triangle L, U;
+    DBuf<int> u_from_l;          // position in L of the row at each position of U (both RING)
+    DBuf<double> y, s1, s2;      // y between the sweeps in row order; vectors in position order
+    DBuf<float> y32, s132, s232;
     int bad_diag_row = -1;       // backward_sub would throw on this row
     bool f32_ready = false;
-    bool wide = false;
-
-    IluLevels<double> view64() const {
-        return IluLevels<double>{n, nlevL, nlevU, ordL.p, lptrL.p, Lrp.p, Lci.p, Lv.p,
-                                 ordU.p, lptrU.p, Urp.p, Uci.p, Uv.p, Ud.p};
-    }
-    IluLevels<float> view32() const {
-        return IluLevels<float>{n, nlevL, nlevU, ordL.p, lptrL.p, Lrp.p, Lci.p, Lv32.p,
-                                ordU.p, lptrU.p, Urp.p, Uci.p, Uv32.p, Ud32.p};
-    }
 
     void check_apply() const {
         if (bad_diag_row >= 0)
@@ -786,41 +1129,136 @@ struct IluPrec : Prec {
                  "ILU backward sub: near-zero U diagonal at row " + std::to_string(bad_diag_row));
     }
 
-    template <typename T>
-    void run(Ctx& ctx, const Lane& L, const IluLevels<T>& F, const T* r, T* yb, T* z, const int* gate) {
-        check_apply();
-        if (!n) return;
-        ProfScope ps(L, "ilu_sweep", (double)sizeof(T) * (nnzL + nnzU + 4.0 * n) + 4.0 * (nnzL + nnzU + 4.0 * n));
-        if (!wide) {
-            k_ilu_apply_block<T, 1024><<<1, 1024, 0, L.stream>>>(F, r, yb, z, gate);
+    template <typename T, bool GATHER>
+    void permute(Ctx& ctx, const Lane& ln, const int* idx, const T* in, T* out, const int* gate) {
+        k_permute<T, GATHER><<<std::max(1, std::min(ceil_div(n, 256), ctx.sm_count * 8)), 256, 0, ln.stream>>>(
+            n, idx, in, out, gate);
+        HAMLSS_LAUNCH_CHECK();
+    }
+
+    // a RING triangle's rows; `pos`: position of each row; `bad`: see k_fill_U
+    template <typename T, bool DIV>
+    void pack(Ctx& ctx, Triangle& t, const int* pos, int* far, int* bad) {
+        tri_places(t, [&](auto k) {
+            constexpr int K = decltype(k)::value;
+            constexpr int RB = TriShape<T, K, DIV>::RB;
+            const int rows = ceil_div(n, RB) * RB;
+            auto [tv, tdg, tcode] = tri_bufs(t, T(0));
+            tv.ensure((size_t)rows * K);
+            tcode.ensure((size_t)rows * K);
+            if (DIV) tdg.ensure((size_t)rows * 2);
+            k_tri_pack<T, K, DIV><<<std::min(ceil_div(rows, 256), ctx.sm_count * 8), 256, 0, ctx.lane.stream>>>(
+                n, t.ord.p, t.level.p, t.lptr.p, pos, prp, pci, lu.p, tv.p, tcode.p, tdg.p, far, bad);
+        });
+        HAMLSS_LAUNCH_CHECK();
+    }
+
+    // a RING triangle's steps, which fit the kernels of both value types
+    template <bool DIV>
+    void make_steps(Ctx& ctx, Triangle& t) {
+        tri_places(t, [&](auto k) {
+            constexpr int K = decltype(k)::value;
+            t.step_rows = std::min(TriShape<double, K, DIV>::max_rows, TriShape<float, K, DIV>::max_rows);
+        });
+        t.step_rows = std::max(32, std::min((t.max_width + 31) / 32 * 32, t.step_rows));
+        cudaStream_t s = ctx.lane.stream;
+        const int g = std::max(1, std::min(ceil_div(t.nlev + 1, 256), ctx.sm_count * 8));
+        DBuf<int> first(t.nlev + 1);
+        HAMLSS_CUDA(cudaMemsetAsync(first.p + t.nlev, 0, sizeof(int), s));
+        k_step_count<<<g, 256, 0, s>>>(t.nlev, t.lptr.p, t.step_rows, first.p);
+        HAMLSS_LAUNCH_CHECK();
+        t.nsteps = (int)exclusive_scan(ctx, first.p, t.nlev + 1);
+        t.sptr.ensure(t.nsteps + 1);
+        k_step_fill<<<g, 256, 0, s>>>(t.nlev, t.lptr.p, t.step_rows, first.p, t.sptr.p);
+        HAMLSS_LAUNCH_CHECK();
+    }
+
+    // rhs -> out: in position order for RING, in row order for the others
+    template <typename T, bool DIV>
+    void sweep(Ctx& ctx, const Lane& ln, Triangle& t, const T* rhs, T* out, const int* gate) {
+        auto [tv, tdg, tcode] = tri_bufs(t, T(0));
+        if (t.mode == TriMode::RING) {
+            const TriView<T> F{n, t.nsteps, t.sptr.p, tv.p, tcode.p, tdg.p};
+            tri_places(t, [&](auto k) {
+                constexpr int K = decltype(k)::value;
+                using S = TriShape<T, K, DIV>;
+                auto kern = t.far ? k_tri_sweep<T, K, DIV, true> : k_tri_sweep<T, K, DIV, false>;
+                static DeviceOnce raised;
+                raised(ctx.device, [] {
+                    for (auto f : {k_tri_sweep<T, K, DIV, true>, k_tri_sweep<T, K, DIV, false>})
+                        HAMLSS_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                        (int)S::smem_bytes));
+                });
+                kern<<<1, t.step_rows + 32, S::smem_bytes, ln.stream>>>(F, rhs, out, gate, ln.err.p);
+            });
+            HAMLSS_LAUNCH_CHECK();
+            return;
+        }
+        TriRows<T> F{n, t.nlev, t.ord.p, t.lptr.p, t.rp.p, t.ci.p, tv.p, tdg.p};
+        if (t.mode == TriMode::BLOCK) {
+            k_tri_block<T, DIV, 1024><<<1, 1024, 0, ln.stream>>>(F, rhs, out, gate);
             HAMLSS_LAUNCH_CHECK();
         } else {
-            static const int blocks = coop_blocks(ctx, k_ilu_apply_grid<T>, 256);
-            void* args[] = {(void*)&F, (void*)&r, (void*)&yb, (void*)&z, (void*)&gate};
-            HAMLSS_CUDA(cudaLaunchCooperativeKernel((const void*)k_ilu_apply_grid<T>, dim3(blocks),
-                                                    dim3(256), args, 0, L.stream));
+            static const int blocks = coop_blocks(ctx, k_tri_grid<T, DIV>, 256);
+            coop_launch(ln.stream, k_tri_grid<T, DIV>, blocks, 256, F, rhs, out, gate);
         }
     }
 
-    void apply(Ctx& ctx, const Lane& L, const double* r, double* z, const int* gate) override {
-        run<double>(ctx, L, view64(), r, y.p, z, gate);
+    template <typename T>
+    void run(Ctx& ctx, const Lane& ln, const T* r, T* yb, T* a, T* c, T* z, const int* gate) {
+        check_apply();
+        if (!n) return;
+        ProfScope ps(ln, "ilu_sweep", (double)sizeof(T) * (L.nnz + U.nnz + 4.0 * n) + 4.0 * (L.nnz + U.nnz + 4.0 * n));
+        const bool lring = L.mode == TriMode::RING, uring = U.mode == TriMode::RING;
+        if (lring) {
+            permute<T, true>(ctx, ln, L.ord.p, r, a, gate);
+            sweep<T, false>(ctx, ln, L, a, c, gate);
+            if (!uring) permute<T, false>(ctx, ln, L.ord.p, c, yb, gate);
+        } else {
+            sweep<T, false>(ctx, ln, L, r, yb, gate);
+        }
+        if (uring) {
+            permute<T, true>(ctx, ln, lring ? u_from_l.p : U.ord.p, lring ? c : yb, a, gate);
+            sweep<T, true>(ctx, ln, U, a, c, gate);
+            permute<T, false>(ctx, ln, U.ord.p, c, z, gate);
+        } else {
+            sweep<T, true>(ctx, ln, U, yb, z, gate);
+        }
+    }
+
+    void apply(Ctx& ctx, const Lane& ln, const double* r, double* z, const int* gate) override {
+        run<double>(ctx, ln, r, y.p, s1.p, s2.p, z, gate);
     }
     void prepare32(Ctx& ctx) override {
         if (f32_ready) return;
         cudaStream_t s = ctx.lane.stream;
-        Lv32.ensure(nnzL); Uv32.ensure(nnzU); Ud32.ensure(n); y32.ensure(n);
-        int g = std::max(1, std::min(ceil_div(n, 256), ctx.sm_count * 8));
         if (n) {
-            k_fill_L<float><<<g, 256, 0, s>>>(n, ordL.p, prp, pci, lu.p, Lrp.p, Lci.p, Lv32.p);
-            k_fill_U<float><<<g, 256, 0, s>>>(n, ordU.p, prp, pci, lu.p, Urp.p, Uci.p, Uv32.p,
-                                              Ud32.p, nullptr);
-            HAMLSS_LAUNCH_CHECK();
+            const int g = std::max(1, std::min(ceil_div(n, 256), ctx.sm_count * 8));
+            for (Triangle* t : {&L, &U}) {
+                if (t->mode == TriMode::RING) {
+                    DBuf<int> pos(n), far(1);          // (t->far is known)
+                    k_invert<<<g, 256, 0, s>>>(n, t->ord.p, pos.p);
+                    if (t == &L) pack<float, false>(ctx, L, pos.p, far.p, nullptr);
+                    else pack<float, true>(ctx, U, pos.p, far.p, nullptr);
+                    continue;
+                }
+                t->v32.ensure(std::max(t->nnz, 1));
+                if (t->nnz) k_to_float<<<std::min(ceil_div(t->nnz, 256), ctx.sm_count * 8), 256, 0, s>>>(t->nnz, t->v.p, t->v32.p);
+                if (t == &U) {
+                    t->dg32.ensure(n);
+                    k_to_float<<<g, 256, 0, s>>>(n, t->dg.p, t->dg32.p);
+                }
+                HAMLSS_LAUNCH_CHECK();
+            }
         }
+        y32.ensure(std::max(n, 1));
+        s132.ensure(std::max(n, 1));
+        s232.ensure(std::max(n, 1));
         f32_ready = true;
     }
-    void apply32(Ctx& ctx, const Lane& L, const float* r, float* z, const int* gate) override {
+    void apply32(Ctx& ctx, const Lane& ln, const float* r, float* z, const int* gate) override {
         prepare32(ctx);
-        run<float>(ctx, L, view32(), r, y32.p, z, gate);
+        run<float>(ctx, ln, r, y32.p, s132.p, s232.p, z, gate);
     }
     bool has32() const override { return true; }
 };
@@ -942,58 +1380,89 @@ void finish_ilu(Ctx& ctx, IluPrec* P, bool factorise) {
     const int g = std::max(1, std::min(ceil_div(n, 256), ctx.sm_count * 8));
     const int* rp = P->prp;
     const int* ci = P->pci;
-    P->y.ensure(n);
     if (n == 0) return;
-    P->dpos.ensure(n); P->lcnt.ensure(n); P->ucnt.ensure(n);
-    k_row_info<<<g, 256, 0, s>>>(n, rp, ci, P->dpos.p, P->lcnt.p, P->ucnt.p);
+    P->y.ensure(n); P->s1.ensure(n); P->s2.ensure(n);
+    Triangle* tri[2] = {&P->L, &P->U};
+    DBuf<int> lcnt(n), ucnt(n);
+    // longest rows (L, U, whole), level counts (2), entries (2), widest levels (2),
+    // entries beyond the ring (2)
+    DBuf<int> facts(11);
+    facts.zero(s);
+    P->dpos.ensure(n);
+    k_row_info<<<g, 256, 0, s>>>(n, rp, ci, P->dpos.p, lcnt.p, ucnt.p);
+    k_max_counts<<<g, 256, 0, s>>>(n, lcnt.p, ucnt.p, rp, facts.p);
     HAMLSS_LAUNCH_CHECK();
-    // transpose of the pattern: counts per column, exclusive scan over n+1 slots
-    P->trp.ensure(n + 1); P->trow.ensure(nnz);
-    HAMLSS_CUDA(cudaMemsetAsync(P->trp.p, 0, sizeof(int) * (n + 1), s));
-    k_col_count<<<g, 256, 0, s>>>(n, rp, ci, P->trp.p);
-    k_scan_inplace<<<1, 1024, 0, s>>>(P->trp.p, n + 1);
-    HAMLSS_LAUNCH_CHECK();
-    {
-        DBuf<int> fill(n);
-        HAMLSS_CUDA(cudaMemcpyAsync(fill.p, P->trp.p, sizeof(int) * n, cudaMemcpyDeviceToDevice, s));
-        k_col_fill<<<g, 256, 0, s>>>(n, rp, ci, fill.p, P->trow.p);
-        HAMLSS_LAUNCH_CHECK();
-        HAMLSS_CUDA(cudaStreamSynchronize(s));
-    }
     // level sets
-    P->indeg.ensure(n); P->cnt.ensure(n + 2); P->nlev.ensure(2);
-    P->ordL.ensure(n); P->lptrL.ensure(n + 1); P->levelL.ensure(n);
-    P->ordU.ensure(n); P->lptrU.ensure(n + 1); P->levelU.ensure(n);
+    P->L.level.ensure(n);
+    P->U.level.ensure(n);
     {
-        int lb = coop_blocks(ctx, k_levels<true>, 256);
-        HAMLSS_CUDA(cudaMemcpyAsync(P->indeg.p, P->lcnt.p, sizeof(int) * n, cudaMemcpyDeviceToDevice, s));
-        HAMLSS_CUDA(cudaMemsetAsync(P->cnt.p, 0, sizeof(int) * (n + 2), s));
-        coop_launch(ctx, k_levels<true>, lb, 256, n, (const int*)P->trp.p, (const int*)P->trow.p,
-                    P->indeg.p, P->ordL.p, P->lptrL.p, P->cnt.p, P->levelL.p, P->nlev.p);
-        HAMLSS_CUDA(cudaMemcpyAsync(P->indeg.p, P->ucnt.p, sizeof(int) * n, cudaMemcpyDeviceToDevice, s));
-        HAMLSS_CUDA(cudaMemsetAsync(P->cnt.p, 0, sizeof(int) * (n + 2), s));
-        coop_launch(ctx, k_levels<false>, lb, 256, n, (const int*)P->trp.p, (const int*)P->trow.p,
-                    P->indeg.p, P->ordU.p, P->lptrU.p, P->cnt.p, P->levelU.p, P->nlev.p + 1);
-        int hl[2];
-        HAMLSS_CUDA(cudaMemcpyAsync(hl, P->nlev.p, sizeof(hl), cudaMemcpyDeviceToHost, s));
-        HAMLSS_CUDA(cudaStreamSynchronize(s));
-        P->nlevL = hl[0];
-        P->nlevU = hl[1];
+        static DeviceOnce raised;
+        raised(ctx.device, [] {
+            HAMLSS_CUDA(cudaFuncSetAttribute(k_levels_chain, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            kChainRing * (int)sizeof(int)));
+        });
+        k_levels_chain<<<2, kChainRows, kChainRing * sizeof(int), s>>>(n, rp, ci, P->L.level.p, P->U.level.p,
+                                                                      facts.p + 3);
+        HAMLSS_LAUNCH_CHECK();
     }
-    P->wide = (double)n / std::max(1, std::min(P->nlevL, P->nlevU)) > 4096.0;
+    int hf[7];
+    facts.download(hf, 7, s);
+    HAMLSS_CUDA(cudaStreamSynchronize(s));
+    const int max_row = hf[2];
+    P->L.max_row = hf[0];
+    P->U.max_row = hf[1];
+    if (hf[3] < 0 || hf[4] < 0) {
+        DBuf<int> dpos;
+        pattern_levels(ctx, n, nnz, rp, ci, dpos, P->L.level, P->U.level, &hf[3], &hf[4]);
+    }
+    P->L.nlev = hf[3];
+    P->U.nlev = hf[4];
+    // rows grouped by level, in index order inside a level
+    DBuf<int> pos[2];
+    for (int k = 0; k < 2; ++k) {
+        Triangle& t = *tri[k];
+        t.lptr.ensure(t.nlev + 1);
+        HAMLSS_CUDA(cudaMemsetAsync(t.lptr.p, 0, sizeof(int) * (t.nlev + 1), s));
+        k_level_hist<<<g, 256, 0, s>>>(n, t.level.p, t.lptr.p);
+        HAMLSS_LAUNCH_CHECK();
+        exclusive_scan(ctx, t.lptr.p, t.nlev + 1);
+        DBuf<int> fill(t.nlev + 1);
+        HAMLSS_CUDA(cudaMemcpyAsync(fill.p, t.lptr.p, sizeof(int) * (t.nlev + 1), cudaMemcpyDeviceToDevice, s));
+        t.ord.ensure(n);
+        pos[k].ensure(n);
+        k_level_place<<<g, 256, 0, s>>>(n, t.level.p, fill.p, t.ord.p);
+        k_level_sort<<<std::min(t.nlev, ctx.sm_count * 8), 256, 0, s>>>(t.nlev, t.lptr.p, t.ord.p, facts.p + 7 + k);
+        k_invert<<<g, 256, 0, s>>>(n, t.ord.p, pos[k].p);
+        HAMLSS_LAUNCH_CHECK();
+        const bool wide = (double)n / t.nlev > 4096.0;
+        t.mode = wide ? TriMode::GRID : t.max_row <= kTriMaxRow ? TriMode::RING : TriMode::BLOCK;
+    }
     // factorisation (ILU(0); ILUT arrives factored)
     if (factorise) {
         DBuf<int> status(1);
         int init = 0x7fffffff;
         status.upload(&init, 1, s);
-        if (!P->wide) {
-            k_ilu_factor_block<<<1, 1024, 0, s>>>(P->nlevL, P->ordL.p, P->lptrL.p, rp, ci, P->dpos.p,
-                                                 P->lu.p, status.p);
+        if (P->L.mode == TriMode::GRID) {
+            int fb = coop_blocks(ctx, k_ilu_factor_grid, 256);
+            coop_launch(s, k_ilu_factor_grid, fb, 256, P->L.nlev, (const int*)P->L.ord.p,
+                        (const int*)P->L.lptr.p, rp, ci, (const int*)P->dpos.p, P->lu.p, status.p);
+        } else if (max_row <= kOpsRow) {
+            DBuf<int> optr(n + 1);
+            HAMLSS_CUDA(cudaMemsetAsync(optr.p + n, 0, sizeof(int), s));
+            k_ilu_ops<false><<<g, 256, 0, s>>>(n, P->L.ord.p, rp, ci, P->dpos.p, optr.p, nullptr, nullptr);
+            HAMLSS_LAUNCH_CHECK();
+            const long long total = exclusive_scan(ctx, optr.p, n + 1);
+            if (total > INT_MAX) fail(HAMLSS_ERR_NOMEM, "ILU(0): elimination list exceeds 2^31 operations");
+            DBuf<int2> ops(std::max<long long>(total, 1));
+            DBuf<int4> info(n);
+            k_ilu_ops<true><<<g, 256, 0, s>>>(n, P->L.ord.p, rp, ci, P->dpos.p, optr.p, ops.p, info.p);
+            k_ilu_factor_ops<<<1, kOpsThreads, kOpsSmem, s>>>(P->L.nlev, P->L.lptr.p, info.p, ci, ops.p, P->lu.p,
+                                                             status.p);
             HAMLSS_LAUNCH_CHECK();
         } else {
-            int fb = coop_blocks(ctx, k_ilu_factor_grid, 256);
-            coop_launch(ctx, k_ilu_factor_grid, fb, 256, P->nlevL, (const int*)P->ordL.p,
-                        (const int*)P->lptrL.p, rp, ci, (const int*)P->dpos.p, P->lu.p, status.p);
+            k_ilu_factor_block<<<1, 1024, 0, s>>>(P->L.nlev, P->L.ord.p, P->L.lptr.p, rp, ci, P->dpos.p,
+                                                 P->lu.p, status.p);
+            HAMLSS_LAUNCH_CHECK();
         }
         int h = 0;
         status.download(&h, 1, s);
@@ -1002,37 +1471,48 @@ void finish_ilu(Ctx& ctx, IluPrec* P, bool factorise) {
             fail(HAMLSS_ERR_ZERO_PIVOT, "ILU(0): near-zero pivot at row " + std::to_string(h));
     }
     // level-ordered factor copies
-    {
-        P->Lrp.ensure(n + 1); P->Urp.ensure(n + 1);
-        HAMLSS_CUDA(cudaMemsetAsync(P->Lrp.p, 0, sizeof(int) * (n + 1), s));
-        HAMLSS_CUDA(cudaMemsetAsync(P->Urp.p, 0, sizeof(int) * (n + 1), s));
-        k_perm_counts<<<g, 256, 0, s>>>(n, P->ordL.p, P->lcnt.p, P->Lrp.p);
-        k_perm_counts<<<g, 256, 0, s>>>(n, P->ordU.p, P->ucnt.p, P->Urp.p);
-        k_scan_inplace<<<1, 1024, 0, s>>>(P->Lrp.p, n + 1);
-        k_scan_inplace<<<1, 1024, 0, s>>>(P->Urp.p, n + 1);
+    DBuf<int> bad(1);
+    int init = 0x7fffffff;
+    bad.upload(&init, 1, s);
+    for (int k = 0; k < 2; ++k) {
+        Triangle& t = *tri[k];
+        t.nnz = hf[5 + k];
+        if (t.mode == TriMode::RING) {
+            if (k == 0) P->pack<double, false>(ctx, t, pos[0].p, facts.p + 9, nullptr);
+            else P->pack<double, true>(ctx, t, pos[1].p, facts.p + 10, bad.p);
+            continue;
+        }
+        t.rp.ensure(n + 1);
+        HAMLSS_CUDA(cudaMemsetAsync(t.rp.p + n, 0, sizeof(int), s));
+        k_perm_counts<<<g, 256, 0, s>>>(n, t.ord.p, k == 0 ? lcnt.p : ucnt.p, t.rp.p);
         HAMLSS_LAUNCH_CHECK();
-        int h[2];
-        HAMLSS_CUDA(cudaMemcpyAsync(&h[0], P->Lrp.p + n, sizeof(int), cudaMemcpyDeviceToHost, s));
-        HAMLSS_CUDA(cudaMemcpyAsync(&h[1], P->Urp.p + n, sizeof(int), cudaMemcpyDeviceToHost, s));
-        HAMLSS_CUDA(cudaStreamSynchronize(s));
-        P->nnzL = h[0];
-        P->nnzU = h[1];
-        P->Lci.ensure(P->nnzL); P->Lv.ensure(P->nnzL);
-        P->Uci.ensure(P->nnzU); P->Uv.ensure(P->nnzU); P->Ud.ensure(n);
-        DBuf<int> bad(1);
-        int init = 0x7fffffff;
-        bad.upload(&init, 1, s);
-        k_fill_L<double><<<g, 256, 0, s>>>(n, P->ordL.p, rp, ci, P->lu.p, P->Lrp.p, P->Lci.p, P->Lv.p);
-        k_fill_U<double><<<g, 256, 0, s>>>(n, P->ordU.p, rp, ci, P->lu.p, P->Urp.p, P->Uci.p, P->Uv.p,
-                                           P->Ud.p, bad.p);
+        exclusive_scan(ctx, t.rp.p, n + 1);
+        t.ci.ensure(std::max(t.nnz, 1));
+        t.v.ensure(std::max(t.nnz, 1));
+        if (k == 0) {
+            k_fill_L<<<g, 256, 0, s>>>(n, t.ord.p, rp, ci, P->lu.p, t.rp.p, t.ci.p, t.v.p);
+        } else {
+            t.dg.ensure(n);
+            k_fill_U<<<g, 256, 0, s>>>(n, t.ord.p, rp, ci, P->lu.p, t.rp.p, t.ci.p, t.v.p, t.dg.p, bad.p);
+        }
         HAMLSS_LAUNCH_CHECK();
-        int hb = 0;
-        bad.download(&hb, 1, s);
-        HAMLSS_CUDA(cudaStreamSynchronize(s));
-        P->bad_diag_row = hb != 0x7fffffff ? hb : -1;
     }
-    P->trow.release();
-    P->indeg.release();
+    if (P->L.mode == TriMode::RING && P->U.mode == TriMode::RING) {
+        P->u_from_l.ensure(n);
+        k_compose<<<g, 256, 0, s>>>(n, P->U.ord.p, pos[0].p, P->u_from_l.p);
+        HAMLSS_LAUNCH_CHECK();
+    }
+    int hb = 0, hw[4];
+    bad.download(&hb, 1, s);
+    HAMLSS_CUDA(cudaMemcpyAsync(hw, facts.p + 7, sizeof(hw), cudaMemcpyDeviceToHost, s));
+    HAMLSS_CUDA(cudaStreamSynchronize(s));
+    P->bad_diag_row = hb != 0x7fffffff ? hb : -1;
+    P->L.max_width = hw[0];
+    P->U.max_width = hw[1];
+    P->L.far = hw[2] != 0;
+    P->U.far = hw[3] != 0;
+    if (P->L.mode == TriMode::RING) P->make_steps<false>(ctx, P->L);
+    if (P->U.mode == TriMode::RING) P->make_steps<true>(ctx, P->U);
 }
 }  // namespace
 
@@ -1062,11 +1542,11 @@ void pattern_levels(Ctx& ctx, int n, int nnz, const int* rp, const int* ci, DBuf
     const int lb = coop_blocks(ctx, k_levels<true>, 256);
     HAMLSS_CUDA(cudaMemcpyAsync(indeg.p, lcnt.p, sizeof(int) * n, cudaMemcpyDeviceToDevice, s));
     HAMLSS_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int) * (n + 2), s));
-    coop_launch(ctx, k_levels<true>, lb, 256, n, (const int*)trp.p, (const int*)trow.p, indeg.p,
+    coop_launch(s, k_levels<true>, lb, 256, n, (const int*)trp.p, (const int*)trow.p, indeg.p,
                 order.p, lptr.p, cnt.p, levelL.p, nl.p);
     HAMLSS_CUDA(cudaMemcpyAsync(indeg.p, ucnt.p, sizeof(int) * n, cudaMemcpyDeviceToDevice, s));
     HAMLSS_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int) * (n + 2), s));
-    coop_launch(ctx, k_levels<false>, lb, 256, n, (const int*)trp.p, (const int*)trow.p, indeg.p,
+    coop_launch(s, k_levels<false>, lb, 256, n, (const int*)trp.p, (const int*)trow.p, indeg.p,
                 order.p, lptr.p, cnt.p, levelU.p, nl.p + 1);
     int h[2];
     HAMLSS_CUDA(cudaMemcpyAsync(h, nl.p, sizeof(h), cudaMemcpyDeviceToHost, s));
@@ -1098,9 +1578,9 @@ int ilu_factor_csr(const Prec* M, int* nnz, int* rp, int* ci, double* v, cudaStr
 int ilu_copy_levels(const Prec* M, int which, int* level, int* nlev, cudaStream_t s) {
     auto* P = dynamic_cast<const IluPrec*>(M);
     if (!P) return HAMLSS_ERR_INVALID;
-    if (P->n) (which == 0 ? P->levelL : P->levelU).download(level, P->n, s);
+    if (P->n) (which == 0 ? P->L : P->U).level.download(level, P->n, s);
     HAMLSS_CUDA(cudaStreamSynchronize(s));
-    *nlev = which == 0 ? P->nlevL : P->nlevU;
+    *nlev = which == 0 ? P->L.nlev : P->U.nlev;
     return HAMLSS_OK;
 }
 
