@@ -5,6 +5,8 @@
 //   K1  q = A p with p = z + beta p_old formed on the fly (p written for own rows), p.q
 //   K2  x += alpha p, r -= alpha q, ||r||^2 (and for Jacobi z = D^-1 r, r.z)
 //   [M^-1 r -> z ; K3 r.z]                      (non-Jacobi preconditioners)
+// Where the matrix fits the chip's shared memory, K1 and K2 of many trips are one
+// persistent launch instead (cg_persist.cuh; Jacobi or no preconditioner).
 // All scalars (rho, alpha, beta, rel) live in device memory; the last block of each
 // reduction computes them, including the reference's convergence test on the recursive
 // residual (:133, :143) and both breakdown restarts (:109-120, :157-167).  The host only
@@ -15,6 +17,7 @@
 #include <cstring>
 #include <vector>
 
+#include "cg_persist.cuh"
 #include "krylov.cuh"
 
 namespace hamlss {
@@ -278,6 +281,102 @@ void precond_apply<float>(Ctx& ctx, Prec* M, const float* r, float* z, const int
     M->apply32(ctx, ctx.lane, r, z, gate);
 }
 
+// ------------------------------------------------------------- persistent iteration
+constexpr int kPersistTrips = 4096;       // trips a launch (state is saved between launches)
+
+// finalisers of k_cg_persist: K1's and K2's (without a preconditioner z = r, so K3's sum
+// arrives with K2's)
+template <bool JAC>
+struct FinTrip {
+    __device__ void pq(CgState* s, const double (&t)[1]) const { FinPQ{s}(t); }
+    __device__ void upd(CgState* s, const double (&t)[2]) const {
+        FinUpd<JAC>{s}(t);
+        if (!JAC && !s->halt) rho_step(s, t[1], 3);
+    }
+    __device__ bool leave(const CgState*) const { return false; }
+    __device__ void timeout(CgState* s) const { s->status = ST_MAXIT; s->halt = 1; }
+};
+
+template <typename T, bool JAC, int SLOTS, bool CLUSTER, typename Fin>
+void launch_persist_t(Ctx& ctx, const PersistArgs<T>& a, CgState* s, int blocks, size_t smem, const Fin& fin) {
+    auto kern = k_cg_persist<T, JAC, SLOTS, CLUSTER, CgState, Fin>;
+    static DeviceOnce raised;
+    raised(ctx.device, [&] {
+        HAMLSS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPersistSmem));
+        if (CLUSTER) HAMLSS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    });
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(a.rows <= 256 ? 256 : 512);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx.lane.stream;
+    cudaLaunchAttribute at{};
+    if (CLUSTER) {
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = blocks;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    } else {
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+    }
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    HAMLSS_CUDA(cudaLaunchKernelEx(&cfg, kern, a, s, fin));
+}
+
+template <typename T, bool JAC, bool CLUSTER, typename Fin>
+void launch_persist_c(Ctx& ctx, const PersistArgs<T>& a, CgState* s, int blocks, size_t smem, const Fin& fin) {
+    if (a.rows <= 512) launch_persist_t<T, JAC, 1, CLUSTER>(ctx, a, s, blocks, smem, fin);
+    else if (a.rows <= 1024) launch_persist_t<T, JAC, 2, CLUSTER>(ctx, a, s, blocks, smem, fin);
+    else if (a.rows <= 2048) launch_persist_t<T, JAC, 4, CLUSTER>(ctx, a, s, blocks, smem, fin);
+    else launch_persist_t<T, JAC, kPersistMaxSlots, CLUSTER>(ctx, a, s, blocks, smem, fin);
+}
+
+// Whether the persistent iteration holds the matrix: its rows a block, their entries and the
+// columns they span fit a block's shared memory (about 500,000 rows of a 5-point grid in
+// FP64).  Otherwise the matrix streams from memory trip by trip and two launches a trip do.
+template <typename T>
+bool persist_fits(Ctx& ctx, hamlss_mat* A) {
+    ensure_persist_plan(ctx, A);
+    return A->persist_rows > 0 && persist_smem<T>(A->persist_entries, A->persist_window) <= kPersistSmem;
+}
+
+// One launch of up to kPersistTrips trips from the state in memory (r, p, x and the
+// scalars) back to it.
+template <typename T, bool JAC, typename Fin>
+void launch_persist(Ctx& ctx, hamlss_mat* A, const Csr<T>& Ad, T* x, T* r, T* p, T* z, const T* dinv, CgState* s,
+                    const Fin& fin) {
+    Lane& L = ctx.lane;
+    constexpr size_t words = 4 * kPersistMaxBlocks;
+    if (!L.sums.p) {
+        AllocScope outside(nullptr);                      // lives as long as the lane
+        L.sums.alloc(words + 1);
+    }
+    if (!A->persist_cluster) HAMLSS_CUDA(cudaMemsetAsync(L.sums.p + words, 0, sizeof(double), L.stream));
+    PersistArgs<T> a;
+    a.n = Ad.n;
+    a.rows = A->persist_rows;
+    a.max_trips = kPersistTrips;
+    a.rp = Ad.rp;
+    a.ci = Ad.ci;
+    a.v = Ad.v;
+    a.x = x;
+    a.r = r;
+    a.p = p;
+    a.z = z;
+    a.dinv = dinv;
+    a.words = L.sums.p;
+    a.count = reinterpret_cast<unsigned*>(L.sums.p + words);
+    a.err = L.err.p;
+    a.window = A->persist_window;
+    a.entries = A->persist_entries;
+    const int blocks = ceil_div(Ad.n, a.rows);
+    const size_t smem = persist_smem<T>(a.entries, a.window);
+    ProfScope ps(L, "cg_trips", csr_bytes(Ad) + (JAC ? 7.0 : 6.0) * sizeof(T) * Ad.n);
+    if (A->persist_cluster) launch_persist_c<T, JAC, true>(ctx, a, s, blocks, smem, fin);
+    else launch_persist_c<T, JAC, false>(ctx, a, s, blocks, smem, fin);
+}
+
 template <typename T, bool JAC>
 SolveResult cg_impl(Ctx& ctx, hamlss_mat* A, Prec* M, const T* b, T* x, double tol,
                     int max_iter, int check_every, Workspace& ws, const LadderCfg* lad) {
@@ -322,6 +421,8 @@ SolveResult cg_impl(Ctx& ctx, hamlss_mat* A, Prec* M, const T* b, T* x, double t
     restart_seq(true);
     poll(h);
     const bool run = !h.halt && max_iter > 0;
+    const bool persist = run && (JAC || !M) && persist_fits<T>(ctx, A);
+    T* zp = persist ? wvec<T>(ws, 1, n) : nullptr;     // z of the persistent iteration
     int parity = 0;
     int chunk = std::max(1, check_every);
     // Launch positions of each trip in the engine profiler: its K1, K2, the rest, its end.
@@ -332,7 +433,8 @@ SolveResult cg_impl(Ctx& ctx, hamlss_mat* A, Prec* M, const T* b, T* x, double t
     while (run) {
         const int iter0 = h.iter;
         trips.clear();
-        for (int t = 0; t < chunk; ++t) {
+        if (persist) launch_persist<T, JAC>(ctx, A, Ad, x, r, p[0], zp, dinv, s, FinTrip<JAC>{});
+        for (int t = 0; t < chunk && !persist; ++t) {
             TripMarks tm;
             tm.k1 = prof_pos(L.prof);
             T* pold = p[parity];
@@ -353,7 +455,7 @@ SolveResult cg_impl(Ctx& ctx, hamlss_mat* A, Prec* M, const T* b, T* x, double t
             parity ^= 1;
         }
         poll(h);
-        if (h.halt) {
+        if (h.halt && !persist) {
             // every trip increments iter once, the halting one included; the launches the
             // gate skipped are booked as "gated", with no bytes
             const int ran = std::max(1, std::min((int)trips.size(), h.iter - iter0));
@@ -539,6 +641,15 @@ struct FinRzRU {
     __device__ void operator()(const double (&t)[NV]) const { rho_step(s, t[0], 4); }
 };
 
+// finalisers of k_cg_persist for the reliable-update iteration: a trip that is due an update
+// leaves the launch, the update's launches finish the trip
+struct FinTripRU {
+    __device__ void pq(CgState* s, const double (&t)[1]) const { FinPQ{s}(t); }
+    __device__ void upd(CgState* s, const double (&t)[2]) const { FinUpdRU<true>{s}(t); }
+    __device__ bool leave(const CgState* s) const { return s->skip_ru == 0; }
+    __device__ void timeout(CgState* s) const { s->status = ST_MAXIT; s->halt = 1; }
+};
+
 template <bool JAC>
 SolveResult cg_reliable_impl(Ctx& ctx, hamlss_mat* A, Prec* M, const double* b, double* x, double tol,
                              int max_iter, int check_every, double delta, Workspace& ws,
@@ -589,11 +700,21 @@ SolveResult cg_reliable_impl(Ctx& ctx, hamlss_mat* A, Prec* M, const double* b, 
         std::memcpy(&h, ctx.host_poll.p, sizeof(CgState));
     };
 
+    // gated by skip_ru: runs only in a trip that is due an update
+    auto update = [&]() {
+        launch_vec<0>(sm, L, n, BodyFold{x, y, s, 0.0}, NoFin{}, skip_ru, "mixed_fold", 2.0 * w8 + 2.0 * w4);
+        launch_spmv<double, JAC ? 2 : 1>(sm, L, A64, XVec<double>{x}, EpiRelRes<JAC>{b, r, dinv, s, 0.0},
+                                         FinRU<JAC>{s}, skip_ru, "mixed_residual",
+                                         2.0 * w8 + (JAC ? 2.0 : 1.0) * w4);
+    };
+
     SolveResult res;
     CgState h{};
     restart_seq(true);
     poll(h);
     const bool run = !h.halt && max_iter > 0;
+    const bool persist = run && JAC && persist_fits<float>(ctx, A);
+    float* zp = persist ? wvec<float>(ws, 1, n) : nullptr;     // z of the persistent iteration
     int parity = 0;
     int chunk = std::max(1, check_every);
     struct TripMarks { size_t k1, k2, ru, rest, end; int iter; };
@@ -604,7 +725,13 @@ SolveResult cg_reliable_impl(Ctx& ctx, hamlss_mat* A, Prec* M, const double* b, 
     while (run) {
         const int iter0 = h.iter;
         trips.clear();
-        for (int t = 0; t < chunk; ++t) {
+        if constexpr (JAC) {
+            if (persist) {
+                launch_persist<float, true>(ctx, A, A32, y, r, p[0], zp, dinv, s, FinTripRU{});
+                update();
+            }
+        }
+        for (int t = 0; t < chunk && !persist; ++t) {
             TripMarks tm;
             tm.iter = iter0 + t;
             tm.k1 = prof_pos(L.prof);
@@ -617,10 +744,7 @@ SolveResult cg_reliable_impl(Ctx& ctx, hamlss_mat* A, Prec* M, const double* b, 
             launch_vec<JAC ? 2 : 1>(sm, L, n, BodyUpd<float, JAC>{y, r, pnew, q, dinv, s, 0.0},
                                     FinUpdRU<JAC>{s}, halt, "cg_update", (JAC ? 7.0 : 6.0) * w4);
             tm.ru = prof_pos(L.prof);
-            launch_vec<0>(sm, L, n, BodyFold{x, y, s, 0.0}, NoFin{}, skip_ru, "mixed_fold", 2.0 * w8 + 2.0 * w4);
-            launch_spmv<double, JAC ? 2 : 1>(sm, L, A64, XVec<double>{x}, EpiRelRes<JAC>{b, r, dinv, s, 0.0},
-                                             FinRU<JAC>{s}, skip_ru, "mixed_residual",
-                                             2.0 * w8 + (JAC ? 2.0 : 1.0) * w4);
+            update();
             tm.rest = prof_pos(L.prof);
             if (!JAC) {
                 if (M) precond_apply<float>(ctx, M, r, z, halt);
@@ -632,8 +756,9 @@ SolveResult cg_reliable_impl(Ctx& ctx, hamlss_mat* A, Prec* M, const double* b, 
         }
         poll(h);
         HAMLSS_CUDA(cudaMemsetAsync(&s->ru_mask, 0, sizeof(unsigned long long), st));
-        const int ran = h.halt ? std::max(1, std::min((int)trips.size(), h.iter - iter0)) : (int)trips.size();
-        if (L.prof) {
+        if (persist) updates += __builtin_popcountll(h.ru_mask);
+        const int ran = persist ? 0 : h.halt ? std::max(1, std::min((int)trips.size(), h.iter - iter0)) : (int)trips.size();
+        if (L.prof && !persist) {
             // updates that did not run, and everything the halt gate skipped
             for (int k = 0; k < ran; ++k)
                 if (!((h.ru_mask >> (trips[k].iter & 63)) & 1ull)) prof_gated(L.prof, trips[k].ru, trips[k].rest);

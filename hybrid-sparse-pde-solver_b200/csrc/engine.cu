@@ -48,6 +48,7 @@ void lane_destroy(Lane& L) {
     L.partials.release();
     L.ticket.release();
     L.err.release();
+    L.sums.release();
 }
 
 namespace {
@@ -117,7 +118,58 @@ __global__ void k_rows_longer(int n, const int* __restrict__ rp, int len, int* l
         if (rp[i + 1] - rp[i] > len) list[atomicAdd(count, 1)] = i;
 }
 
+// most[0], most[1] = the most entries, and columns spanned, of `rows` consecutive rows
+// (block b: rows [b * rows, ...)) of a matrix with sorted rows; the block's own rows count
+// as columns.
+__global__ void __launch_bounds__(256)
+k_persist_plan(int n, int rows, const int* __restrict__ rp, const int* __restrict__ ci, int* most) {
+    __shared__ int lo, hi;
+    const int r0 = blockIdx.x * rows, r1 = min(n, r0 + rows);
+    if (threadIdx.x == 0) { lo = r0; hi = r1; }
+    __syncthreads();
+    for (int row = r0 + threadIdx.x; row < r1; row += blockDim.x) {
+        const int b = rp[row], e = rp[row + 1];
+        if (b < e) {
+            atomicMin(&lo, ci[b]);
+            atomicMax(&hi, ci[e - 1] + 1);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        atomicMax(&most[0], rp[r1] - rp[r0]);
+        atomicMax(&most[1], hi - lo);
+    }
+}
+
 }  // namespace
+
+void ensure_persist_plan(Ctx& ctx, hamlss_mat* M) {
+    if (M->persist_rows >= 0) return;
+    M->persist_rows = 0;
+    const int n = M->A.n;
+    if (n == 0 || ctx.sm_count < 1) return;
+    // equal shares of whole warps, one 256-row tile at least: of a cluster's blocks up to
+    // kPersistClusterRows rows where a block's memory holds them, else of a block per SM
+    for (const bool cluster : {true, false}) {
+        if (cluster && n > kPersistClusterRows) continue;
+        const int blocks = cluster ? kPersistClusterBlocks : ctx.sm_count;
+        const int rows = std::max(256, ceil_div(ceil_div(n, blocks), 32) * 32);
+        if (rows > kPersistMaxRows) return;
+        cudaStream_t s = ctx.lane.stream;
+        DBuf<int> most(2);
+        most.zero(s);
+        k_persist_plan<<<ceil_div(n, rows), 256, 0, s>>>(n, rows, M->A.rp.p, M->A.ci.p, most.p);
+        HAMLSS_LAUNCH_CHECK();
+        int h[2];
+        most.download(h, 2, s);
+        HAMLSS_CUDA(cudaStreamSynchronize(s));
+        M->persist_entries = h[0];
+        M->persist_window = h[1];
+        M->persist_rows = rows;
+        M->persist_cluster = cluster;
+        if (persist_smem<double>(h[0], h[1]) <= kPersistSmem) return;
+    }
+}
 
 Csr<float> DevMat::f32(cudaStream_t s) {
     if (!v32_valid) {

@@ -64,7 +64,8 @@ struct Lane {
     DBuf<double> partials;
     DBuf<unsigned> ticket;
     size_t red_cap = 0;       // entries of `partials`
-    DBuf<int> err;            // set by a bulk-copy SpMV whose wait ran out (zero otherwise)
+    DBuf<int> err;            // set by a kernel whose bounded wait ran out (zero otherwise)
+    DBuf<double> sums;        // block sums and barrier counter of a persistent kernel (cg_persist.cuh)
     Profiler* prof = nullptr;
     Reducer red() const { return Reducer{partials.p, ticket.p}; }
     // a grid of `blocks` blocks, each storing `nred` partial sums, must fit `partials`
@@ -126,6 +127,21 @@ bool lane_take_timeout(const Lane& L);
 constexpr int kSkewRow = 1024;
 constexpr double kSkewRatio = 32.0;
 void ensure_row_profile(Ctx& ctx, hamlss_mat* M);
+// Rows a block, and the entries and columns its rows span at most, of the persistent CG
+// (once per matrix; the pattern is fixed).
+constexpr int kPersistMaxRows = 3584;
+constexpr int kPersistClusterBlocks = 16;
+// (us a trip, Jacobi on grids: cluster 3.2 at 4,096 rows, 4.4 at 16,384, 6.7 at 32,761, 9.6 at
+// 48,841; grid 6.5 at 65,536, 8.0 at 160,000, 11.8 at 491,401)
+constexpr int kPersistClusterRows = 28672;
+constexpr int kPersistMaxBlocks = 256;
+constexpr size_t kPersistSmem = 224 * 1024;   // shared memory of a block beside the kernel's own
+// Shared memory of a block: p window, matrix values and 16-bit column offsets.
+template <typename T>
+size_t persist_smem(int entries, int window) {
+    return (size_t)((window + 1) & ~1) * sizeof(T) + (size_t)((entries + 3) & ~3) * (sizeof(T) + 2) + 16;
+}
+void ensure_persist_plan(Ctx& ctx, hamlss_mat* M);
 
 // Device view of a CSR matrix.
 template <typename T>
@@ -308,6 +324,12 @@ struct hamlss_mat {
     hamlss::DBuf<int> long_rows;
     int n_long = -1;
     int long_len = INT_MAX;
+    // shared-memory needs of the persistent CG (hamlss::ensure_persist_plan): rows a block
+    // (0: too many rows, < 0: not worked out yet), entries and columns of the largest block
+    int persist_rows = -1;
+    int persist_entries = 0;
+    int persist_window = 0;
+    bool persist_cluster = false;   // one thread-block cluster holds it
     uint64_t version = 0;           // bumped by hamlss_mat_update_values
     hamlss::Workspace ws;
 };
