@@ -210,6 +210,29 @@ bool long_rows_warp(const Csr<T>& A) {
     return sizeof(T) == 4 && A.n > 0 && (double)A.nnz / A.n >= 48.0;
 }
 
+// Rows a warp of the ordered-product kernel (k_spmv_prod), or 0 where the lane-per-row
+// kernels do as well: FP64 operators of more than 5.5 entries a row (the bulk-copy kernel's
+// limit).  A warp's rows fit its 512 products on average, and are halved while fewer than
+// four warps an SM would have work.
+template <typename T>
+int prod_rows(int sm_count, const Csr<T>& A) {
+    if (sizeof(T) != 8 || A.n == 0) return 0;
+    const double avg = (double)A.nnz / A.n;
+    if (avg <= 5.5) return 0;
+    const int fit = (int)(kProdFill * kProdTile / avg), share = A.n / (4 * sm_count);
+    return std::max(1, std::min(32, std::min(fit, share)));
+}
+
+template <typename XOp, typename Epi>
+void launch_spmv_prod(int sm_count, const Lane& L, const Csr<double>& A, const XOp& xop, const Epi& epi,
+                      const int* gate, int R) {
+    auto kern = k_spmv_prod<XOp, Epi>;
+    static const int per_sm = occupancy_blocks(kern, 32 * kProdWarps);
+    const int blocks = std::max(1, std::min(ceil_div(ceil_div(A.n, R), kProdWarps), sm_count * per_sm));
+    kern<<<blocks, 32 * kProdWarps, 0, L.stream>>>(A.n, R, A.rp, A.ci, A.v, xop, epi, gate);
+    HAMLSS_LAUNCH_CHECK();
+}
+
 // Max co-resident CTAs of a bulk-copy SpMV instantiation (its dynamic shared memory
 // raised above the 48 KB default once).
 template <typename K>
@@ -269,6 +292,11 @@ void launch_spmv(int sm_count, const Lane& L, const Csr<T>& A, const XOp& xop, c
             HAMLSS_LAUNCH_CHECK();
             return;
         }
+    }
+    if constexpr (sizeof(T) == 8 && NRED == 0) {
+        // (a skewed matrix's long rows are split off by the lane-per-row kernels only)
+        const int R = skip_len == INT_MAX ? prod_rows(sm_count, A) : 0;
+        if (R) return launch_spmv_prod(sm_count, L, A, xop, epi, gate, R);
     }
     auto kern = k_spmv<T, NRED, XOp, Epi, Fin>;
     // thread-safe one-time initialisation (contexts may be driven from several threads)

@@ -230,6 +230,92 @@ k_spmv_rows_seq(const int* __restrict__ rows, int nrows, const int* __restrict__
     }
 }
 
+// FP64 operators with more than a few entries a row, in the reference's order: R consecutive
+// rows a warp.  A lane per row (k_spmv) reads its row from its own place, 32 cache lines a
+// load, and waits for each group of four entries in turn; here the warp walks the R rows'
+// entries as one range -- coalesced loads of columns and values, eight gathers of x in
+// flight a lane -- and leaves the products a_ij * x_j in shared memory, where lane r adds
+// row r's in column order (separate multiply and add: bit-identical to the plain loop,
+// sparse_matrix.cpp:80-86).  The additions are a chain a row (~9 cycles each), so R falls as
+// rows get longer or too few for the chip (prod_rows); what bounds it then is that chain on
+// the longest rows, or the gathers: on scattered columns each lane touches its own line
+// (L1 81 % busy at 300,007 ragged rows of 24 entries).  More warps an SM with fewer loads
+// each, or tiles of 256 to 1,024 products, were no faster there and up to 1.6x slower on
+// aggregation levels.  Measured, lane a row -> this: 300,007 x 24 ragged 53 -> 36 us, 50,021
+// x 100 107 -> 47 us, an FP64 V-cycle on 1024^2 2.19 -> 0.93 ms.
+constexpr int kProdWarps = 8;
+constexpr int kProdTile = 512;               // products a warp holds
+constexpr double kProdFill = 0.85;           // average share of them its rows take
+constexpr int kProdLoads = 8;                // entries a lane loads at a time
+
+template <typename XOp, typename Epi>
+__global__ void __launch_bounds__(32 * kProdWarps)
+k_spmv_prod(int n, int R, const int* __restrict__ rp, const int* __restrict__ ci, const double* __restrict__ v, XOp xop,
+            Epi epi, const int* gate) {
+    __shared__ double prod[kProdWarps][kProdTile];
+    if (gate && *(volatile const int*)gate) return;
+    XOp xop_l = xop;
+    Epi epi_l = epi;
+    xop_l.load();
+    epi_l.load();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    double* pw = prod[wid];
+    const int tiles = (n + R - 1) / R;
+    double none[1];
+    for (int t = blockIdx.x * kProdWarps + wid; t < tiles; t += gridDim.x * kProdWarps) {
+        const int row = t * R + lane;
+        const bool own = lane < R && row < n;
+        int b = 0, e = 0;
+        if (own) {
+            b = __ldg(&rp[row]);
+            e = __ldg(&rp[row + 1]);
+        }
+        const int rows = min(R, n - t * R);
+        const int e0 = __shfl_sync(0xffffffffu, b, 0), e1 = __shfl_sync(0xffffffffu, e, rows - 1);
+        double sum = 0.0;
+        for (int base = e0; base < e1; base += kProdTile) {
+            const int cnt = min(kProdTile, e1 - base);
+            for (int k0 = 0; k0 < cnt; k0 += 32 * kProdLoads) {
+                double a[kProdLoads];
+                int c[kProdLoads];
+#pragma unroll
+                for (int u = 0; u < kProdLoads; ++u) {
+                    const int k = k0 + u * 32 + lane;
+                    if (k < cnt) {
+                        c[u] = __ldg(&ci[base + k]);
+                        a[u] = __ldg(&v[base + k]);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < kProdLoads; ++u) {
+                    const int k = k0 + u * 32 + lane;
+                    if (k < cnt) a[u] = __dmul_rn(a[u], xop_l(c[u]));
+                }
+#pragma unroll
+                for (int u = 0; u < kProdLoads; ++u) {
+                    const int k = k0 + u * 32 + lane;
+                    if (k < cnt) pw[k] = a[u];
+                }
+            }
+            __syncwarp();
+            if (own) {
+                int k = max(b, base) - base;
+                const int lim = min(e - base, cnt);
+                for (; k + 8 <= lim; k += 8) {
+                    double q[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) q[u] = pw[k + u];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) sum = __dadd_rn(sum, q[u]);
+                }
+                for (; k < lim; ++k) sum = __dadd_rn(sum, pw[k]);
+            }
+            __syncwarp();
+        }
+        if (own) epi_l(row, sum, none);
+    }
+}
+
 // Elementwise kernel with the same reduction / finalize machinery (no matrix).
 template <int NRED, typename Body, typename Fin>
 __global__ void __launch_bounds__(256)
