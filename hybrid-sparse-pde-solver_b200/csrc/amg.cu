@@ -756,6 +756,135 @@ __global__ void k_spgemm_classify(int m, const int* __restrict__ arp, const int*
     }
 }
 
+// C = A B for small right operands, held dense (Bd: B.n x ld, zeros where B has no entry):
+// a block per row, a thread per column of the row's window [lo_i, lo_i + span_i), each adding
+// a_t * Bd[j_t][c] over the left row in order, from 0.0, with separate multiply and add --
+// the arithmetic of k_spgemm; the zero products it adds leave a sum as it is (the launcher
+// makes sure A is finite).  No step waits for another, so a row costs its left entries' loads
+// (sixteen in flight a thread) and adds: the near-dense levels of a few hundred rows took
+// 2 ms a product in the merging kernels, one output column at a time, and take ~10 us here.
+constexpr int kGatherThreads = 128;
+constexpr int kGatherLeft = 256;             // left entries staged at a time
+constexpr int kGatherLoads = 8;
+
+__global__ void k_dense_rows(int n, const int* __restrict__ rp, const int* __restrict__ ci,
+                             const double* __restrict__ v, int ld, double* Bd) {
+    const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nw)
+        for (int k = rp[i] + lane; k < rp[i + 1]; k += 32) Bd[(size_t)i * ld + ci[k]] = v[k];
+}
+
+// sums[0] += products, sums[1] += pairs (left entry, window column) of every row;
+// *notfinite: A has a non-finite value
+__global__ void k_gather_cost(int m, const int* __restrict__ arp, const int* __restrict__ aci,
+                              const double* __restrict__ av, const int* __restrict__ brp,
+                              const int* __restrict__ bci, int* wlo, int* wspan, unsigned long long* sums,
+                              int* notfinite) {
+    unsigned long long prods = 0, pairs = 0;
+    bool bad = false;
+    const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < m; i += nw) {
+        const int s = arp[i], e = arp[i + 1];
+        int lo = INT_MAX, hi = -1;
+        for (int t = s + lane; t < e; t += 32) {
+            const int j = aci[t], p0 = brp[j], p1 = brp[j + 1];
+            prods += p1 - p0;
+            bad |= !isfinite(av[t]);
+            if (p1 > p0) {
+                lo = min(lo, bci[p0]);
+                hi = max(hi, bci[p1 - 1]);
+            }
+        }
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        const int span = hi >= lo ? hi - lo + 1 : 0;
+        if (lane == 0) {
+            wlo[i] = span ? lo : 0;
+            wspan[i] = span;
+            pairs += (unsigned long long)(e - s) * (unsigned)span;
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) prods += __shfl_xor_sync(0xffffffffu, prods, o);
+    if (lane == 0) {
+        atomicAdd(&sums[0], prods);
+        atomicAdd(&sums[1], pairs);
+    }
+    if (bad) *notfinite = 1;
+}
+
+__global__ void __launch_bounds__(kGatherThreads)
+k_spgemm_gather(int m, const int* __restrict__ wlo, const int* __restrict__ wspan, const int* __restrict__ arp,
+                const int* __restrict__ aci, const double* __restrict__ av, const double* __restrict__ Bd, int ld,
+                int* ccnt, const int* __restrict__ off, int* cci, double* cv) {
+    __shared__ double sa[kGatherLeft];
+    __shared__ int sj[kGatherLeft];
+    __shared__ int s_warp[kGatherThreads / 32];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    for (int i = blockIdx.x; i < m; i += gridDim.x) {
+        const int s = arp[i], k = arp[i + 1] - s, lo = wlo[i], span = wspan[i];
+        int o = off[i];
+        for (int c0 = 0; c0 < span; c0 += 2 * kGatherThreads) {
+            // columns c and c + kGatherThreads of this thread (clamped; unused beyond the window)
+            const int c1 = c0 + tid, c2 = c1 + kGatherThreads;
+            const double* b1 = Bd + lo + min(c1, span - 1);
+            const double* b2 = Bd + lo + min(c2, span - 1);
+            double s1 = 0.0, s2 = 0.0;
+            for (int t0 = 0; t0 < k; t0 += kGatherLeft) {
+                const int kk = min(kGatherLeft, k - t0);
+                __syncthreads();
+                for (int t = tid; t < kk; t += kGatherThreads) {
+                    sa[t] = av[s + t0 + t];
+                    sj[t] = aci[s + t0 + t];
+                }
+                __syncthreads();
+                int t = 0;
+                for (; t + kGatherLoads <= kk; t += kGatherLoads) {
+                    double v1[kGatherLoads], v2[kGatherLoads];
+#pragma unroll
+                    for (int u = 0; u < kGatherLoads; ++u) {
+                        const size_t r = (size_t)sj[t + u] * ld;
+                        v1[u] = __ldg(&b1[r]);
+                        v2[u] = __ldg(&b2[r]);
+                    }
+#pragma unroll
+                    for (int u = 0; u < kGatherLoads; ++u) {
+                        s1 = __dadd_rn(s1, __dmul_rn(sa[t + u], v1[u]));
+                        s2 = __dadd_rn(s2, __dmul_rn(sa[t + u], v2[u]));
+                    }
+                }
+                for (; t < kk; ++t) {
+                    const size_t r = (size_t)sj[t] * ld;
+                    s1 = __dadd_rn(s1, __dmul_rn(sa[t], __ldg(&b1[r])));
+                    s2 = __dadd_rn(s2, __dmul_rn(sa[t], __ldg(&b2[r])));
+                }
+            }
+            // survivors in column order: the first 128 columns, then the second
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int c = h == 0 ? c1 : c2;
+                const double sum = h == 0 ? s1 : s2;
+                const bool keep = c < span && fabs(sum) > kEps * kEps;
+                const unsigned bal = __ballot_sync(0xffffffffu, keep);
+                __syncthreads();
+                if (lane == 0) s_warp[wid] = __popc(bal);
+                __syncthreads();
+                int at = o;
+                for (int w = 0; w < kGatherThreads / 32; ++w) {
+                    if (w < wid) at += s_warp[w];
+                    o += s_warp[w];
+                }
+                if (keep) {
+                    at += __popc(bal & ((1u << lane) - 1u));
+                    cci[at] = lo + c;
+                    cv[at] = sum;
+                }
+            }
+        }
+        if (tid == 0) ccnt[i] = o - off[i];
+        __syncthreads();
+    }
+}
+
 // Row i of C = A B for the listed rows, one warp per row: a k-way merge of the selected
 // rows of B with the k merge heads in shared memory (lane l owns heads l, l+32, ...).  Each
 // output column is the warp-wide minimum of the heads; its products are added in the
@@ -1421,105 +1550,158 @@ __global__ void k_d2f(const double* __restrict__ a, float* b, long long n) {
 }
 
 // ------------------------------------------------------------- coarsest level
-// Dense Gaussian elimination with partial pivoting (amg.cpp:260-291), one block, on the
-// n x n matrix M (row-major).  Stores the multipliers below the diagonal, the pivot row
-// of each column and whether the column was skipped (|pivot| < 1e-14).
-__global__ void k_dense_factor(int n, double* M, int* piv, int* skip) {
-    __shared__ int sp;
+// Dense Gaussian elimination with partial pivoting (amg.cpp:260-291) of the n x n matrix W
+// (row-major, destroyed) by one thread-block cluster.  Writes the multipliers below the
+// diagonal and the pivot rows' remaining entries into M, the pivot row of each column and
+// whether the column was skipped (|pivot| < 1e-14).  Rows are not swapped in memory: every
+// block keeps the order of the remaining rows, so a step is one round of reads (the column,
+// then the pivot row and the rows below) and one cluster barrier.  A step is bound by those
+// latencies: 155 rows in 5.25 ms by one block that searched the pivot with one thread and
+// walked rows in place, 0.25 ms here.
+constexpr int kFactorBlocks = 16, kFactorThreads = 512;
+__global__ void __launch_bounds__(kFactorThreads)
+k_dense_factor(int n, double* W, double* M, int* piv, int* skip) {
+    __shared__ int order[kBlockedCoarse];
+    __shared__ double prow[kBlockedCoarse];
+    __shared__ double s_v[kFactorThreads / 32];
+    __shared__ int s_r[kFactorThreads / 32];
+    __shared__ int s_p;
+    auto cluster = cg::this_cluster();
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    for (int r = tid; r < n; r += kFactorThreads) order[r] = r;
+    __syncthreads();
     for (int col = 0; col < n; ++col) {
-        if (threadIdx.x == 0) {
-            int p = col;
-            for (int r = col + 1; r < n; ++r)
-                if (fabs(M[(size_t)r * n + col]) > fabs(M[(size_t)p * n + col])) p = r;
-            piv[col] = p;
-            sp = p;
+        // the first row of the largest |entry| above the one on the diagonal (NaN never wins)
+        const double v0 = fabs(__ldcg(&W[(size_t)order[col] * n + col]));
+        double bv = v0;
+        int br = col;
+        for (int r = col + 1 + tid; r < n; r += kFactorThreads) {
+            const double v = fabs(__ldcg(&W[(size_t)order[r] * n + col]));
+            if (v > bv) { bv = v; br = r; }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double ov = __shfl_xor_sync(0xffffffffu, bv, o);
+            const int orr = __shfl_xor_sync(0xffffffffu, br, o);
+            if (ov > bv || (ov == bv && orr < br)) { bv = ov; br = orr; }
+        }
+        if (lane == 0) { s_v[wid] = bv; s_r[wid] = br; }
+        __syncthreads();
+        if (tid == 0) {
+            for (int w = 1; w < kFactorThreads / 32; ++w)
+                if (s_v[w] > bv || (s_v[w] == bv && s_r[w] < br)) { bv = s_v[w]; br = s_r[w]; }
+            s_p = br;
+            const int t = order[col];
+            order[col] = order[br];
+            order[br] = t;
         }
         __syncthreads();
-        const int p = sp;
-        // columns < col hold multipliers that belong to the row position at their step
-        if (p != col)
-            for (int c = col + threadIdx.x; c < n; c += blockDim.x) {
-                double t = M[(size_t)col * n + c];
-                M[(size_t)col * n + c] = M[(size_t)p * n + c];
-                M[(size_t)p * n + c] = t;
-            }
+        const double* pr = W + (size_t)order[col] * n;
+        for (int c = col + tid; c < n; c += kFactorThreads) prow[c] = __ldcg(&pr[c]);
         __syncthreads();
-        const double d = M[(size_t)col * n + col];
+        const double d = prow[col];
         const bool sk = fabs(d) < 1e-14;
-        if (threadIdx.x == 0) skip[col] = sk;
+        if (blockIdx.x == 0) {
+            if (tid == 0) { piv[col] = s_p; skip[col] = sk; }
+            for (int c = col + tid; c < n; c += kFactorThreads) M[(size_t)col * n + c] = prow[c];
+        }
         if (!sk) {
             const double inv = 1.0 / d;
-            for (int r = col + 1 + threadIdx.x; r < n; r += blockDim.x) {
-                double f = __dmul_rn(M[(size_t)r * n + col], inv);
-                for (int c = col + 1; c < n; ++c)
-                    M[(size_t)r * n + c] = __dsub_rn(M[(size_t)r * n + c], __dmul_rn(f, M[(size_t)col * n + c]));
-                M[(size_t)r * n + col] = f;       // multiplier (the reference's entry becomes 0)
+            const int w0 = blockIdx.x * (kFactorThreads / 32) + wid, nw = gridDim.x * (kFactorThreads / 32);
+            for (int r = col + 1 + w0; r < n; r += nw) {
+                double* wr = W + (size_t)order[r] * n;
+                const double f = __dmul_rn(__ldcg(&wr[col]), inv);
+                if (lane == 0) M[(size_t)r * n + col] = f;      // the multiplier, by row position
+                for (int c = col + 1 + lane; c < n; c += 32)
+                    wr[c] = __dsub_rn(__ldcg(&wr[c]), __dmul_rn(f, prow[c]));
             }
         }
-        __syncthreads();
+        cluster.sync();
+    }
+}
+
+// U z = y with the stored factors, one warp: the lanes form row i's products, lane 0
+// subtracts them in column order (the reference's order, a chain of ~10 cycles an entry;
+// with one lane loading and multiplying as well it was ~55).  y and z in shared memory,
+// prod: 32 doubles of it.
+__device__ __forceinline__ void warp_back_solve(int n, const double* __restrict__ M, const double* y, double* z,
+                                                double* prod) {
+    const int lane = threadIdx.x & 31;
+    for (int i = n - 1; i >= 0; --i) {
+        const double* row = M + (size_t)i * n;
+        double s = y[i];
+        double m = i + 1 + lane < n ? __ldg(&row[i + 1 + lane]) : 0.0;
+        for (int j0 = i + 1; j0 < n; j0 += 32) {
+            const int j = j0 + lane;
+            prod[lane] = j < n ? __dmul_rn(m, z[j]) : 0.0;
+            m = j + 32 < n ? __ldg(&row[j + 32]) : 0.0;          // the next 32, in flight
+            __syncwarp();
+            if (lane == 0) {
+                const int cnt = min(32, n - j0);
+                int q = 0;
+                for (; q + 8 <= cnt; q += 8) {
+                    double t[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) t[u] = prod[q + u];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) s = __dsub_rn(s, t[u]);
+                }
+                for (; q < cnt; ++q) s = __dsub_rn(s, prod[q]);
+            }
+            __syncwarp();
+        }
+        if (lane == 0) {
+            const double d = __ldg(&row[i]);
+            z[i] = (fabs(d) > 1e-14) ? s / d : 0.0;
+        }
+        __syncwarp();
+    }
+}
+
+// Forward elimination of y with the stored factors, one warp (y in shared memory).
+__device__ __forceinline__ void warp_forward_solve(int n, const double* __restrict__ M, const int* __restrict__ piv,
+                                                   const int* __restrict__ skip, double* y) {
+    const int lane = threadIdx.x & 31;
+    for (int col = 0; col < n; ++col) {
+        const int p = __ldg(&piv[col]);
+        if (p != col && lane == 0) { const double t = y[col]; y[col] = y[p]; y[p] = t; }
+        __syncwarp();
+        if (!__ldg(&skip[col])) {
+            const double yc = y[col];
+            for (int r = col + 1 + lane; r < n; r += 32)
+                y[r] = __dsub_rn(y[r], __dmul_rn(__ldg(&M[(size_t)r * n + col]), yc));
+        }
+        __syncwarp();
     }
 }
 
 // x = A^-1 b with the stored factors, one warp, the reference's operation order.
 template <typename T>
 __global__ void k_dense_solve(int n, const double* __restrict__ M, const int* __restrict__ piv,
-                              const int* __restrict__ skip, const T* __restrict__ b, T* x,
-                              double* work, const int* gate) {
+                              const int* __restrict__ skip, const T* __restrict__ b, T* x, const int* gate) {
+    extern __shared__ double dense_y[];                  // y, z, 32 products
     if (gate && *(volatile const int*)gate) return;
-    double* y = work;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) y[i] = (double)b[i];
+    double* y = dense_y;
+    double* z = y + n;
+    for (int i = threadIdx.x; i < n; i += 32) y[i] = (double)b[i];
     __syncwarp();
-    for (int col = 0; col < n; ++col) {
-        const int p = piv[col];
-        if (p != col && threadIdx.x == 0) { double t = y[col]; y[col] = y[p]; y[p] = t; }
-        __syncwarp();
-        if (!skip[col]) {
-            const double yc = y[col];
-            for (int r = col + 1 + threadIdx.x; r < n; r += blockDim.x)
-                y[r] = __dsub_rn(y[r], __dmul_rn(M[(size_t)r * n + col], yc));
-        }
-        __syncwarp();
-    }
-    if (threadIdx.x == 0) {
-        for (int i = n - 1; i >= 0; --i) {
-            double s = y[i];
-            for (int j = i + 1; j < n; ++j) s = __dsub_rn(s, __dmul_rn(M[(size_t)i * n + j], y[n + j]));
-            double d = M[(size_t)i * n + i];
-            y[n + i] = (fabs(d) > 1e-14) ? s / d : 0.0;
-        }
-    }
-    __syncwarp();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) x[i] = (T)y[n + i];
+    warp_forward_solve(n, M, piv, skip, y);
+    warp_back_solve(n, M, y, z, z + n);
+    for (int i = threadIdx.x; i < n; i += 32) x[i] = (T)z[i];
 }
 
 // Columns of the inverse, one warp per unit right-hand side e_k: Minv[r][k].
 __global__ void k_dense_inverse(int n, const double* __restrict__ M, const int* __restrict__ piv,
-                                const int* __restrict__ skip, double* work, double* Minv) {
+                                const int* __restrict__ skip, double* Minv) {
+    extern __shared__ double dense_y[];
     const int k = blockIdx.x;
-    double* y = work + (size_t)k * 2 * n;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) y[i] = (i == k) ? 1.0 : 0.0;
+    double* y = dense_y;
+    double* z = y + n;
+    for (int i = threadIdx.x; i < n; i += 32) y[i] = (i == k) ? 1.0 : 0.0;
     __syncwarp();
-    for (int col = 0; col < n; ++col) {
-        const int p = piv[col];
-        if (p != col && threadIdx.x == 0) { double t = y[col]; y[col] = y[p]; y[p] = t; }
-        __syncwarp();
-        if (!skip[col]) {
-            const double yc = y[col];
-            for (int r = col + 1 + threadIdx.x; r < n; r += blockDim.x)
-                y[r] = __dsub_rn(y[r], __dmul_rn(M[(size_t)r * n + col], yc));
-        }
-        __syncwarp();
-    }
-    if (threadIdx.x == 0) {
-        for (int i = n - 1; i >= 0; --i) {
-            double t = y[i];
-            for (int j = i + 1; j < n; ++j) t = __dsub_rn(t, __dmul_rn(M[(size_t)i * n + j], y[n + j]));
-            double d = M[(size_t)i * n + i];
-            y[n + i] = (fabs(d) > 1e-14) ? t / d : 0.0;
-        }
-    }
-    __syncwarp();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) Minv[(size_t)i * n + k] = y[n + i];
+    warp_forward_solve(n, M, piv, skip, y);
+    warp_back_solve(n, M, y, z, z + n);
+    for (int i = threadIdx.x; i < n; i += 32) Minv[(size_t)i * n + k] = z[i];
 }
 
 // Explicit inverse applied as a dense matrix-vector product (large coarsest levels); the
@@ -1779,6 +1961,9 @@ struct AmgLevel {
     int n = 0;
 };
 
+// Shared memory of k_dense_solve / k_dense_inverse.
+inline size_t dense_solve_smem(int n) { return sizeof(double) * (2 * (size_t)n + 32); }
+
 struct AmgPrec : Prec {
     hamlss_mat* A0 = nullptr;
     std::vector<std::unique_ptr<AmgLevel>> lev;
@@ -1787,7 +1972,7 @@ struct AmgPrec : Prec {
     // coarsest dense data
     int nc = 0;
     bool coarse_inverse = false;
-    DBuf<double> Md, Minv, cwork;
+    DBuf<double> Md, Minv;
     DBuf<float> Minv32;                 // FP32 copy of Minv for the FP32 V-cycle
     DBuf<int> piv, skip;
     bool f32_ready = false;
@@ -1820,7 +2005,7 @@ struct AmgPrec : Prec {
                 k_dense_gemv<T, double><<<g, 256, 0, L.stream>>>(nc, Minv.p, b, x, gate);
         } else {
             ProfScope ps(L, "amg_coarse", 8.0 * nc * nc);
-            k_dense_solve<T><<<1, 32, 0, L.stream>>>(nc, Md.p, piv.p, skip.p, b, x, cwork.p, gate);
+            k_dense_solve<T><<<1, 32, dense_solve_smem(nc), L.stream>>>(nc, Md.p, piv.p, skip.p, b, x, gate);
         }
         HAMLSS_LAUNCH_CHECK();
     }
@@ -2216,7 +2401,58 @@ void seq_rows(Ctx& ctx, bool fill, const int* rows, int nrows, int span, const i
     HAMLSS_LAUNCH_CHECK();
 }
 
+// C = A B with B held dense (k_spgemm_gather), where B is small and the pairs it visits are
+// few for the products they hold: below kGatherPairs always (the merging classes cost ~2 ms
+// on near-dense levels whatever their size), else up to kGatherRatio a product, as long as
+// they stay below kGatherMost.  (L2 delivers ~1.4e12 pairs a second; the classes handle ~1e11
+// products.)  false: not taken.
+constexpr long long kGatherDense = 16LL << 20;           // entries of B held dense
+constexpr unsigned long long kGatherPairs = 200ull * 1000 * 1000;
+constexpr unsigned long long kGatherMost = 1000ull * 1000 * 1000;
+constexpr unsigned long long kGatherRatio = 8;
+
+bool spgemm_gather(Ctx& ctx, const Csr<double>& A, const Csr<double>& B, DCsr& C) {
+    if (!A.n || !A.nnz || !B.m || (long long)B.n * B.m > kGatherDense) return false;
+    // (cheap bounds first: small rows belong to the sequential classes)
+    if ((double)A.nnz / A.n < 48.0 && (double)A.nnz * B.m > (double)kGatherPairs) return false;
+    cudaStream_t s = ctx.lane.stream;
+    const int gw = std::max(1, std::min(ceil_div(A.n, 8), ctx.sm_count * 8));
+    DBuf<int> wlo(A.n), wspan(A.n), bad(1);
+    DBuf<unsigned long long> sums(2);
+    sums.zero(s);
+    bad.zero(s);
+    k_gather_cost<<<gw, 256, 0, s>>>(A.n, A.rp, A.ci, A.v, B.rp, B.ci, wlo.p, wspan.p, sums.p, bad.p);
+    HAMLSS_LAUNCH_CHECK();
+    unsigned long long h[2];
+    int hb = 0;
+    sums.download(h, 2, s);
+    bad.download(&hb, 1, s);
+    HAMLSS_CUDA(cudaStreamSynchronize(s));
+    if (hb || h[1] > kGatherMost || (h[1] > kGatherPairs && h[1] > kGatherRatio * h[0])) return false;
+    DBuf<double> Bd((size_t)B.n * B.m);
+    HAMLSS_CUDA(cudaMemsetAsync(Bd.p, 0, sizeof(double) * (size_t)B.n * B.m, s));
+    k_dense_rows<<<std::max(1, std::min(ceil_div(B.n, 8), ctx.sm_count * 8)), 256, 0, s>>>(B.n, B.rp, B.ci, B.v,
+                                                                                        B.m, Bd.p);
+    HAMLSS_LAUNCH_CHECK();
+    DBuf<int> off(A.n + 1), cnt(A.n);
+    HAMLSS_CUDA(cudaMemcpyAsync(off.p, wspan.p, sizeof(int) * (size_t)A.n, cudaMemcpyDeviceToDevice, s));
+    HAMLSS_CUDA(cudaMemsetAsync(off.p + A.n, 0, sizeof(int), s));
+    const long long total = exclusive_scan(ctx, off.p, A.n + 1);     // a slot a window column
+    if (total > INT_MAX) return false;
+    DBuf<int> wci(std::max(total, 1LL));
+    DBuf<double> wv(std::max(total, 1LL));
+    k_spgemm_gather<<<std::min(A.n, ctx.sm_count * 16), kGatherThreads, 0, s>>>(A.n, wlo.p, wspan.p, A.rp, A.ci, A.v,
+                                                                                Bd.p, B.m, cnt.p, off.p, wci.p, wv.p);
+    HAMLSS_LAUNCH_CHECK();
+    build_csr_counts(ctx, C, A.n, B.m, cnt);
+    k_spgemm_compact<<<std::max(1, std::min(ceil_div(A.n, 8), ctx.sm_count * 16)), 256, 0, s>>>(
+        A.n, off.p, cnt.p, wci.p, wv.p, C.rp.p, C.ci.p, C.v.p);
+    HAMLSS_LAUNCH_CHECK();
+    return true;
+}
+
 void spgemm(Ctx& ctx, const Csr<double>& A, const Csr<double>& B, DCsr& C) {
+    if (spgemm_gather(ctx, A, B, C)) return;
     cudaStream_t s = ctx.lane.stream;
     const int g = grid_for(ctx, A.n);
     DBuf<int> heads(3LL * std::max(A.nnz, 1));
@@ -2451,7 +2687,6 @@ std::unique_ptr<Prec> make_amg(Ctx& ctx, hamlss_mat* A, const hamlss_params& p) 
         M->Md.ensure((size_t)std::max(nc, 1) * std::max(nc, 1));
         M->piv.ensure(std::max(nc, 1));
         M->skip.ensure(std::max(nc, 1));
-        M->cwork.ensure(2 * std::max(nc, 1));
         HAMLSS_CUDA(cudaMemsetAsync(M->Md.p, 0, sizeof(double) * (size_t)nc * nc, s));
         if (nc) {
             k_csr_to_dense<<<std::max(1, std::min(ceil_div(nc, 8), ctx.sm_count * 8)), 256, 0, s>>>(
@@ -2468,15 +2703,29 @@ std::unique_ptr<Prec> make_amg(Ctx& ctx, hamlss_mat* A, const hamlss_params& p) 
             return M;
         }
         if (nc) {
-            k_dense_factor<<<1, 256, 0, s>>>(nc, M->Md.p, M->piv.p, M->skip.p);
-            HAMLSS_LAUNCH_CHECK();
+            DBuf<double> W((size_t)nc * nc);
+            HAMLSS_CUDA(cudaMemcpyAsync(W.p, M->Md.p, sizeof(double) * (size_t)nc * nc, cudaMemcpyDeviceToDevice, s));
+            static DeviceOnce raised;
+            raised(ctx.device, [] {
+                HAMLSS_CUDA(cudaFuncSetAttribute(k_dense_factor, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            });
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(kFactorBlocks);
+            cfg.blockDim = dim3(kFactorThreads);
+            cfg.stream = s;
+            cudaLaunchAttribute at{};
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = kFactorBlocks;
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            HAMLSS_CUDA(cudaLaunchKernelEx(&cfg, k_dense_factor, nc, W.p, M->Md.p, M->piv.p, M->skip.p));
         }
         phase(M->levels() - 1, "coarse LU");
         M->coarse_inverse = nc > 96;
         if (M->coarse_inverse) {
             M->Minv.ensure((size_t)nc * nc);
-            DBuf<double> work((size_t)nc * 2 * nc);
-            k_dense_inverse<<<nc, 32, 0, s>>>(nc, M->Md.p, M->piv.p, M->skip.p, work.p, M->Minv.p);
+            k_dense_inverse<<<nc, 32, dense_solve_smem(nc), s>>>(nc, M->Md.p, M->piv.p, M->skip.p, M->Minv.p);
             HAMLSS_LAUNCH_CHECK();
             HAMLSS_CUDA(cudaStreamSynchronize(s));
         }
