@@ -46,7 +46,12 @@ struct Batch {
     hamlss_params params{};
     std::vector<int> row_off;
     std::vector<BProb> hprob;
-    int width[kBatchClasses] = {32, 64, 128, 256};
+    // Default widths: about eight rows a thread in the smallest class, 32 in the largest.  A
+    // system is solved by its own team to the end, so a narrow team sets a batch's time
+    // however many systems wait beside it.  Measured, {32, 64, 128, 256} -> these: 384 systems
+    // of side 16-128 151 -> 36 ms, 2,048 of them 237 -> 140 ms, 2,000 of side 12-40 10.1 ->
+    // 6.0 ms, 100 of side 16-64 32 -> 8.4 ms ({256, 512, 512, 512}: 34, 140, 6.9, 6.7).
+    int width[kBatchClasses] = {128, 256, 512, 512};
     DBuf<int> rp, ci, dpos, lptrL, lordL, lptrU, lordU, pstatus, order, tickets;
     DBuf<double> v64, r64, xb, bb, xt;
     DBuf<float> v32, dinv, lu, work;
