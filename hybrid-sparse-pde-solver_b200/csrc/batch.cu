@@ -23,6 +23,7 @@ constexpr int kMaxPhases = kBatchClasses;
 
 struct Phase {
     int begin, end, width;              // systems order[begin, end), team width
+    int vec;                            // floats of a team's shared-memory vector (0: none)
 };
 
 struct BArgs {
@@ -36,12 +37,13 @@ struct BArgs {
     const double* v64;
     const float* v32;
     const float* dinv;
-    const float* lu;
-    const int* dpos;
     const int* lptrL;
-    const int* lordL;
     const int* lptrU;
-    const int* lordU;
+    const int2* infoL;
+    const int2* infoU;
+    const int2* entL;
+    const int2* entU;
+    const float* dgU;
     const int* pstatus;
     const double* b;
     double* x;
@@ -50,6 +52,7 @@ struct BArgs {
     hamlss_batch_result* out;
     double tol, inner_tol;
     int max_iter, max_outer, m;
+    int vec_at;                         // byte offset of the shared-memory vectors
 };
 
 // ------------------------------------------------------------------ shared layout
@@ -58,9 +61,15 @@ __host__ __device__ inline int team_stride(int W, int m) {
     const int R = m + 2;
     return (W / 32) * R + R + (m + 1) * m + 4 * m + 1 + 2;
 }
-inline size_t batch_smem(int W, int m) {
-    return sizeof(double) * (size_t)(kBatchThreads / W) * team_stride(W, m);
+inline size_t batch_team_smem(int W, int m) {
+    return (sizeof(double) * (size_t)(kBatchThreads / W) * team_stride(W, m) + 15) & ~(size_t)15;
 }
+// Largest system of a size class whose gathered vector (CG's p, the preconditioner's) a team
+// keeps in shared memory, and the most of it a block gives to these vectors.  (The rest stays
+// L1, which the rows' entries and the other vectors go through: with r and q in shared memory
+// too a 16,384-row CG system took 27 ms for 21, and two blocks an SM at 64 registers 27.)
+constexpr int kBatchVec[kBatchClasses] = {1024, 4096, 16384, 0};
+constexpr size_t kBatchVecBytes = 64 * 1024;
 
 struct Team {
     int W, lt, id, wit, R, m;
@@ -72,8 +81,9 @@ struct Team {
     double* g;
     double* y;
     int* slot;
+    float* vec;            // shared-memory vector, or null
 
-    __device__ void init(int width, int mm, double* smem) {
+    __device__ void init(int width, int mm, int vecn, double* smem, float* vecs) {
         W = width;
         m = mm;
         R = m + 2;
@@ -89,6 +99,7 @@ struct Team {
         g = sn + m;
         y = g + m + 1;
         slot = reinterpret_cast<int*>(y + m);
+        vec = vecn ? vecs + (size_t)id * vecn : nullptr;
     }
     // team barrier: a warp syncs itself; wider teams use named barrier id + 1 (0 is the
     // CTA barrier), at most kBatchThreads / 64 = 8 of them
@@ -121,12 +132,36 @@ __device__ __forceinline__ double row_ax64(int g, const BArgs& a, const double* 
     return s;
 }
 
-// FP32 row product over a local vector (column c lives at v[c - row0])
-__device__ __forceinline__ float row_ax32(int g, int row0, const BArgs& a, const float* v) {
-    float s = 0.f;
-    for (int k = __ldg(&a.rp[g]); k < __ldg(&a.rp[g + 1]); ++k)
-        s = __fmaf_rn(__ldg(&a.v32[k]), v[__ldg(&a.ci[k]) - row0], s);
-    return s;
+// FP32 products of rows i and i + W over a local vector (column c lives at v[c - row0]), in
+// column order each, five entries of both rows loaded before the first is used.
+constexpr int kRowPre = 5;
+struct RowPair {
+    float s0, s1;
+};
+template <typename V>
+__device__ __forceinline__ RowPair rows_ax32(int g0, int g1, bool two, int row0, const BArgs& a, const V& v) {
+    const int b0 = __ldg(&a.rp[g0]), e0 = __ldg(&a.rp[g0 + 1]);
+    int b1 = 0, e1 = 0;
+    if (two) {
+        b1 = __ldg(&a.rp[g1]);
+        e1 = __ldg(&a.rp[g1 + 1]);
+    }
+    int c0[kRowPre], c1[kRowPre];
+    float m0[kRowPre], m1[kRowPre];
+#pragma unroll
+    for (int k = 0; k < kRowPre; ++k) {
+        if (b0 + k < e0) { c0[k] = __ldg(&a.ci[b0 + k]) - row0; m0[k] = __ldg(&a.v32[b0 + k]); }
+        if (b1 + k < e1) { c1[k] = __ldg(&a.ci[b1 + k]) - row0; m1[k] = __ldg(&a.v32[b1 + k]); }
+    }
+    RowPair r{0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < kRowPre; ++k) {
+        if (b0 + k < e0) r.s0 = __fmaf_rn(m0[k], v[c0[k]], r.s0);
+        if (b1 + k < e1) r.s1 = __fmaf_rn(m1[k], v[c1[k]], r.s1);
+    }
+    for (int k = b0 + kRowPre; k < e0; ++k) r.s0 = __fmaf_rn(__ldg(&a.v32[k]), v[__ldg(&a.ci[k]) - row0], r.s0);
+    for (int k = b1 + kRowPre; k < e1; ++k) r.s1 = __fmaf_rn(__ldg(&a.v32[k]), v[__ldg(&a.ci[k]) - row0], r.s1);
+    return r;
 }
 
 // ---------------------------------------------------------------- inner PCG (FP32)
@@ -142,8 +177,7 @@ __device__ int inner_cg(const Team& T, const BArgs& a, const BProb& P, float* w,
                         int maxit) {
     const int n = P.n, r0 = P.row0;
     float* R = w;
-    float* Pa = w + n;
-    float* Pb = w + 2 * (size_t)n;
+    float* p = T.vec ? T.vec : w + n;
     float* Q = w + 3 * (size_t)n;
     float* D = w + 4 * (size_t)n;
     const CgZ z{R, P.method == BM_CG_JAC ? a.dinv + r0 : nullptr};
@@ -152,7 +186,7 @@ __device__ int inner_cg(const Team& T, const BArgs& a, const BProb& P, float* w,
         const float r = R[i];
         rz += (double)r * (double)z(i);
         rr += (double)r * (double)r;
-        Pa[i] = 0.f;
+        p[i] = 0.f;
     }
     T.put(rz, 0);
     T.put(rr, 1);
@@ -161,23 +195,33 @@ __device__ int inner_cg(const Team& T, const BArgs& a, const BProb& P, float* w,
     const double rn0 = sqrt(T.res[1]);
     if (!(rn0 > 0.0)) return 0;
     float beta = 0.f;
-    const float* pold = Pa;
-    float* pnew = Pb;
     int it = 0;
     while (it < maxit) {
-        // q = A p with p = z + beta p_old formed on the fly; p.q
-        double pq = 0.0;
-        for (int i = T.lt; i < n; i += T.W) {
-            const int g = r0 + i;
-            float s = 0.f;
-            for (int k = __ldg(&a.rp[g]); k < __ldg(&a.rp[g + 1]); ++k) {
-                const int j = __ldg(&a.ci[k]) - r0;
-                s = __fmaf_rn(__ldg(&a.v32[k]), __fmaf_rn(beta, pold[j], z(j)), s);
+        // p = z + beta p, then q = A p and p.q (gathering p alone: formed inside the product it
+        // cost three gathers an entry)
+        {
+            int i = T.lt;
+            for (; i + 3 * T.W < n; i += 4 * T.W) {
+                float zz[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) zz[u] = z(i + u * T.W);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) p[i + u * T.W] = __fmaf_rn(beta, p[i + u * T.W], zz[u]);
             }
-            const float pi = __fmaf_rn(beta, pold[i], z(i));
-            pnew[i] = pi;
-            Q[i] = s;
-            pq += (double)pi * (double)s;
+            for (; i < n; i += T.W) p[i] = __fmaf_rn(beta, p[i], z(i));
+        }
+        T.sync();
+        double pq = 0.0;
+        for (int i = T.lt; i < n; i += 2 * T.W) {
+            const int j = i + T.W;
+            const bool two = j < n;
+            const RowPair s = rows_ax32(r0 + i, r0 + j, two, r0, a, p);
+            Q[i] = s.s0;
+            pq += (double)p[i] * (double)s.s0;
+            if (two) {
+                Q[j] = s.s1;
+                pq += (double)p[j] * (double)s.s1;
+            }
         }
         T.put(pq, 0);
         T.finish(1);
@@ -186,12 +230,29 @@ __device__ int inner_cg(const Team& T, const BArgs& a, const BProb& P, float* w,
         const float af = (float)(rho / pq);
         rr = 0.0;
         rz = 0.0;
-        for (int i = T.lt; i < n; i += T.W) {
-            D[i] = __fmaf_rn(af, pnew[i], D[i]);
-            const float r = __fmaf_rn(-af, Q[i], R[i]);
-            R[i] = r;
-            rr += (double)r * (double)r;
-            rz += (double)r * (double)z(i);
+        for (int i0 = T.lt; i0 < n; i0 += 4 * T.W) {
+            float d[4], r[4], q[4], dv[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = i0 + u * T.W;
+                if (i < n) {
+                    d[u] = D[i];
+                    r[u] = R[i];
+                    q[u] = Q[i];
+                    dv[u] = z.dinv ? __ldg(&z.dinv[i]) : 1.f;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = i0 + u * T.W;
+                if (i < n) {
+                    D[i] = __fmaf_rn(af, p[i], d[u]);
+                    const float ri = __fmaf_rn(-af, q[u], r[u]);
+                    R[i] = ri;
+                    rr += (double)ri * (double)ri;
+                    rz += (double)ri * (double)(z.dinv ? __fmul_rn(dv[u], ri) : ri);
+                }
+            }
         }
         T.put(rr, 0);
         T.put(rz, 1);
@@ -202,51 +263,104 @@ __device__ int inner_cg(const Team& T, const BArgs& a, const BProb& P, float* w,
         if (!(fabs(rho) > 0.0)) break;
         beta = (float)(T.res[1] / rho);
         rho = T.res[1];
-        const float* t = pold;
-        pold = pnew;
-        pnew = const_cast<float*>(t);
     }
     return it;
 }
 
 // ------------------------------------------------------------- preconditioner (FP32)
-// z = M^-1 v for the FGMRES systems; ends with a team barrier.
-__device__ void bprec(const Team& T, const BArgs& a, const BProb& P, const float* v, float* z,
-                      float* Y) {
+// One triangular sweep in place on the team's vector x, level by level.  A level's rows read
+// only the vector (shared memory) behind the barrier: row, entries and diagonal of a thread's
+// first row are loaded two levels ahead, its bounds three (walking the pattern inside the
+// level, four dependent loads, took ~1.2 us a level).
+constexpr int kSweepPre = 2;
+struct SweepRow {
+    int row, e0, e1;       // row < 0: none
+    int2 en[kSweepPre];
+    float d;
+};
+
+template <bool DIV>
+__device__ __forceinline__ void bsweep(const Team& T, const int* __restrict__ lptr, int nlev,
+                                       const int2* __restrict__ info, const int2* __restrict__ ent,
+                                       const float* __restrict__ dg, float* x) {
+    auto solve = [&](const SweepRow& q) {
+        float s = x[q.row];
+#pragma unroll
+        for (int k = 0; k < kSweepPre; ++k)
+            if (q.e0 + k < q.e1) s = __fmaf_rn(-__int_as_float(q.en[k].y), x[q.en[k].x], s);
+        for (int e = q.e0 + kSweepPre; e < q.e1; ++e) {
+            const int2 en = __ldg(&ent[e]);
+            s = __fmaf_rn(-__int_as_float(en.y), x[en.x], s);
+        }
+        x[q.row] = DIV ? __fdiv_rn(s, q.d) : s;
+    };
+    // bounds of this thread's first row of level l
+    struct Place { int t, row, e0, e1; };
+    auto place = [&](int l) {
+        Place p{-1, -1, 0, 0};
+        if (l < nlev) {
+            const int t = __ldg(&lptr[l]) + T.lt;
+            if (t < __ldg(&lptr[l + 1])) {
+                const int2 a = __ldg(&info[t]);
+                p.t = t;
+                p.row = a.x;
+                p.e0 = a.y;
+                p.e1 = __ldg(&info[t + 1].y);
+            }
+        }
+        return p;
+    };
+    auto load = [&](const Place& p) {
+        SweepRow q;
+        q.row = p.row;
+        q.e0 = p.e0;
+        q.e1 = p.e1;
+        q.d = 1.f;
+        if (p.row >= 0) {
+#pragma unroll
+            for (int k = 0; k < kSweepPre; ++k)
+                if (p.e0 + k < p.e1) q.en[k] = __ldg(&ent[p.e0 + k]);
+            if (DIV) q.d = __ldg(&dg[p.t]);
+        }
+        return q;
+    };
+    SweepRow cur = load(place(0)), nx1 = load(place(1));
+    Place nx2 = place(2);
+    for (int l = 0; l < nlev; ++l) {
+        const SweepRow nn = load(nx2);
+        nx2 = place(l + 3);
+        if (cur.row >= 0) {
+            solve(cur);
+            const int e = __ldg(&lptr[l + 1]);
+            for (int t = __ldg(&lptr[l]) + T.lt + T.W; t < e; t += T.W) {     // rows beyond the team's width
+                const int2 a = __ldg(&info[t]);
+                solve(load(Place{t, a.x, a.y, __ldg(&info[t + 1].y)}));
+            }
+        }
+        T.sync();
+        cur = nx1;
+        nx1 = nn;
+    }
+}
+
+// z = M^-1 v for the FGMRES systems (Y: work vector, used where the team has no shared one);
+// ends with a team barrier.  Returns where the products A z should gather z from.
+__device__ const float* bprec(const Team& T, const BArgs& a, const BProb& P, const float* v, float* z, float* Y) {
     const int n = P.n, r0 = P.row0;
     if (P.method == BM_GM_ILU) {
-        // L y = v (unit lower, ilu.cpp:225-239), level by level
-        for (int l = 0; l < P.nlevL; ++l) {
-            const int b = __ldg(&a.lptrL[P.levL + l]), e = __ldg(&a.lptrL[P.levL + l + 1]);
-            for (int t = b + T.lt; t < e; t += T.W) {
-                const int g = __ldg(&a.lordL[t]);
-                float s = v[g - r0];
-                // columns are sorted, so the entries left of the diagonal are exactly c < g
-                const int d = __ldg(&a.dpos[g]);
-                for (int p = __ldg(&a.rp[g]); p < d; ++p)
-                    s = __fmaf_rn(-__ldg(&a.lu[p]), Y[__ldg(&a.ci[p]) - r0], s);
-                Y[g - r0] = s;
-            }
-            T.sync();
-        }
-        // U z = y (ilu.cpp:244-262), level by level
-        for (int l = 0; l < P.nlevU; ++l) {
-            const int b = __ldg(&a.lptrU[P.levU + l]), e = __ldg(&a.lptrU[P.levU + l + 1]);
-            for (int t = b + T.lt; t < e; t += T.W) {
-                const int g = __ldg(&a.lordU[t]);
-                const int d = __ldg(&a.dpos[g]);
-                float s = Y[g - r0];
-                for (int p = d + 1; p < __ldg(&a.rp[g + 1]); ++p)
-                    s = __fmaf_rn(-__ldg(&a.lu[p]), z[__ldg(&a.ci[p]) - r0], s);
-                z[g - r0] = __fdiv_rn(s, __ldg(&a.lu[d]));
-            }
-            T.sync();
-        }
-        return;
+        float* x = T.vec ? T.vec : Y;
+        for (int i = T.lt; i < n; i += T.W) x[i] = v[i];
+        T.sync();
+        bsweep<false>(T, a.lptrL + P.levL, P.nlevL, a.infoL, a.entL, nullptr, x);     // ilu.cpp:225-239
+        bsweep<true>(T, a.lptrU + P.levU, P.nlevU, a.infoU, a.entU, a.dgU, x);        // ilu.cpp:244-262
+        for (int i = T.lt; i < n; i += T.W) z[i] = x[i];
+        T.sync();
+        return x;
     }
     const float* dv = P.method == BM_GM_JAC ? a.dinv + r0 : nullptr;
     for (int i = T.lt; i < n; i += T.W) z[i] = dv ? __fmul_rn(__ldg(&dv[i]), v[i]) : v[i];
     T.sync();
+    return z;
 }
 
 // Team sums of V_k . w for k < nv (w read from W), staged in groups of kGroup.
@@ -286,7 +400,7 @@ __device__ int inner_gmres(const Team& T, const BArgs& a, const BProb& P, float*
         double bb = 0.0;
         for (int i = T.lt; i < n; i += T.W) {
             float s = R[i];
-            if (beta0 >= 0.0) s -= row_ax32(r0 + i, r0, a, D);
+            if (beta0 >= 0.0) s -= rows_ax32(r0 + i, 0, false, r0, a, D).s0;
             V[i] = s;
             bb += (double)s * (double)s;
         }
@@ -307,9 +421,13 @@ __device__ int inner_gmres(const Team& T, const BArgs& a, const BProb& P, float*
         for (int j = 0; j < m && it < maxit; ++j) {
             const float* Vj = V + (size_t)j * nn;
             float* Zj = Z + (size_t)j * nn;
-            bprec(T, a, P, Vj, Zj, Y);
+            const float* zj = bprec(T, a, P, Vj, Zj, Y);
             // w = A z_j ; h = V^T w
-            for (int i = T.lt; i < n; i += T.W) Wv[i] = row_ax32(r0 + i, r0, a, Zj);
+            for (int i = T.lt; i < n; i += 2 * T.W) {
+                const RowPair s = rows_ax32(r0 + i, r0 + i + T.W, i + T.W < n, r0, a, zj);
+                Wv[i] = s.s0;
+                if (i + T.W < n) Wv[i + T.W] = s.s1;
+            }
             multi_dot(T, V, nn, j + 1, Wv);
             if (T.lt <= j) T.H[T.lt * m + j] = T.res[T.lt];
             T.sync();
@@ -448,11 +566,11 @@ __device__ void solve_one(const Team& T, const BArgs& a, int k) {
     T.sync();
 }
 
-__global__ void __launch_bounds__(kBatchThreads) k_batch_solve(BArgs a) {
+__global__ void __launch_bounds__(kBatchThreads, 1) k_batch_solve(BArgs a) {
     extern __shared__ double smem[];
     for (int p = 0; p < a.nphase; ++p) {
         Team T;
-        T.init(a.ph[p].width, a.m, smem);
+        T.init(a.ph[p].width, a.m, a.ph[p].vec, smem, reinterpret_cast<float*>(reinterpret_cast<char*>(smem) + a.vec_at));
         const int cnt = a.ph[p].end - a.ph[p].begin;
         for (;;) {
             if (T.lt == 0) *T.slot = atomicAdd(&a.tickets[p], 1);
@@ -550,10 +668,33 @@ __global__ void k_batch_ilu(int nsys, const int* __restrict__ sys, const BProb* 
     }
 }
 
-__global__ void k_d2f_batch(const double* __restrict__ a, float* b, long long n) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x)
-        b[i] = (float)a[i];
+// A triangle's rows in level order: entries of row ord[t] counted (FILL = false), or written
+// from first[t] on with the row's place (and U's diagonal, 1 where absent).
+template <bool LOWER, bool FILL>
+__global__ void k_batch_pack(int rows, const int* __restrict__ ord, const int* __restrict__ prow,
+                             const BProb* __restrict__ prob, const int* __restrict__ rp, const int* __restrict__ ci,
+                             const double* __restrict__ lu, int* first, int2* info, int2* ent, float* dg) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t <= rows; t += gridDim.x * blockDim.x) {
+        if (t == rows) {
+            if (FILL) info[t] = make_int2(0, first[t]);
+            else first[t] = 0;
+            continue;
+        }
+        const int i = ord[t], row0 = prob[prow[i]].row0;
+        int o = FILL ? first[t] : 0;
+        if (FILL) info[t] = make_int2(i - row0, o);
+        float d = 1.f;
+        for (int p = rp[i]; p < rp[i + 1]; ++p) {
+            const int j = ci[p];
+            if (FILL && j == i) d = (float)lu[p];
+            if (LOWER ? j < i : j > i) {
+                if (FILL) ent[o] = make_int2(j - row0, __float_as_int((float)lu[p]));
+                ++o;
+            }
+        }
+        if (FILL && !LOWER) dg[t] = d;
+        if (!FILL) first[t] = o;
+    }
 }
 
 int klass_of(int n) {
@@ -595,6 +736,7 @@ std::unique_ptr<Batch> batch_create(Ctx& ctx, hamlss_ctx* h, int count, const in
     B->params = p;
     B->row_off.assign(row_off, row_off + count + 1);
     cudaStream_t s = ctx.lane.stream;
+    AllocScope scope(s);                 // buffers from the stream-ordered pool
     const int N = B->N;
     // structure
     B->rp.ensure(N + 1);
@@ -671,7 +813,6 @@ std::unique_ptr<Batch> batch_create(Ctx& ctx, hamlss_ctx* h, int count, const in
     if (hbad != INT_MAX)
         fail(HAMLSS_ERR_MALFORMED, "batch: row " + std::to_string(hbad) + " reaches outside its system");
     // ILU(0) of the ILU systems
-    B->lu.ensure(std::max(nnz, 1));
     if (any_ilu) {
         DBuf<int> dpos2, lvL, lvU;
         int nlL = 0, nlU = 0;
@@ -709,13 +850,12 @@ std::unique_ptr<Batch> batch_create(Ctx& ctx, hamlss_ctx* h, int count, const in
         HAMLSS_LAUNCH_CHECK();
         long long rowsL = exclusive_scan(ctx, B->lptrL.p, (int)tl + 1);
         exclusive_scan(ctx, B->lptrU.p, (int)tu + 1);
-        B->lordL.ensure(std::max<long long>(rowsL, 1));
-        B->lordU.ensure(std::max<long long>(rowsL, 1));
+        DBuf<int> lordL(std::max<long long>(rowsL, 1)), lordU(std::max<long long>(rowsL, 1));
         DBuf<int> fL(tl + 1), fU(tu + 1);
         HAMLSS_CUDA(cudaMemcpyAsync(fL.p, B->lptrL.p, sizeof(int) * (tl + 1), cudaMemcpyDeviceToDevice, s));
         HAMLSS_CUDA(cudaMemcpyAsync(fU.p, B->lptrU.p, sizeof(int) * (tu + 1), cudaMemcpyDeviceToDevice, s));
-        k_level_bucket<true><<<g, 256, 0, s>>>(N, prow.p, B->prob.p, lvL.p, lvU.p, fL.p, fU.p, B->lordL.p,
-                                               B->lordU.p);
+        k_level_bucket<true><<<g, 256, 0, s>>>(N, prow.p, B->prob.p, lvL.p, lvU.p, fL.p, fU.p, lordL.p,
+                                               lordU.p);
         HAMLSS_LAUNCH_CHECK();
         DBuf<double> lu64(std::max(nnz, 1));
         if (nnz)
@@ -725,17 +865,29 @@ std::unique_ptr<Batch> batch_create(Ctx& ctx, hamlss_ctx* h, int count, const in
         std::vector<int> zinit(count, INT_MAX);
         zp.upload(zinit.data(), count, s);
         k_batch_ilu<<<std::min<int>((int)sys.size(), ctx.sm_count * 16), 256, 0, s>>>(
-            (int)sys.size(), dsys.p, B->prob.p, B->lptrL.p, B->lordL.p, B->rp.p, B->ci.p, B->dpos.p, lu64.p,
+            (int)sys.size(), dsys.p, B->prob.p, B->lptrL.p, lordL.p, B->rp.p, B->ci.p, B->dpos.p, lu64.p,
             zp.p, B->pstatus.p);
         HAMLSS_LAUNCH_CHECK();
-        if (nnz) k_d2f_batch<<<g, 256, 0, s>>>(lu64.p, B->lu.p, nnz);
+        // the factors in level order
+        const int rows = (int)rowsL;
+        DBuf<int> first(rows + 1);
+        B->infoL.ensure(rows + 1);
+        B->infoU.ensure(rows + 1);
+        B->dgU.ensure(std::max(rows, 1));
+        k_batch_pack<true, false><<<g, 256, 0, s>>>(rows, lordL.p, prow.p, B->prob.p, B->rp.p, B->ci.p, lu64.p,
+                                                    first.p, nullptr, nullptr, nullptr);
+        HAMLSS_LAUNCH_CHECK();
+        B->entL.ensure(std::max(exclusive_scan(ctx, first.p, rows + 1), 1LL));
+        k_batch_pack<true, true><<<g, 256, 0, s>>>(rows, lordL.p, prow.p, B->prob.p, B->rp.p, B->ci.p, lu64.p,
+                                                   first.p, B->infoL.p, B->entL.p, nullptr);
+        k_batch_pack<false, false><<<g, 256, 0, s>>>(rows, lordU.p, prow.p, B->prob.p, B->rp.p, B->ci.p, lu64.p,
+                                                     first.p, nullptr, nullptr, nullptr);
+        HAMLSS_LAUNCH_CHECK();
+        B->entU.ensure(std::max(exclusive_scan(ctx, first.p, rows + 1), 1LL));
+        k_batch_pack<false, true><<<g, 256, 0, s>>>(rows, lordU.p, prow.p, B->prob.p, B->rp.p, B->ci.p, lu64.p,
+                                                    first.p, B->infoU.p, B->entU.p, B->dgU.p);
         HAMLSS_LAUNCH_CHECK();
         HAMLSS_CUDA(cudaStreamSynchronize(s));
-    } else {
-        B->lptrL.ensure(1);
-        B->lptrU.ensure(1);
-        B->lordL.ensure(1);
-        B->lordU.ensure(1);
     }
     // schedule: classes largest first, longest system first inside a class
     std::vector<int> ord(count);
@@ -767,12 +919,15 @@ double batch_run(Ctx& ctx, Batch& B, const double* b, double* x, unsigned class_
     a.nphase = 0;
     std::vector<int> per(kBatchClasses, 0);
     for (const auto& P : B.hprob) per[P.klass]++;
-    int wmin = kBatchThreads;
+    size_t team_bytes = 0, vec_bytes = 0;
     for (int c = kBatchClasses - 1; c >= 0; --c) {
         if (!per[c]) continue;
         if (class_mask & (1u << c)) {
-            a.ph[a.nphase++] = Phase{pos, pos + per[c], B.width[c]};
-            wmin = std::min(wmin, B.width[c]);
+            const int teams = kBatchThreads / B.width[c];
+            const int vec = sizeof(float) * (size_t)teams * kBatchVec[c] <= kBatchVecBytes ? kBatchVec[c] : 0;
+            a.ph[a.nphase++] = Phase{pos, pos + per[c], B.width[c], vec};
+            team_bytes = std::max(team_bytes, batch_team_smem(B.width[c], B.m));
+            vec_bytes = std::max(vec_bytes, sizeof(float) * (size_t)teams * vec);
         }
         pos += per[c];
     }
@@ -785,12 +940,13 @@ double batch_run(Ctx& ctx, Batch& B, const double* b, double* x, unsigned class_
     a.v64 = B.v64.p;
     a.v32 = B.v32.p;
     a.dinv = B.dinv.p;
-    a.lu = B.lu.p;
-    a.dpos = B.dpos.p;
     a.lptrL = B.lptrL.p;
-    a.lordL = B.lordL.p;
     a.lptrU = B.lptrU.p;
-    a.lordU = B.lordU.p;
+    a.infoL = B.infoL.p;
+    a.infoU = B.infoU.p;
+    a.entL = B.entL.p;
+    a.entU = B.entU.p;
+    a.dgU = B.dgU.p;
     a.pstatus = B.pstatus.p;
     a.b = b;
     a.x = x;
@@ -802,7 +958,8 @@ double batch_run(Ctx& ctx, Batch& B, const double* b, double* x, unsigned class_
     a.max_iter = B.params.max_iter;
     a.max_outer = B.params.ir_max_outer;
     a.m = B.m;
-    const size_t smem = batch_smem(wmin, B.m);
+    a.vec_at = (int)team_bytes;
+    const size_t smem = team_bytes + vec_bytes;
     static DeviceOnce raised;            // the device's opt-in maximum, so no call lowers it
     raised(ctx.device, [&] {
         int optin = 0;

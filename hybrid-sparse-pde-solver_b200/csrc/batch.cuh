@@ -9,7 +9,9 @@
 //   the batch is one block-diagonal CSR: system k owns rows [row_off[k], row_off[k+1]) and
 //   its entries' columns lie in the same range (checked); int32 indices, FP64 values and an
 //   FP32 copy.  Per-row: the diagonal position, w/a_ii in FP32, and for ILU systems the
-//   FP32 factor values in A's pattern plus the rows of every system grouped by level.
+//   FP32 factors with the rows of every system grouped by level, L's and U's entries in that
+//   order.  A team keeps the vector its products and sweeps gather from (CG's p, the
+//   preconditioner's work vector) in shared memory where its size class fits.
 //   Per-system FP32 work vectors are laid end to end (CG 5n, FGMRES (2m+5)n floats).
 // Arithmetic: FP32 values, vectors and SpMV inside an FP64 iterative-refinement loop per
 // system (FP64 residual b - A x with FP64 values, x += ||r|| d in FP64); dot products
@@ -52,9 +54,11 @@ struct Batch {
     // of side 16-128 151 -> 36 ms, 2,048 of them 237 -> 140 ms, 2,000 of side 12-40 10.1 ->
     // 6.0 ms, 100 of side 16-64 32 -> 8.4 ms ({256, 512, 512, 512}: 34, 140, 6.9, 6.7).
     int width[kBatchClasses] = {128, 256, 512, 512};
-    DBuf<int> rp, ci, dpos, lptrL, lordL, lptrU, lordU, pstatus, order, tickets;
+    DBuf<int> rp, ci, dpos, lptrL, lptrU, pstatus, order, tickets;
+    DBuf<int2> infoL, infoU, entL, entU;   // ILU rows in level order: (local row, first entry),
+                                           // entries (local column, value bits)
     DBuf<double> v64, r64, xb, bb, xt;
-    DBuf<float> v32, dinv, lu, work;
+    DBuf<float> v32, dinv, dgU, work;
     DBuf<BProb> prob;
     DBuf<hamlss_batch_result> out;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
