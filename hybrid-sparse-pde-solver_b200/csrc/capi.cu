@@ -485,6 +485,8 @@ int hamlss_precond_apply(hamlss_ctx* ctx, const hamlss_prec* M, const double* r,
         M->p->apply(c, c.lane, dr, dz, nullptr);
         if (where == HAMLSS_HOST) ws.d[7].download(z, n, s);
         HAMLSS_CUDA(cudaStreamSynchronize(s));
+        if (lane_take_timeout(c.lane))
+            return set_err(HAMLSS_ERR_TIMEOUT, "a preconditioner kernel gave up waiting for its bulk copies");
         return HAMLSS_OK;
     });
 }
@@ -662,7 +664,7 @@ int hamlss_solve(hamlss_ctx* ctx, int solver, const hamlss_mat* A, const hamlss_
         if (r.status != HAMLSS_OK)
             return set_err(r.status, "non-finite values met during the solve");
         if (lane_take_timeout(c.lane))
-            return set_err(HAMLSS_ERR_TIMEOUT, "an SpMV gave up waiting for its bulk copies");
+            return set_err(HAMLSS_ERR_TIMEOUT, "a kernel of the solve gave up a bounded wait");
         return HAMLSS_OK;
     });
 }
@@ -757,6 +759,8 @@ int hamlss_solve_adaptive(hamlss_ctx* ctx, const hamlss_mat* A, const double* b,
         if (n_log) *n_log = nlog;
         if (where == HAMLSS_HOST) Am->ws.d[7].download(x, A->A.n, s);
         HAMLSS_CUDA(cudaStreamSynchronize(s));
+        if (lane_take_timeout(c.lane))
+            return set_err(HAMLSS_ERR_TIMEOUT, "a kernel of the solve gave up a bounded wait");
         return HAMLSS_OK;
     });
 }

@@ -289,7 +289,7 @@ k_cg_persist(PersistArgs<T> a, State* gs, Fin fin) {
     }
     if (CLUSTER) cooperative_groups::this_cluster().sync();   // no block leaves while sums are stored into it
     if (tid == 0) {
-        if (!ok && a.err) atomicExch(a.err, 1);
+        if (!ok) raise_word(a.err);
         if (blockIdx.x == 0) {
             if (!ok) fin.timeout(&S);
             *gs = S;

@@ -26,17 +26,16 @@ void lane_init(Lane& L, int sm_count) {
     L.red_cap = (size_t)std::max(sm_count, 1) * kMaxBlocksPerSm * kMaxRed;
     L.partials.alloc(L.red_cap);
     L.err.alloc(1);
-    L.err.zero(L.stream);
+    *L.err.p = 0;
     L.ticket.alloc(1);
     L.ticket.zero(L.stream);
 }
 
 bool lane_take_timeout(const Lane& L) {
-    int e = 0;
-    HAMLSS_CUDA(cudaMemcpyAsync(&e, L.err.p, sizeof(int), cudaMemcpyDeviceToHost, L.stream));
-    HAMLSS_CUDA(cudaStreamSynchronize(L.stream));
-    if (e) HAMLSS_CUDA(cudaMemsetAsync(L.err.p, 0, sizeof(int), L.stream));
-    return e != 0;
+    volatile int* e = L.err.p;
+    const bool out = *e != 0;
+    if (out) *e = 0;
+    return out;
 }
 
 void lane_destroy(Lane& L) {
@@ -47,7 +46,6 @@ void lane_destroy(Lane& L) {
     }
     L.partials.release();
     L.ticket.release();
-    L.err.release();
     L.sums.release();
 }
 

@@ -64,7 +64,8 @@ struct Lane {
     DBuf<double> partials;
     DBuf<unsigned> ticket;
     size_t red_cap = 0;       // entries of `partials`
-    DBuf<int> err;            // set by a kernel whose bounded wait ran out (zero otherwise)
+    HBuf<int> err;            // set by a kernel whose bounded wait ran out (zero otherwise); in
+                              // pinned host memory, so reading it costs no copy
     DBuf<double> sums;        // block sums and barrier counter of a persistent kernel (cg_persist.cuh)
     Profiler* prof = nullptr;
     Reducer red() const { return Reducer{partials.p, ticket.p}; }
@@ -118,8 +119,9 @@ constexpr int kMaxRed = 72;   // widest reduction (multi-dot of an FGMRES basis 
 
 void lane_init(Lane& L, int sm_count);
 void lane_destroy(Lane& L);
-// Whether a bulk-copy SpMV on the lane gave up waiting for its copies since the last call
-// (it then read the matrix from global memory, so its results stand); clears the word.
+// Whether a kernel on the lane gave up a bounded wait since the last call; clears the word.
+// The caller has synchronised the lane's stream.  (A bulk-copy SpMV then read the matrix from
+// global memory, so its results stand; a triangular sweep's or persistent iteration's do not.)
 bool lane_take_timeout(const Lane& L);
 // The matrix's row-length profile for hamlss_spmv: when its longest row has more than
 // kSkewRow entries and more than kSkewRatio times the average, the rows above

@@ -195,7 +195,7 @@ k_tri_sweep(TriView<T> F, const T* __restrict__ rhs, T* out, const int* gate, in
             if (!mbar_try_wait(&full[blk % NB], phase) && !mbar_wait_bounded(&full[blk % NB], phase)) {
                 tid = 1 << 30;            // no rows for this thread from here on
                 s_stop = 1;
-                if (err) atomicExch(err, 1);
+                raise_word(err);
             }
             landed += RB;
         }

@@ -75,6 +75,11 @@ __device__ __forceinline__ void l2_prefetch_rows(const T* v, int r0, int r1) {
     if (v && r1 > r0) l2_prefetch(v + r0, (size_t)(r1 - r0) * sizeof(T));
 }
 
+// Sets a lane's error word (pinned host memory).
+__device__ __forceinline__ void raise_word(int* err) {
+    if (err) *(volatile int*)err = 1;
+}
+
 struct NoFin {
     template <int NV>
     __device__ void operator()(const double (&)[NV]) const {}

@@ -233,7 +233,7 @@ k_spmv_stream(int n, const int* __restrict__ rp, const int* __restrict__ ci, con
                 if constexpr (has_prefetch<Epi>::value) epi_l.prefetch(r0, r1);
                 *staged = w + 1;
             } else {
-                if (err) atomicExch(err, 1);
+                raise_word(err);
                 *stop = 1;
             }
         }
@@ -243,7 +243,7 @@ k_spmv_stream(int n, const int* __restrict__ rp, const int* __restrict__ ci, con
             const long long t0 = clock64();
             while (u >= *staged && !*stop) {
                 if (clock64() - t0 > (1ll << 31)) {
-                    if (err) atomicExch(err, 1);
+                    raise_word(err);
                     *stop = 1;
                     break;
                 }
@@ -255,7 +255,7 @@ k_spmv_stream(int n, const int* __restrict__ rp, const int* __restrict__ ci, con
         if (landed) {                     // phase u / S of stage s; bounded (~1 s)
             landed = mbar_wait_bounded(&full[s], (unsigned)((u / S) & 1));
             if (!landed) {
-                if (err) atomicExch(err, 1);
+                raise_word(err);
                 *stop = 1;
             }
         }
