@@ -709,7 +709,7 @@ struct IlutArgs {
     double* eval;
     int* lcnt;
     int* ucnt;
-    int* done;
+    unsigned long long* done;            // of a finished row: U's first slot, its entries << 32; else 0
     int* ticket;
     int* err;                            // 1 bounded wait ran out, 2 work row overflow
     int* finished;                       // rows published so far
@@ -901,32 +901,45 @@ __global__ void __launch_bounds__(32 * kIlutWarps) k_ilut_rows(IlutArgs a) {
                 __syncwarp();
                 continue;
             }
-            // row k must be finished
+            // row k must be finished: its published word says where its U entries are.  Row i
+            // usually waits for row i - 1, so this wait, and what follows it, is the chain that
+            // bounds the factorisation: one load a poll (progress and errors are looked at
+            // every 32nd), and the pivot comes with the first 32 entries instead of before them
+            unsigned long long at = 0;
             if (lane == 0) {
-                const volatile int* d = a.done + k;
-                if (*d == 0) {
+                const volatile unsigned long long* d = a.done + k;
+                at = *d;
+                if (at == 0) {
                     int seen = *(volatile int*)a.finished;
                     long long t0 = clock64();
-                    while (*d == 0) {
-                        if (*(volatile int*)a.err) break;
-                        const int now = *(volatile int*)a.finished;
-                        if (now != seen) {
-                            seen = now;
-                            t0 = clock64();
-                        } else if (clock64() - t0 > kIlutWaitCycles) {
-                            atomicExch(a.err, 1);
-                            break;
+                    for (int poll = 1; (at = *d) == 0; ++poll) {
+                        if ((poll & 31) == 0) {
+                            if (*(volatile int*)a.err) break;
+                            const int now = *(volatile int*)a.finished;
+                            if (now != seen) {
+                                seen = now;
+                                t0 = clock64();
+                            } else if (clock64() - t0 > kIlutWaitCycles) {
+                                atomicExch(a.err, 1);
+                                break;
+                            }
                         }
-                        __nanosleep(64);
+                        __nanosleep(20);
                     }
                 }
                 __threadfence();
             }
-            __syncwarp();
-            const int kk = __ldcg(&a.rp[k + 1]) - __ldcg(&a.rp[k]) + a.fill_p;
-            const int us = __ldcg(&a.off[k]) + (kk > 1 ? kk : 1);
-            const int ul = __ldcg(&a.ucnt[k]);
-            const double ukk = (ul > 0 && __ldcg(&a.ecol[us]) == k) ? __ldcg(&a.eval[us]) : 0.0;
+            at = __shfl_sync(0xffffffffu, at, 0);
+            const int us = (int)(unsigned)at, ul = (int)(at >> 32);       // (a wait that ran out: no entries)
+            int j0 = -1;
+            double u0 = 0.0;
+            if (lane < ul) {
+                j0 = __ldcg(&a.ecol[us + lane]);
+                u0 = __ldcg(&a.eval[us + lane]);
+            }
+            const int jd = __shfl_sync(0xffffffffu, j0, 0);
+            const double ud = __shfl_sync(0xffffffffu, u0, 0);
+            const double ukk = jd == k ? ud : 0.0;
             if (fabs(ukk) < 2.220446049250313e-16) {
                 __syncwarp();
                 if (lane == 0) sact[sk] = 0;
@@ -942,9 +955,9 @@ __global__ void __launch_bounds__(32 * kIlutWarps) k_ilut_rows(IlutArgs a) {
                 int j = -1;
                 double prod = 0.0;
                 if (q < ul) {
-                    j = __ldcg(&a.ecol[us + q]);
+                    j = q0 ? __ldcg(&a.ecol[us + q]) : j0;
                     if (j <= k) j = -1;
-                    else prod = __dmul_rn(lik, __ldcg(&a.eval[us + q]));
+                    else prod = __dmul_rn(lik, q0 ? __ldcg(&a.eval[us + q]) : u0);
                 }
                 int slot = -1;
                 if (j >= 0)
@@ -981,18 +994,9 @@ __global__ void __launch_bounds__(32 * kIlutWarps) k_ilut_rows(IlutArgs a) {
                 __syncwarp();
             }
         }
-        // collect L and U (the warp gathers and sorts by column; lane 0 applies the fill
-        // limit, a sequential heap select) and publish the row
-        int nl = ilut_gather_sorted(scol, sval, sact, nt, i, tau, true, row, lane);
-        if (lane == 0) ilut_keep(row, &nl, keep);
-        nl = __shfl_sync(0xffffffffu, nl, 0);
-        __syncwarp();
+        // collect U and L (the warp gathers and sorts by column; lane 0 applies the fill
+        // limit, a sequential heap select): U first, since later rows wait for it alone
         const int o = a.off[i];
-        for (int t = lane; t < nl; t += 32) {
-            a.ecol[o + t] = row[t].col;
-            a.eval[o + t] = row[t].val;
-        }
-        __syncwarp();                                  // row[] is reused for U
         double diag = 0.0;
         for (int b0 = 0; b0 < nt; b0 += 32) {
             const int t = b0 + lane;
@@ -1015,16 +1019,25 @@ __global__ void __launch_bounds__(32 * kIlutWarps) k_ilut_rows(IlutArgs a) {
             a.ecol[o + half + t] = row[t].col;
             a.eval[o + half + t] = row[t].val;
         }
+        __threadfence();                               // every lane's entries, then the word
+        __syncwarp();
+        if (lane == 0) {
+            *(volatile unsigned long long*)(a.done + i) = (unsigned long long)nu << 32 | (unsigned)(o + half);
+            atomicAdd(a.finished, 1);
+        }
+        __syncwarp();                                  // row[] is reused for L
+        int nl = ilut_gather_sorted(scol, sval, sact, nt, i, tau, true, row, lane);
+        if (lane == 0) ilut_keep(row, &nl, keep);
+        nl = __shfl_sync(0xffffffffu, nl, 0);
+        __syncwarp();
+        for (int t = lane; t < nl; t += 32) {
+            a.ecol[o + t] = row[t].col;
+            a.eval[o + t] = row[t].val;
+        }
         if (lane == 0) {
             a.lcnt[i] = nl;
             a.ucnt[i] = nu;
             if (overflow) atomicExch(a.err, 2);
-        }
-        __threadfence();                               // every lane's entries, then the flag
-        __syncwarp();
-        if (lane == 0) {
-            *(volatile int*)(a.done + i) = 1;
-            atomicAdd(a.finished, 1);
         }
         __syncwarp();
     }
@@ -1298,7 +1311,8 @@ std::unique_ptr<Prec> make_ilut(Ctx& ctx, hamlss_mat* A, double drop_tol, int fi
     AllocScope scope(s);
     const int g = std::max(1, std::min(ceil_div(n, 256), ctx.sm_count * 8));
     // capacity layout: row i owns 2 * max(row length + fill_p, 1) slots
-    DBuf<int> off(n + 1), lcnt(std::max(n, 1)), ucnt(std::max(n, 1)), done(std::max(n, 1)), flags(3);
+    DBuf<int> off(n + 1), lcnt(std::max(n, 1)), ucnt(std::max(n, 1)), flags(3);
+    DBuf<unsigned long long> done(std::max(n, 1));
     HAMLSS_CUDA(cudaMemsetAsync(off.p + n, 0, sizeof(int), s));
     if (n) k_ilut_caps<<<g, 256, 0, s>>>(n, A->A.rp.p, fill_p, off.p);
     HAMLSS_LAUNCH_CHECK();
