@@ -46,7 +46,13 @@ namespace hamlss {
 constexpr int kTriRing = 4096;            // solution values kept (positions); slot kTriRing holds 0
 constexpr int kTriSteps = 512;            // step bounds kept in shared memory at a time (even)
 
-template <typename T, int K, bool DIV>
+// What a step does with a row: FORWARD s = rhs - sum v y, BACKWARD the same divided by the
+// diagonal, FACTOR the ILU(0) elimination of a row whose lower entries each update only its
+// diagonal (five-point grids): l_k = v_k / d_k, d = a_ii - sum l_k u_k, with d_k the earlier
+// rows' diagonals (the ring) and u_k the matrix's own upper entries.
+enum class TriOp { FORWARD, BACKWARD, FACTOR };
+
+template <typename T, int K, TriOp OP>
 struct TriShape {
     // rows in the ring, and a refill of it
     static constexpr int RR = K <= 2 ? 4096 : K <= 4 ? 2048 : K <= 8 ? 1024 : 512;
@@ -55,7 +61,9 @@ struct TriShape {
     static constexpr int cap = (RR - RB) / 2 / 32 * 32;
     static constexpr int most = K <= 2 ? 864 : 416;                    // leaves 72 or 144 registers a thread
     static constexpr int max_rows = cap < most ? cap : most;           // rows a step
-    static constexpr size_t row_bytes = K * (sizeof(T) + 4) + (DIV ? 3 : 1) * sizeof(T);
+    // T's a row beside its entries' values: diagonal and reciprocal, or the upper entries
+    static constexpr int extra = OP == TriOp::BACKWARD ? 2 : OP == TriOp::FACTOR ? K : 0;
+    static constexpr size_t row_bytes = K * (sizeof(T) + 4) + (extra + 1) * sizeof(T);
     static constexpr size_t ring_bytes = (kTriRing + 16) * sizeof(T);
     static constexpr size_t smem_bytes = ring_bytes + RR * row_bytes + 4 * (kTriSteps + 4);
     static_assert(max_rows >= 32 && smem_bytes <= 227 * 1024 - 256, "ring shape");
@@ -68,7 +76,11 @@ struct TriView {
     const int* sptr;                      // nsteps + 1: step s holds rows [sptr[s], sptr[s + 1])
     const T* val;                         // [row][place]
     const int* code;                      // [row][place]
-    const T* dg;                          // [row]: diagonal, its reciprocal (DIV)
+    const T* dg;                          // [row]: diagonal, its reciprocal (BACKWARD), or
+                                          // [row][place] upper entries (FACTOR)
+    T* low;                               // FACTOR: [row][place] eliminated entries
+    const int* order;                     // FACTOR: the row at each position
+    int* status;                          // FACTOR: the smallest row with a vanishing pivot
 };
 
 template <typename T>
@@ -124,10 +136,10 @@ __device__ __forceinline__ T div_by(T s, T d, T r) {
     return s / d;
 }
 
-template <typename T, int K>
+template <typename T, int K, int EXTRA>
 struct TriRow {
     T rv;
-    alignas(16) T d[2];
+    alignas(16) T d[EXTRA > 0 ? EXTRA : 1];
     alignas(16) int c[K];                 // byte offset of the value in the ring, or ~position
     alignas(16) T v[K];
 };
@@ -145,11 +157,12 @@ __device__ __forceinline__ void load_packed(X (&dst)[COUNT], const X* src) {
 }
 
 // FAR: the triangle has entries beyond the ring.
-template <typename T, int K, bool DIV, bool FAR>
-__global__ void __launch_bounds__(TriShape<T, K, DIV>::max_rows + 32, 1)
+template <typename T, int K, TriOp OP, bool FAR>
+__global__ void __launch_bounds__(TriShape<T, K, OP>::max_rows + 32, 1)
 k_tri_sweep(TriView<T> F, const T* __restrict__ rhs, T* out, const int* gate, int* err) {
-    using S = TriShape<T, K, DIV>;
-    constexpr int RR = S::RR, RB = S::RB, NB = S::NB;
+    using S = TriShape<T, K, OP>;
+    constexpr int RR = S::RR, RB = S::RB, NB = S::NB, EX = S::extra;
+    using Row = TriRow<T, K, EX>;
     extern __shared__ __align__(128) unsigned char tri_smem[];
     __shared__ uint64_t full[NB];
     __shared__ int s_stop;
@@ -158,7 +171,7 @@ k_tri_sweep(TriView<T> F, const T* __restrict__ rhs, T* out, const int* gate, in
     T* s_val = reinterpret_cast<T*>(tri_smem + S::ring_bytes);
     T* s_rhs = s_val + RR * K;
     T* s_dg = s_rhs + RR;
-    int* s_code = reinterpret_cast<int*>(s_dg + (DIV ? 2 * RR : 0));
+    int* s_code = reinterpret_cast<int*>(s_dg + EX * RR);
     int* s_ptr = s_code + RR * K;                                      // bounds of steps sbase ..
     const int NT = (int)blockDim.x - 32;                               // rows a step
     const bool rows = (int)threadIdx.x < NT;
@@ -170,10 +183,10 @@ k_tri_sweep(TriView<T> F, const T* __restrict__ rhs, T* out, const int* gate, in
         for (; issued < nblk && (issued - NB + 1) * RB <= row0; ++issued) {
             const int slot = issued % NB, r0 = issued * RB, q0 = slot * RB;
             const unsigned nr = (unsigned)((min(RB, F.n - r0) + 3) & ~3);
-            mbar_arrive_tx(&full[slot], nr * (unsigned)sizeof(T) + (unsigned)(RB * (K * (sizeof(T) + 4) + (DIV ? 2 : 0) * sizeof(T))));
+            mbar_arrive_tx(&full[slot], nr * (unsigned)sizeof(T) + (unsigned)(RB * (K * (sizeof(T) + 4) + EX * sizeof(T))));
             bulk_load(s_val + q0 * K, F.val + (size_t)r0 * K, RB * K * sizeof(T), &full[slot]);
             bulk_load(s_code + q0 * K, F.code + (size_t)r0 * K, RB * K * 4, &full[slot]);
-            if (DIV) bulk_load(s_dg + q0 * 2, F.dg + (size_t)r0 * 2, RB * 2 * sizeof(T), &full[slot]);
+            if (EX) bulk_load(s_dg + q0 * EX, F.dg + (size_t)r0 * EX, RB * EX * sizeof(T), &full[slot]);
             bulk_load(s_rhs + q0, rhs + r0, nr * (unsigned)sizeof(T), &full[slot]);
         }
     };
@@ -181,7 +194,7 @@ k_tri_sweep(TriView<T> F, const T* __restrict__ rhs, T* out, const int* gate, in
         for (int k = 0; k < NB; ++k) mbar_init(&full[k], 1);
         mbar_fence_init();
         s_stop = 0;
-        *reinterpret_cast<T*>(ring + kTriRing * sizeof(T)) = T(0);
+        *reinterpret_cast<T*>(ring + kTriRing * sizeof(T)) = T(OP == TriOp::FACTOR ? 1 : 0);
     }
     __syncthreads();
     if (producer) refill(0);
@@ -200,16 +213,29 @@ k_tri_sweep(TriView<T> F, const T* __restrict__ rhs, T* out, const int* gate, in
             landed += RB;
         }
     };
-    auto load_row = [&](TriRow<T, K>& q, int t) {
+    auto load_row = [&](Row& q, int t) {
         const int r = t & (RR - 1);
         load_packed<K>(q.c, s_code + r * K);
         load_packed<K>(q.v, s_val + r * K);
         q.rv = s_rhs[r];
-        if (DIV) load_packed<2>(q.d, s_dg + r * 2);
+        if constexpr (EX > 0) load_packed<EX>(q.d, s_dg + r * EX);
+    };
+    // entry `place` of the row at position t met a pivot below eps: note the pivot's row
+    auto vanishing = [&](int t, int place) {
+        const int c = F.code[(size_t)t * K + place];
+        int p;                                                         // its position, from the ring slot
+        if (c < 0) p = ~c;
+        else {
+            // the latest position before t in that slot
+            const int slot = c / (int)sizeof(T);
+            p = (t & ~(kTriRing - 1)) + slot;
+            if (p >= t) p -= kTriRing;
+        }
+        atomicMin(F.status, F.order[p]);
     };
     // one step: this thread's row of [b, e) (in q) is solved while its row of the next step,
     // [e, ne), is loaded
-    auto step = [&](const TriRow<T, K>& q, TriRow<T, K>& nq, int b, int e, int ne) {
+    auto step = [&](const Row& q, Row& nq, int b, int e, int ne) {
         const int t = b + tid, nt = e + tid;
         const bool has = t < e;
         T y[K];
@@ -225,14 +251,27 @@ k_tri_sweep(TriView<T> F, const T* __restrict__ rhs, T* out, const int* gate, in
         if (nt < ne) load_row(nq, nt);
         if (has) {
             T sum = q.rv;
+            if constexpr (OP == TriOp::FACTOR) {
+                // (an unused place divides 0 by the slot that holds 1 here)
+                T l[K];
 #pragma unroll
-            for (int k = 0; k < K; ++k) sum = sub_mul<T>(sum, q.v[k], y[k]);
-            if (DIV) sum = div_by<T>(sum, q.d[0], q.d[1]);
+                for (int k = 0; k < K; ++k) l[k] = q.v[k] / y[k];
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    if (fabs(y[k]) < T(2.220446049250313e-16)) vanishing(t, k);
+                    F.low[(size_t)t * K + k] = l[k];
+                    sum = sub_mul<T>(sum, l[k], q.d[k]);
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < K; ++k) sum = sub_mul<T>(sum, q.v[k], y[k]);
+                if (OP == TriOp::BACKWARD) sum = div_by<T>(sum, q.d[0], q.d[1]);
+            }
             *reinterpret_cast<T*>(ring + (t & (kTriRing - 1)) * sizeof(T)) = sum;
             out[t] = sum;
         }
     };
-    TriRow<T, K> qa, qb;
+    Row qa, qb;
     for (int sbase = 0; sbase < F.nsteps; sbase += kTriSteps) {
         // the window's bounds and two more (past the last step: n)
         const int steps = min(kTriSteps, F.nsteps - sbase);
@@ -285,12 +324,13 @@ __global__ void k_step_fill(int nlev, const int* __restrict__ lptr, int rows, co
 // A triangle's rows from the factor's pattern and values into position order; `end - q` is
 // how far position q lies behind the end of the row's level (*far is set when that is beyond
 // the ring).  Places of rows from n up to a multiple of RB are padded.
-template <typename T, int K, bool DIV>
+template <typename T, int K, TriOp OP>
 __global__ void __launch_bounds__(256)
 k_tri_pack(int n, const int* __restrict__ order, const int* __restrict__ level, const int* __restrict__ lptr,
            const int* __restrict__ pos, const int* __restrict__ rp, const int* __restrict__ ci,
            const double* __restrict__ lu, T* val, int* code, T* dg, int* far, int* bad) {
-    constexpr int RB = TriShape<T, K, DIV>::RB;
+    constexpr int RB = TriShape<T, K, OP>::RB;
+    constexpr bool DIV = OP == TriOp::BACKWARD;
     const int total = (n + RB - 1) / RB * RB;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
         T* v = val + (size_t)t * K;
@@ -324,6 +364,74 @@ k_tri_pack(int n, const int* __restrict__ order, const int* __restrict__ level, 
             c[k] = kTriRing * (int)sizeof(T);
             v[k] = T(0);
         }
+    }
+}
+
+// The FACTOR form of a matrix's rows: lower entries, their codes, the upper entries (k, i)
+// they meet, and the diagonals.  *no is set when a row does not have that form: a lower entry
+// (i, k) whose elimination touches anything but a_ii, or a row without a diagonal.
+template <int K>
+__global__ void __launch_bounds__(256)
+k_factor_pack(int n, const int* __restrict__ order, const int* __restrict__ level, const int* __restrict__ lptr,
+              const int* __restrict__ pos, const int* __restrict__ rp, const int* __restrict__ ci,
+              const int* __restrict__ dpos, const double* __restrict__ a, double* val, int* code, double* up,
+              double* diag, int* far, int* no) {
+    constexpr int RB = TriShape<double, K, TriOp::FACTOR>::RB;
+    const int total = (n + RB - 1) / RB * RB;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+        int k = 0;
+        double d = 1.0;
+        if (t < n) {
+            const int i = order[t], end = lptr[level[i] + 1], e = rp[i + 1], di = dpos[i];
+            if (di < 0) *no = 1;
+            else d = a[di];
+            for (int p = rp[i]; p < e; ++p) {
+                const int j = ci[p];
+                if (j >= i) break;
+                // entries of row j right of its diagonal that row i has too: only column i
+                double u = 0.0;
+                bool hit = false, other = false;
+                int pi = p + 1;
+                for (int q = rp[j]; q < rp[j + 1]; ++q) {
+                    const int c = ci[q];
+                    if (c <= j) continue;
+                    while (pi < e && ci[pi] < c) ++pi;
+                    if (pi < e && ci[pi] == c) {
+                        if (c == i) { hit = true; u = a[q]; }
+                        else other = true;
+                    }
+                }
+                if (!hit || other) *no = 1;
+                const int q = pos[j];
+                if (end - q <= kTriRing) {
+                    code[(size_t)t * K + k] = (q & (kTriRing - 1)) * (int)sizeof(double);
+                } else {
+                    code[(size_t)t * K + k] = ~q;
+                    *far = 1;
+                }
+                val[(size_t)t * K + k] = a[p];
+                up[(size_t)t * K + k] = u;
+                ++k;
+            }
+        }
+        diag[t] = d;
+        for (; k < K; ++k) {
+            code[(size_t)t * K + k] = kTriRing * (int)sizeof(double);
+            val[(size_t)t * K + k] = 0.0;
+            up[(size_t)t * K + k] = 0.0;
+        }
+    }
+}
+
+template <int K>
+__global__ void __launch_bounds__(256)
+k_factor_unpack(int n, const int* __restrict__ order, const int* __restrict__ rp, const int* __restrict__ ci,
+                const int* __restrict__ dpos, const double* __restrict__ low, const double* __restrict__ diag,
+                double* lu) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        const int i = order[t];
+        for (int p = rp[i], k = 0; p < rp[i + 1] && ci[p] < i; ++p, ++k) lu[p] = low[(size_t)t * K + k];
+        lu[dpos[i]] = diag[t];
     }
 }
 
