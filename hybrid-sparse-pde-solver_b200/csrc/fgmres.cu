@@ -109,39 +109,100 @@ struct BodyScaleV0 {
 // MODE 0: acc_k = v_k . w
 // MODE 1: w -= sum_k hp_k v_k (stored), then acc_k = v_k . w
 // MODE 2: w -= sum_k hp_k v_k (stored), then acc_0 = w . w
+// A block takes 256 entries at a time: a thread an entry for the update (eight basis entries
+// loaded together), then the entries of w lie in shared memory and each warp forms the dots
+// of its own vectors, k = warp, warp + 8, ..  A thread
+// that forms all NV dots of its entries leaves NV sums across the block, a shuffle tree a warp
+// each, which were most of the time: 262,144 entries of up to 32 vectors 33.9 / 41.4 us
+// (MODE 0 / 1) against 14.4 / 25.9 here, 32,761 entries of up to 64 27.4 / 37.9 against 9.5 /
+// 26.4.  What is left is latency, of the update's chain over the vectors above all.
+constexpr int kMdotLoads = 8;
+
 template <int NV, int MODE, typename Fin>
 __global__ void __launch_bounds__(256)
 k_mdot(int n, int nv, const double* __restrict__ V, long long ld, double* w,
        const double* __restrict__ hprev, Reducer red, Fin fin, const int* gate) {
-    constexpr int NR = (MODE == 2) ? 1 : NV;
-    __shared__ double hp[NV];
-    __shared__ double rsh[8 * NR];
+    constexpr int PER = (NV + 7) / 8;              // vectors a warp
+    __shared__ double hp[NV], sw[256], tot[NV];
+    __shared__ double rsh[8];
+    __shared__ bool last;
     if (gate && *(volatile const int*)gate) return;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     if (MODE >= 1) {
-        for (int k = threadIdx.x; k < NV; k += blockDim.x) hp[k] = (k < nv) ? hprev[k] : 0.0;
+        for (int k = tid; k < NV; k += blockDim.x) hp[k] = (k < nv) ? hprev[k] : 0.0;
         __syncthreads();
     }
-    double acc[NR];
+    double acc[PER];
 #pragma unroll
-    for (int k = 0; k < NR; ++k) acc[k] = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        double wi = w[i];
-        if (MODE >= 1) {
+    for (int q = 0; q < PER; ++q) acc[q] = 0.0;
+    for (int c0 = blockIdx.x * 256; c0 < n; c0 += gridDim.x * 256) {
+        const int i = c0 + tid;
+        double wi = 0.0;
+        if (i < n) {
+            wi = w[i];
+            if (MODE >= 1) {
+                for (int k0 = 0; k0 < nv; k0 += kMdotLoads) {
+                    double v[kMdotLoads];
 #pragma unroll
-            for (int k = 0; k < NV; ++k)
-                if (k < nv) wi -= hp[k] * __ldg(&V[k * ld + i]);
-            w[i] = wi;
+                    for (int u = 0; u < kMdotLoads; ++u) v[u] = k0 + u < nv ? __ldg(&V[(k0 + u) * ld + i]) : 0.0;
+#pragma unroll
+                    for (int u = 0; u < kMdotLoads; ++u)
+                        if (k0 + u < nv) wi -= hp[k0 + u] * v[u];
+                }
+                w[i] = wi;
+            }
         }
-        if (MODE <= 1) {
-#pragma unroll
-            for (int k = 0; k < NV; ++k)
-                if (k < nv) acc[k] += __ldg(&V[k * ld + i]) * wi;
-        } else {
+        if (MODE == 2) {
             acc[0] += wi * wi;
+        } else {
+            sw[tid] = wi;
+            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < PER; ++q) {
+                const int k = wid + 8 * q;
+                if (k < nv) {
+                    double v[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) v[u] = c0 + lane + 32 * u < n ? __ldg(&V[k * ld + c0 + lane + 32 * u]) : 0.0;
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) acc[q] += v[u] * sw[lane + 32 * u];
+                }
+            }
+            __syncthreads();
         }
     }
-    double tot[NR];
-    if (grid_reduce<NR>(red, acc, rsh, tot)) fin(tot);
+    if constexpr (MODE == 2) {
+        double one[1] = {acc[0]}, sum[1];
+        if (grid_reduce<1>(red, one, rsh, sum)) fin(sum);
+    } else {
+        // block totals vector by vector; the block that finishes last adds them in block order
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const int k = wid + 8 * q;
+            const double t = warp_sum(acc[q]);
+            if (lane == 0 && k < nv) red.partials[(size_t)k * gridDim.x + blockIdx.x] = t;
+        }
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) last = atomicAdd(red.ticket, 1u) == gridDim.x - 1;
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const int k = wid + 8 * q;
+            double t = 0.0;
+            if (k < nv)
+                for (int b = lane; b < (int)gridDim.x; b += 32) t += __ldcg(&red.partials[(size_t)k * gridDim.x + b]);
+            t = warp_sum(t);
+            if (lane == 0 && k < NV) tot[k] = t;
+        }
+        __syncthreads();
+        if (tid == 0) {
+            *red.ticket = 0u;
+            fin(tot);
+        }
+    }
 }
 
 template <int NV>

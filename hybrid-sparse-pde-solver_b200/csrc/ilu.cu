@@ -8,8 +8,10 @@
 //      order, one grid barrier per level).
 //   2. the factorisation, level by level of the lower sets: each row runs the reference's
 //      IKJ elimination (same pivots, same update order, separate multiply and subtract),
-//      so the factor values equal the reference's lu_val_ bit for bit.  Short rows run from
-//      an operation list worked out beforehand for all rows at once (k_ilu_factor_ops).
+//      so the factor values equal the reference's lu_val_ bit for bit.  Where a lower entry
+//      updates only its row's diagonal (five-point grids) that is a sweep over the diagonals
+//      (TriOp::FACTOR); other short rows run from an operation list worked out beforehand for
+//      all rows at once (k_ilu_factor_ops).
 //   3. level-ordered copies of L (strictly lower part) and U (diagonal + upper part), so
 //      the rows of one level are contiguous in memory.
 // Apply: forward then backward sweep, each by the kernel its triangle's shape asks for

@@ -98,3 +98,28 @@ def test_ilu0_shapes_fp32(orc, name):
     assert s.solve(M, b, x)
     r = b - orc.spmv(*A, x)
     assert np.linalg.norm(r) <= 1.05e-10 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("n,off,zero", [(5000, 1, [0]), (5000, 1, [4998]), (5000, 1, [3, 2047, 4000]),
+                                        (9000, 1500, [1499]), (9000, 700, [20, 8290]), (9000, 5000, [17, 3900])])
+def test_ilu0_vanishing_pivot(orc, n, off, zero):
+    # rows i and i + off: a pivot that is exactly 0 where row i + off eliminates with it; the
+    # first such pivot in index order is reported
+    rp, ci, v = from_offsets(n, [-off, off], 40)
+    row = np.repeat(np.arange(n), np.diff(rp))
+    v[row == ci] = 4.0
+    v[row != ci] = -1.0
+    for z in zero:
+        v[(row == z) & (ci != z)] = 0.0
+        v[(row == z) & (ci == z)] = 0.0
+    assert orc.ilu0(rp, ci, v)[0] == H._abi.ERR_ZERO_PIVOT
+    M = H.SparseMatrix(n, n, rp, ci, v)
+    with pytest.raises(H.HamlssError) as e:
+        H.ILUPreconditioner().setup(M)
+    assert e.value.code == H._abi.ERR_ZERO_PIVOT
+    assert str(e.value).rstrip().endswith("row %d" % min(zero))
+    v[row == ci] = 4.0                                     # and the same pattern factors again
+    M = H.SparseMatrix(n, n, rp, ci, v)
+    I = H.ILUPreconditioner()
+    I.setup(M)
+    assert np.array_equal(I.factors(), orc.ilu0(rp, ci, v)[1])
