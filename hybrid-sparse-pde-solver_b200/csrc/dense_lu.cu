@@ -17,8 +17,8 @@
 //   U12       L11^-1 A12, one thread per column (unit lower triangular solve)
 //   trailing  A22 -= L21 U12, a DGEMM on the FP64 tensor cores (k_dgemm below)
 // The inverse solves A X = I: X = P I, then L Y = X and U X = Y, blocked the same way
-// (each 64-row block multiplied by its diagonal block's inverse, DGEMM update of the
-// rest): every step is a GEMM, where column-per-thread triangular solves were a long
+// (each 64-row block multiplied by its diagonal block's inverse, DGEMM updates of the
+// rest, 256 rows at a time): every step is a GEMM, where column-per-thread triangular solves were a long
 // dependent chain per launch.
 #include <vector>
 #include <cooperative_groups.h>
@@ -36,6 +36,7 @@ namespace hamlss {
 namespace {
 
 constexpr int kNb = 64;
+constexpr int kSup = 4 * kNb;            // rows of the inverse's outer blocks
 constexpr int kPanelThreads = 256;
 
 __device__ __forceinline__ bool better(double v, int i, double bv, int bi) {
@@ -348,15 +349,9 @@ __global__ void __launch_bounds__(256) k_lu_diag_inv(int n, int k0, int kb, doub
     block_inverses_smem(kb, a, li, ui, Li, Li + kNb * kNb);
 }
 
-// dst (rows x cols, ld ldd) = src (ld lds), row-major.
-__global__ void k_copy_block(int rows, int cols, const double* __restrict__ src, int lds, double* dst,
-                             int ldd) {
-    const long long total = (long long)rows * cols;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int r = (int)(t / cols), c = (int)(t - (long long)r * cols);
-        dst[(size_t)r * ldd + c] = src[(size_t)r * lds + c];
-    }
+// the identity over zeros
+__global__ void k_identity(int n, double* X) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) X[(size_t)i * n + i] = 1.0;
 }
 
 // X = P I: the identity with the factorisation's row interchanges applied in order.
@@ -376,35 +371,41 @@ __global__ void k_perm_identity(int n, const int* __restrict__ piv, double* X) {
 // ------------------------------------------------------------------------ DGEMM
 // C (m x p, ldc) = alpha * A (m x k, lda) * B (k x p, ldb) + beta * C, all row-major FP64,
 // on the FP64 tensor cores (mma.sync m8n8k4 .f64 -- the FP64 matrix path of sm_100a;
-// tcgen05 has no FP64 kind).  A CTA computes a 128 x 64 tile with 8 warps of 32 x 32
-// (4 x 4 MMA tiles each); K advances in steps of 16 staged in shared memory, the next
-// step's tile loaded into registers while the current one is multiplied.  Row strides
-// of the staged tiles (20 and 68 doubles) keep each half-warp's fragment loads on distinct
-// banks.  Edges are zero-filled, so any m, p, k works.
-constexpr int kGBM = 128, kGBN = 64, kGBK = 16, kGThreads = 256;
+// tcgen05 has no FP64 kind).  A CTA computes a BM x BN tile with 8 warps, WN of them across;
+// K advances in steps of 16 staged in shared memory, the next step's tile loaded into
+// registers while the current one is multiplied.  Row strides of the staged tiles (20 and
+// BN + 4 doubles) keep each half-warp's fragment loads on distinct banks.  Edges are
+// zero-filled, so any m, p, k works.  An element's sum does not depend on the tile.
+// A CTA writes C after its last read of A and B, so C may be A where a CTA's tile spans all
+// columns (p = k <= BN), and B where it spans all rows (m = k <= BM).
+// Tiles: 128 x 64 for the large updates; a 64-row multiply of it takes 4.3 us of an SM's
+// FP64 matrix pipe (512 operations a cycle over the chip's 148), so what fills no wave of
+// those is spread over 32 x 64 (narrow: p <= 64) or 64 x 32 tiles, a quarter of that.
+constexpr int kGBK = 16, kGThreads = 256;
 constexpr int kGAS = kGBK + 4;       // A tile row stride (doubles)
-constexpr int kGBS = kGBN + 4;       // B tile row stride
 
 __device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
                  : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
 }
 
-__global__ void __launch_bounds__(kGThreads) k_dgemm(int m, int p, int k, double alpha,
-                                                     const double* __restrict__ A, int lda,
-                                                     const double* __restrict__ B, int ldb, double beta,
-                                                     double* __restrict__ C, int ldc) {
+template <int kGBM, int kGBN, int WN>
+__global__ void __launch_bounds__(kGThreads) k_dgemm(int m, int p, int k, double alpha, const double* A, int lda,
+                                                     const double* B, int ldb, double beta, double* C, int ldc) {
+    constexpr int kGBS = kGBN + 4;                           // B tile row stride
+    constexpr int TM = kGBM / (8 / WN), TN = kGBN / WN;      // a warp's part
+    constexpr int MI = TM / 8, NJ = TN / 8;
     __shared__ double As[kGBM * kGAS];
     __shared__ double Bs[kGBK * kGBS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = warp >> 1, wn = warp & 1;                 // 4 x 2 warps of 32 x 32
+    const int wm = warp / WN, wn = warp % WN;
     const int bm = blockIdx.y * kGBM, bn = blockIdx.x * kGBN;
     const int fr = lane >> 2, fk = lane & 3;                 // fragment row / k (A), k / col (B)
-    double acc[4][4][2];
+    double acc[MI][NJ][2];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < MI; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+        for (int j = 0; j < NJ; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
     double ra[(kGBM * kGBK) / kGThreads], rb[(kGBK * kGBN) / kGThreads];
     auto load = [&](int k0) {
 #pragma unroll
@@ -442,15 +443,15 @@ __global__ void __launch_bounds__(kGThreads) k_dgemm(int m, int p, int k, double
         if (kt + 1 < nk) load((kt + 1) * kGBK);
 #pragma unroll
         for (int ks = 0; ks < kGBK; ks += 4) {
-            double af[4], bf[4];
+            double af[MI], bf[NJ];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) af[i] = As[(wm * 32 + i * 8 + fr) * kGAS + ks + fk];
+            for (int i = 0; i < MI; ++i) af[i] = As[(wm * TM + i * 8 + fr) * kGAS + ks + fk];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) bf[j] = Bs[(ks + fk) * kGBS + wn * 32 + j * 8 + fr];
+            for (int j = 0; j < NJ; ++j) bf[j] = Bs[(ks + fk) * kGBS + wn * TN + j * 8 + fr];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < MI; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) dmma_8x8x4(acc[i][j], af[i], bf[j]);
+                for (int j = 0; j < NJ; ++j) dmma_8x8x4(acc[i][j], af[i], bf[j]);
         }
         __syncthreads();
         if (kt + 1 < nk) {
@@ -460,12 +461,12 @@ __global__ void __launch_bounds__(kGThreads) k_dgemm(int m, int p, int k, double
     }
     // accumulator element h of tile (i, j): row fr, column 2 * fk + h of the 8 x 8 tile
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < MI; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < NJ; ++j)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int r = bm + wm * 32 + i * 8 + fr, c = bn + wn * 32 + j * 8 + 2 * fk + h;
+                const int r = bm + wm * TM + i * 8 + fr, c = bn + wn * TN + j * 8 + 2 * fk + h;
                 if (r < m && c < p) {
                     double* cp = C + (size_t)r * ldc + c;
                     const double v = alpha * acc[i][j][h];
@@ -478,8 +479,15 @@ __global__ void __launch_bounds__(kGThreads) k_dgemm(int m, int p, int k, double
 void dgemm(Ctx& ctx, int m, int p, int k, double alpha, const double* A, int lda, const double* B, int ldb,
            double beta, double* C, int ldc, cudaStream_t st = nullptr) {
     if (m <= 0 || p <= 0) return;
-    const dim3 grid(ceil_div(p, kGBN), ceil_div(m, kGBM));
-    k_dgemm<<<grid, kGThreads, 0, st ? st : ctx.lane.stream>>>(m, p, k, alpha, A, lda, B, ldb, beta, C, ldc);
+    if (!st) st = ctx.lane.stream;
+    if (p <= 64)
+        k_dgemm<32, 64, 4><<<dim3(1, ceil_div(m, 32)), kGThreads, 0, st>>>(m, p, k, alpha, A, lda, B, ldb, beta, C, ldc);
+    else if (m <= 64 || (long long)ceil_div(p, 64) * ceil_div(m, 128) < ctx.sm_count)
+        k_dgemm<64, 32, 2><<<dim3(ceil_div(p, 32), ceil_div(m, 64)), kGThreads, 0, st>>>(m, p, k, alpha, A, lda, B,
+                                                                                       ldb, beta, C, ldc);
+    else
+        k_dgemm<128, 64, 2><<<dim3(ceil_div(p, 64), ceil_div(m, 128)), kGThreads, 0, st>>>(m, p, k, alpha, A, lda, B,
+                                                                                         ldb, beta, C, ldc);
     HAMLSS_LAUNCH_CHECK();
 }
 
@@ -490,15 +498,20 @@ void gemm_sub(Ctx& ctx, int n, int m, int p, int k, const double* A, const doubl
     dgemm(ctx, m, p, k, -1.0, A, n, B, n, 1.0, C, n, st);
 }
 
-// Row-major C (m x p, ldc) = A (m x k, lda) * B (k x p, ldb).
-void gemm_set(Ctx& ctx, int m, int p, int k, const double* A, int lda, const double* B, int ldb,
-              double* C, int ldc, cudaStream_t st = nullptr) {
-    if (m <= 0 || p <= 0 || k <= 0) return;
-    dgemm(ctx, m, p, k, 1.0, A, lda, B, ldb, 0.0, C, ldc, st);
+// C (m x kb, kb <= kNb) = C * R, R a kb x kb block (ld kNb): a CTA's 32 x 64 tile holds all
+// columns of its rows.
+void gemm_right(Ctx& ctx, int m, int kb, double* C, int ldc, const double* R, cudaStream_t st) {
+    if (m <= 0) return;
+    k_dgemm<32, kNb, 4><<<dim3(1, ceil_div(m, 32)), kGThreads, 0, st>>>(m, kb, kb, 1.0, C, ldc, R, kNb, 0.0, C, ldc);
+    HAMLSS_LAUNCH_CHECK();
 }
 
-int copy_grid(Ctx& ctx, long long count) {
-    return (int)std::max<long long>(1, std::min<long long>((count + 255) / 256, ctx.sm_count * 8LL));
+// C (kb x p, kb <= kNb) = L * C, L a kb x kb block (ld kNb): a CTA's 64 x 32 tile holds all
+// rows of its columns.
+void gemm_left(Ctx& ctx, int kb, int p, const double* L, double* C, int ldc, cudaStream_t st) {
+    if (p <= 0) return;
+    k_dgemm<kNb, 32, 2><<<dim3(ceil_div(p, 32), 1), kGThreads, 0, st>>>(kb, p, kb, 1.0, L, kNb, C, ldc, 0.0, C, ldc);
+    HAMLSS_LAUNCH_CHECK();
 }
 
 int col_grid(Ctx& ctx, int cols) {
@@ -512,7 +525,7 @@ __global__ void k_iota(int n, int* piv) {
 
 // Blocked LU without row interchanges; false when a pivot falls below `floor`.
 // L21 = A21 U11^-1 and U12 = L11^-1 A12 are GEMMs with the diagonal block's inverses
-// (k_block_inverses) through the scratch T (n x kNb doubles).
+// (k_block_inverses), in place.
 //
 // With look-ahead: step k's update of block column and block row k + 1 runs first, on a
 // second stream, followed there by step k + 1's diagonal block and panels, while the rest of
@@ -520,7 +533,7 @@ __global__ void k_iota(int n, int* piv) {
 // look-ahead writes block column / row k + 1, the trailing update the part beyond it; the
 // second stream waits for trailing update k - 1 (the last writer of block k + 1) and the
 // context's stream for panel k (the operands of trailing update k).
-bool factor_nopivot(Ctx& ctx, int n, double* M, double floor, double* inv, double* T) {
+bool factor_nopivot(Ctx& ctx, int n, double* M, double floor, double* inv) {
     cudaStream_t s = ctx.lane.stream;
     DBuf<int> tiny(1);
     tiny.zero(s);
@@ -561,12 +574,8 @@ bool factor_nopivot(Ctx& ctx, int n, double* M, double floor, double* inv, doubl
                 const double* Ui = Li + kNb * kNb;
                 double* A21 = M + (size_t)(k0 + kb) * n + k0;
                 double* A12 = M + (size_t)k0 * n + k0 + kb;
-                gemm_set(ctx, rest, kb, kb, A21, n, Ui, kNb, T, kNb, pst);
-                k_copy_block<<<copy_grid(ctx, (long long)rest * kb), 256, 0, pst>>>(rest, kb, T, kNb, A21, n);
-                HAMLSS_LAUNCH_CHECK();
-                gemm_set(ctx, kb, rest, kb, Li, kNb, A12, n, T, rest, pst);
-                k_copy_block<<<copy_grid(ctx, (long long)rest * kb), 256, 0, pst>>>(kb, rest, T, rest, A12, n);
-                HAMLSS_LAUNCH_CHECK();
+                gemm_right(ctx, rest, kb, A21, n, Ui, pst);
+                gemm_left(ctx, kb, rest, Li, A12, n, pst);
             }
             HAMLSS_CUDA(cudaEventRecord(panel_ev[k], pst));
         };
@@ -738,8 +747,8 @@ void dense_lu_inverse(Ctx& ctx, int n, double* M, double* Minv, int* piv) {
     double big = 0.0;
     std::memcpy(&big, &bits, sizeof big);
     const int nblk = (n + kNb - 1) / kNb;
-    DBuf<double> inv(2LL * nblk * kNb * kNb), T((size_t)n * kNb);
-    const bool nopiv = factor_nopivot(ctx, n, M, 1e-10 * big, inv.p, T.p);
+    DBuf<double> inv(2LL * nblk * kNb * kNb);
+    const bool nopiv = factor_nopivot(ctx, n, M, 1e-10 * big, inv.p);
     if (nopiv) {
         k_iota<<<cg_, 128, 0, s>>>(n, piv);
         HAMLSS_LAUNCH_CHECK();
@@ -751,31 +760,42 @@ void dense_lu_inverse(Ctx& ctx, int n, double* M, double* Minv, int* piv) {
     }
     // X = P I; L Y = X (forward, unit lower); U X = Y (backward).  The diagonal blocks are
     // applied as GEMMs with their inverses, the off-diagonal blocks as GEMM updates.
-    k_perm_identity<<<cg_, 128, 0, s>>>(n, piv, Minv);
+    if (nopiv) {
+        HAMLSS_CUDA(cudaMemsetAsync(Minv, 0, bytes, s));
+        k_identity<<<cg_, 128, 0, s>>>(n, Minv);
+    } else {
+        k_perm_identity<<<cg_, 128, 0, s>>>(n, piv, Minv);
+    }
     HAMLSS_LAUNCH_CHECK();
-    DBuf<double> W((size_t)kNb * n);
     // Without interchanges X = I, so Y = L^-1 is lower triangular: block row k0 of Y has
     // nonzeros only in columns < k0 + kb, and the forward sweep touches only those
     // (n^3 / 3 multiply-adds instead of n^3).
-    for (int k0 = 0; k0 < n; k0 += kNb) {
-        const int kb = std::min(kNb, n - k0);
-        const int w = nopiv ? k0 + kb : n;
-        const double* Li = inv.p + 2LL * (k0 / kNb) * kNb * kNb;
-        gemm_set(ctx, kb, w, kb, Li, kNb, Minv + (size_t)k0 * n, n, W.p, n);
-        k_copy_block<<<copy_grid(ctx, (long long)kb * w), 256, 0, s>>>(kb, w, W.p, n, Minv + (size_t)k0 * n, n);
-        HAMLSS_LAUNCH_CHECK();
-        const int rest = n - k0 - kb;
-        gemm_sub(ctx, n, rest, w, kb, M + (size_t)(k0 + kb) * n + k0, Minv + (size_t)k0 * n,
-                 Minv + (size_t)(k0 + kb) * n);
+    // Rows are taken kSup at a time: block by block inside, then one update of the rows
+    // beyond, which reads and writes them once for kSup / kNb blocks.  With that, the small
+    // tiles and the panels in place, the factorisation and inverse of 4,761 rows went from 32
+    // to 21 ms; the rest is mostly the factorisation's chain of diagonal blocks (77 us each)
+    // and panels.
+    for (int s0 = 0; s0 < n; s0 += kSup) {
+        const int s1 = std::min(s0 + kSup, n);
+        for (int k0 = s0; k0 < s1; k0 += kNb) {
+            const int kb = std::min(kNb, s1 - k0);
+            const int w = nopiv ? k0 + kb : n;
+            gemm_left(ctx, kb, w, inv.p + 2LL * (k0 / kNb) * kNb * kNb, Minv + (size_t)k0 * n, n, s);
+            gemm_sub(ctx, n, s1 - k0 - kb, w, kb, M + (size_t)(k0 + kb) * n + k0, Minv + (size_t)k0 * n,
+                     Minv + (size_t)(k0 + kb) * n);
+        }
+        gemm_sub(ctx, n, n - s1, nopiv ? s1 : n, s1 - s0, M + (size_t)s1 * n + s0, Minv + (size_t)s0 * n,
+                 Minv + (size_t)s1 * n);
     }
-    const int last = ((n - 1) / kNb) * kNb;
-    for (int k0 = last; k0 >= 0; k0 -= kNb) {
-        const int kb = std::min(kNb, n - k0);
-        const double* Ui = inv.p + 2LL * (k0 / kNb) * kNb * kNb + kNb * kNb;
-        gemm_set(ctx, kb, n, kb, Ui, kNb, Minv + (size_t)k0 * n, n, W.p, n);
-        k_copy_block<<<copy_grid(ctx, (long long)kb * n), 256, 0, s>>>(kb, n, W.p, n, Minv + (size_t)k0 * n, n);
-        HAMLSS_LAUNCH_CHECK();
-        gemm_sub(ctx, n, k0, n, kb, M + k0, Minv + (size_t)k0 * n, Minv);
+    for (int s0 = (n - 1) / kSup * kSup; s0 >= 0; s0 -= kSup) {
+        const int s1 = std::min(s0 + kSup, n);
+        for (int k0 = s0 + (s1 - s0 - 1) / kNb * kNb; k0 >= s0; k0 -= kNb) {
+            const int kb = std::min(kNb, s1 - k0);
+            gemm_left(ctx, kb, n, inv.p + (2LL * (k0 / kNb) + 1) * kNb * kNb, Minv + (size_t)k0 * n, n, s);
+            gemm_sub(ctx, n, k0 - s0, n, kb, M + (size_t)s0 * n + k0, Minv + (size_t)k0 * n,
+                     Minv + (size_t)s0 * n);
+        }
+        gemm_sub(ctx, n, s0, n, s1 - s0, M + s0, Minv + (size_t)s0 * n, Minv);
     }
     HAMLSS_CUDA(cudaStreamSynchronize(s));
 }
