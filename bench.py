@@ -1239,6 +1239,14 @@ def main():
     out, data = run_ours(args, rank, world, local)
     if out is None:
         return
+    import oracle
+
+    if rank == 0 and world == 1 and not oracle.reference_available(fast=True):
+        # the side measurements that time the reference beside the device
+        args.no_cpu_baseline = args.no_same_algorithm = args.no_configs = True
+        args.no_batch = args.no_variants = args.no_ilut = True
+        args.serving_full = 0
+        out["cpu_baseline"] = {"unavailable": "the reference is not built here (oracle/_ref)"}
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         log("timing the reference sample")
         cb = cpu_baseline(args, data)

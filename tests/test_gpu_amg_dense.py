@@ -72,12 +72,14 @@ def test_coarse_inverse(n):
 @pytest.mark.parametrize("n", [1025, 1087, 1088, 1089, 1279, 1281, 1345, 2305])
 @pytest.mark.parametrize("shuffled", [False, True])
 def test_coarse_inverse_blocked(n, shuffled):
-    # beyond 1,024 rows: blocks of 64 in groups of 256, with and (shuffled) without a
-    # diagonal that serves as pivots; the same bound, a factor of 10 at 2,305
+    # beyond 1,024 rows: blocks of 64 in groups of 256.  With its diagonal in place D needs
+    # no interchanges (the same bound, a factor of 10 at 2,305); shuffled, with zeros on the
+    # diagonal that end the attempt without them, it takes the pivoted form.
     rng = np.random.default_rng(n)
     D = rng.standard_normal((n, n)) / np.sqrt(n) + 3.0 * np.eye(n)
     if shuffled:
         D = D[rng.permutation(n)]
+        D[np.arange(0, n, 7), np.arange(0, n, 7)] = 0.0
     r = rng.standard_normal(n)
     z = one_level(csr(D), n).apply(r)
     assert np.linalg.norm(r - D @ z) <= 1e-11 * np.linalg.norm(r)
