@@ -109,21 +109,21 @@ struct BodyScaleV0 {
 // MODE 0: acc_k = v_k . w
 // MODE 1: w -= sum_k hp_k v_k (stored), then acc_k = v_k . w
 // MODE 2: w -= sum_k hp_k v_k (stored), then acc_0 = w . w
-// A block takes 256 entries at a time: a thread an entry for the update (eight basis entries
-// loaded together), then the entries of w lie in shared memory and each warp forms the dots
-// of its own vectors, k = warp, warp + 8, ..  A thread
-// that forms all NV dots of its entries leaves NV sums across the block, a shuffle tree a warp
-// each, which were most of the time: 262,144 entries of up to 32 vectors 33.9 / 41.4 us
-// (MODE 0 / 1) against 14.4 / 25.9 here, 32,761 entries of up to 64 27.4 / 37.9 against 9.5 /
-// 26.4.  What is left is latency, of the update's chain over the vectors above all.
-constexpr int kMdotLoads = 8;
-
+// A block takes 256 entries at a time, and each warp the vectors k = warp, warp + 8, .. of
+// them: its part of the update, the warps' parts added through shared memory, then its own
+// dots with the new entries of w, also there.  With a thread an entry the update is a chain
+// over the vectors, the dots leave NV sums across the block, a shuffle tree a warp each, and
+// what one thread did afterwards (fin) went value by value: 262,144 entries of up to 32
+// vectors took 33.9 / 41.4 / 18.7 us (MODE 0 / 1 / 2) and 32,761 entries of up to 64
+// 27.4 / 37.9 / 20.2, against 15.0 / 17.9 / 14.6 and 8.9 / 11.0 / 11.0 here.  Now bound by
+// the vectors' loads from L2 and the sums' latency.
 template <int NV, int MODE, typename Fin>
 __global__ void __launch_bounds__(256)
 k_mdot(int n, int nv, const double* __restrict__ V, long long ld, double* w,
        const double* __restrict__ hprev, Reducer red, Fin fin, const int* gate) {
     constexpr int PER = (NV + 7) / 8;              // vectors a warp
     __shared__ double hp[NV], sw[256], tot[NV];
+    __shared__ double ssub[MODE >= 1 ? 8 : 1][256];
     __shared__ double rsh[8];
     __shared__ bool last;
     if (gate && *(volatile const int*)gate) return;
@@ -137,23 +137,31 @@ k_mdot(int n, int nv, const double* __restrict__ V, long long ld, double* w,
     for (int q = 0; q < PER; ++q) acc[q] = 0.0;
     for (int c0 = blockIdx.x * 256; c0 < n; c0 += gridDim.x * 256) {
         const int i = c0 + tid;
-        double wi = 0.0;
-        if (i < n) {
-            wi = w[i];
-            if (MODE >= 1) {
-                for (int k0 = 0; k0 < nv; k0 += kMdotLoads) {
-                    double v[kMdotLoads];
+        double wi = i < n ? w[i] : 0.0;
+        if (MODE >= 1) {
+            double sub[8] = {};
 #pragma unroll
-                    for (int u = 0; u < kMdotLoads; ++u) v[u] = k0 + u < nv ? __ldg(&V[(k0 + u) * ld + i]) : 0.0;
+            for (int q = 0; q < PER; ++q) {
+                const int k = wid + 8 * q;
+                if (k < nv) {
+                    const double h = hp[k];
+                    double v[8];
 #pragma unroll
-                    for (int u = 0; u < kMdotLoads; ++u)
-                        if (k0 + u < nv) wi -= hp[k0 + u] * v[u];
+                    for (int u = 0; u < 8; ++u) v[u] = c0 + lane + 32 * u < n ? __ldg(&V[k * ld + c0 + lane + 32 * u]) : 0.0;
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) sub[u] += h * v[u];
                 }
-                w[i] = wi;
             }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) ssub[wid][lane + 32 * u] = sub[u];
+            __syncthreads();
+            wi -= ((ssub[0][tid] + ssub[1][tid]) + (ssub[2][tid] + ssub[3][tid])) +
+                  ((ssub[4][tid] + ssub[5][tid]) + (ssub[6][tid] + ssub[7][tid]));
+            if (i < n) w[i] = wi;
         }
         if (MODE == 2) {
-            acc[0] += wi * wi;
+            if (i < n) acc[0] += wi * wi;
+            __syncthreads();                               // ssub is written again
         } else {
             sw[tid] = wi;
             __syncthreads();
@@ -198,28 +206,24 @@ k_mdot(int n, int nv, const double* __restrict__ V, long long ld, double* w,
             if (lane == 0 && k < NV) tot[k] = t;
         }
         __syncthreads();
-        if (tid == 0) {
-            *red.ticket = 0u;
-            fin(tot);
-        }
+        if (tid == 0) *red.ticket = 0u;
+        if (tid < nv) fin(tid, tot[tid]);
     }
 }
 
-template <int NV>
-struct FinH1 {
+struct FinH1 {                                             // a thread a vector
     GmArrays a;
     int j;
-    __device__ void operator()(const double (&t)[NV]) const {
-        for (int k = 0; k <= j && k < NV; ++k) { a.h1[k] = t[k]; a.H[k * a.m + j] = t[k]; }
+    __device__ void operator()(int k, double t) const {
+        if (k <= j) { a.h1[k] = t; a.H[k * a.m + j] = t; }
     }
 };
 
-template <int NV>
 struct FinH2 {
     GmArrays a;
     int j;
-    __device__ void operator()(const double (&t)[NV]) const {
-        for (int k = 0; k <= j && k < NV; ++k) { a.h2[k] = t[k]; a.H[k * a.m + j] += t[k]; }
+    __device__ void operator()(int k, double t) const {
+        if (k <= j) { a.h2[k] = t; a.H[k * a.m + j] += t; }
     }
 };
 
@@ -249,7 +253,23 @@ struct FinNorm {
         // PipelinedFGMRESSolver leaves the cycle on a lucky breakdown before rotating
         // column j (pipelined_fgmres_solver.cpp:117-123)
         if (s->pipelined && !(hn > kEps)) { s->jcount = j + 1; s->halt = 1; return; }
-        for (int i = 0; i < j; ++i) rot(a.H[i * m + j], a.H[(i + 1) * m + j], a.cs[i], a.sn[i]);
+        // (eight rotations' operands loaded together: one by one, each behind the store of the
+        // one before, they were half of the kernel at 60 vectors)
+        double x = a.H[j];
+        for (int i0 = 0; i0 < j; i0 += 8) {
+            double y[8], c[8], q[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (i0 + u < j) { y[u] = a.H[(i0 + u + 1) * m + j]; c[u] = a.cs[i0 + u]; q[u] = a.sn[i0 + u]; }
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (i0 + u < j) {
+                    rot(x, y[u], c[u], q[u]);
+                    a.H[(i0 + u) * m + j] = x;
+                    x = y[u];
+                }
+        }
+        a.H[j * m + j] = x;
         double r;
         givens(a.H[j * m + j], a.H[(j + 1) * m + j], a.cs[j], a.sn[j], r);
         a.H[j * m + j] = r;
@@ -308,11 +328,11 @@ void launch_mdot_t(Ctx& ctx, int mode, int n, int nv, const double* V, long long
     L.red_check(blocks, mode == 2 ? 1 : NV);
     ProfScope ps(L, "gmres_mdot", 8.0 * n * (nv + (mode == 0 ? 1 : 2)));
     if (mode == 0)
-        k_mdot<NV, 0, FinH1<NV>><<<blocks, 256, 0, L.stream>>>(n, nv, V, ld, w, hprev, L.red(),
-                                                                FinH1<NV>{a, j}, gate);
+        k_mdot<NV, 0, FinH1><<<blocks, 256, 0, L.stream>>>(n, nv, V, ld, w, hprev, L.red(),
+                                                                FinH1{a, j}, gate);
     else if (mode == 1)
-        k_mdot<NV, 1, FinH2<NV>><<<blocks, 256, 0, L.stream>>>(n, nv, V, ld, w, hprev, L.red(),
-                                                                FinH2<NV>{a, j}, gate);
+        k_mdot<NV, 1, FinH2><<<blocks, 256, 0, L.stream>>>(n, nv, V, ld, w, hprev, L.red(),
+                                                                FinH2{a, j}, gate);
     else
         k_mdot<NV, 2, FinNorm><<<blocks, 256, 0, L.stream>>>(n, nv, V, ld, w, hprev, L.red(),
                                                               FinNorm{s, a, j}, gate);
