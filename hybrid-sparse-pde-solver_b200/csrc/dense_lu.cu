@@ -299,41 +299,34 @@ __global__ void __launch_bounds__(256) k_lu_diag_inv(int n, int k0, int kb, doub
             const int r = ty + 16 * i, c = tx + 16 * q;
             e[i][q] = (r < kb && c < kb) ? M[(size_t)(k0 + r) * n + k0 + c] : 0.0;
         }
-    for (int j = 0; j < kb; ++j) {
-        const int jq = j >> 4, jm = j & 15;
-        // (compile-time register indices: the block of column / row j is selected by q == jq)
+    // 16 columns at a time, unrolled, so that the parts of e behind them are known to the
+    // compiler: the step's instructions, not its barriers, are most of its time.  Rows and
+    // columns past kb hold zeros (and are not written back).
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+    for (int jq = 0; jq < 4; ++jq)
+        for (int jm = 0; jm < 16 && jq * 16 + jm < kb; ++jm) {
+            const int j = jq * 16 + jm;
+            if (tx == jm)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                if (tx == jm && q == jq) colj[ty + 16 * i] = e[i][q];   // column j (unscaled)
-                if (ty == jm && i == jq) rowj[tx + 16 * q] = e[i][q];   // row j
+                for (int i = jq; i < 4; ++i) colj[ty + 16 * i] = e[i][jq];    // column j (unscaled)
+            if (ty == jm)
+#pragma unroll
+                for (int q = jq; q < 4; ++q) rowj[tx + 16 * q] = e[jq][q];    // row j
+            __syncthreads();
+            const double d = rowj[j];
+            if (threadIdx.x == 0 && !(fabs(d) > floor)) *tiny = 1;
+            const double inv_d = (d != 0.0) ? 1.0 / d : 0.0;
+#pragma unroll
+            for (int i = jq; i < 4; ++i) {
+                if (i == jq && ty <= jm) continue;                            // rows up to j
+                const double l = __dmul_rn(colj[ty + 16 * i], inv_d);
+#pragma unroll
+                for (int q = jq; q < 4; ++q)
+                    if (q > jq || tx > jm) e[i][q] = __dsub_rn(e[i][q], __dmul_rn(l, rowj[tx + 16 * q]));
+                if (tx == jm) e[i][jq] = l;                                   // the multipliers of column j
             }
-        __syncthreads();
-        const double d = rowj[j];
-        if (threadIdx.x == 0 && !(fabs(d) > floor)) *tiny = 1;
-        const double inv_d = (d != 0.0) ? 1.0 / d : 0.0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int r = ty + 16 * i;
-            if (r <= j || r >= kb) continue;
-            const double l = __dmul_rn(colj[r], inv_d);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int c = tx + 16 * q;
-                if (c > j && c < kb) e[i][q] = __dsub_rn(e[i][q], __dmul_rn(l, rowj[c]));
-            }
+            __syncthreads();                                                  // colj / rowj reused
         }
-        if (tx == jm)                                             // the multipliers of column j
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int r = ty + 16 * i;
-                    if (q == jq && r > j && r < kb) e[i][q] = __dmul_rn(e[i][q], inv_d);
-                }
-        __syncthreads();                                          // colj / rowj reused
-    }
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -773,7 +766,7 @@ void dense_lu_inverse(Ctx& ctx, int n, double* M, double* Minv, int* piv) {
     // Rows are taken kSup at a time: block by block inside, then one update of the rows
     // beyond, which reads and writes them once for kSup / kNb blocks.  With that, the small
     // tiles and the panels in place, the factorisation and inverse of 4,761 rows went from 32
-    // to 21 ms; the rest is mostly the factorisation's chain of diagonal blocks (77 us each)
+    // to about 20 ms; the rest is mostly the factorisation's chain of diagonal blocks (56 us each; 77 with columns selected at run time)
     // and panels.
     for (int s0 = 0; s0 < n; s0 += kSup) {
         const int s1 = std::min(s0 + kSup, n);
