@@ -766,8 +766,8 @@ void dense_lu_inverse(Ctx& ctx, int n, double* M, double* Minv, int* piv) {
     // Rows are taken kSup at a time: block by block inside, then one update of the rows
     // beyond, which reads and writes them once for kSup / kNb blocks.  With that, the small
     // tiles and the panels in place, the factorisation and inverse of 4,761 rows went from 32
-    // to about 20 ms; the rest is mostly the factorisation's chain of diagonal blocks (56 us each; 77 with columns selected at run time)
-    // and panels.
+    // to about 20 ms; the rest is mostly the factorisation's chain of diagonal blocks (56 us
+    // each; 77 with columns selected at run time) and panels.
     for (int s0 = 0; s0 < n; s0 += kSup) {
         const int s1 = std::min(s0 + kSup, n);
         for (int k0 = s0; k0 < s1; k0 += kNb) {
