@@ -35,6 +35,17 @@ int guarded(F&& f) {
     }
 }
 
+// guarded() for calls whose kernels wait with a bound: the lane's error word is taken on every
+// way out, so that a wait that ran out is reported by the call it happened in and by no other.
+template <typename F>
+int on_lane(hamlss_ctx* ctx, const char* what, F&& f) {
+    const int rc = guarded(f);
+    if (!ctx) return rc;
+    if (rc != HAMLSS_OK) cudaStreamSynchronize(ctx->c.lane.stream);     // (kernels may still be queued)
+    if (lane_take_timeout(ctx->c.lane)) return set_err(HAMLSS_ERR_TIMEOUT, what);
+    return rc;
+}
+
 double now_s() {
     return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
@@ -149,6 +160,12 @@ int hamlss_ctx_synchronize(hamlss_ctx* ctx) {
 int hamlss_ctx_stream(hamlss_ctx* ctx, void** stream) {
     if (!ctx || !stream) return set_err(HAMLSS_ERR_INVALID, "null argument");
     *stream = (void*)ctx->c.lane.stream;
+    return HAMLSS_OK;
+}
+
+int hamlss_ctx_wait_word(hamlss_ctx* ctx, int32_t** word) {
+    if (!ctx || !word) return set_err(HAMLSS_ERR_INVALID, "null argument");
+    *word = ctx->c.lane.err.p;
     return HAMLSS_OK;
 }
 
@@ -429,7 +446,7 @@ int hamlss_scale(hamlss_ctx* ctx, int32_t n, double alpha, double* x) {
 // ---------------------------------------------------------------- preconditioners
 int hamlss_precond_setup(hamlss_ctx* ctx, const hamlss_mat* A, int kind,
                          const hamlss_params* params, hamlss_prec** out, double* setup_time_s) {
-    return guarded([&]() -> int {
+    return on_lane(ctx, "a kernel of the preconditioner setup gave up a bounded wait", [&]() -> int {
         if (!ctx || !A || !out) return set_err(HAMLSS_ERR_INVALID, "null argument");
         hamlss_params p;
         if (params) p = *params; else hamlss_params_default(&p);
@@ -455,6 +472,8 @@ int hamlss_precond_setup(hamlss_ctx* ctx, const hamlss_mat* A, int kind,
                 return set_err(HAMLSS_ERR_INVALID, "SolverFactory: unknown PrecondType");
         }
         HAMLSS_CUDA(cudaStreamSynchronize(ctx->c.lane.stream));
+        if (lane_take_timeout(ctx->c.lane))
+            return set_err(HAMLSS_ERR_TIMEOUT, "a kernel of the preconditioner setup gave up a bounded wait");
         auto* h = new hamlss_prec();
         h->ctx = ctx;
         h->A = Am;

@@ -1531,6 +1531,8 @@ void finish_ilu(Ctx& ctx, IluPrec* P, bool factorise) {
         int h = 0;
         status.download(&h, 1, s);
         HAMLSS_CUDA(cudaStreamSynchronize(s));
+        if (lane_take_timeout(ctx.lane))
+            fail(HAMLSS_ERR_TIMEOUT, "ILU(0): the elimination gave up waiting for its bulk copies");
         if (h != 0x7fffffff)
             fail(HAMLSS_ERR_ZERO_PIVOT, "ILU(0): near-zero pivot at row " + std::to_string(h));
     }

@@ -223,6 +223,7 @@ def _declare(L: C.CDLL) -> None:
         "hamlss_ctx_destroy": (C.c_int, [P]),
         "hamlss_ctx_synchronize": (C.c_int, [P]),
         "hamlss_ctx_stream": (C.c_int, [P, pp]),
+        "hamlss_ctx_wait_word": (C.c_int, [P, C.POINTER(pi)]),
         "hamlss_profile_enable": (C.c_int, [P, C.c_int, I32]),
         "hamlss_profile_read": (C.c_int, [P, I32, V, V, V, V, pi]),
         "hamlss_energy_read": (C.c_int, [C.c_int, pd]),

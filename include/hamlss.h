@@ -169,6 +169,10 @@ int hamlss_ctx_destroy(hamlss_ctx* ctx);
 int hamlss_ctx_synchronize(hamlss_ctx* ctx);
 /* The context's cudaStream_t, as an opaque pointer, so callers can order their own work. */
 int hamlss_ctx_stream(hamlss_ctx* ctx, void** stream);
+/* The context's error word, in pinned host memory: a kernel whose bounded wait runs out
+ * writes 1 to it, and the call that launched the kernel returns HAMLSS_ERR_TIMEOUT (and no
+ * handle) and clears it.  For monitors, and for tests that set it. */
+int hamlss_ctx_wait_word(hamlss_ctx* ctx, int32_t** word);
 
 /* Measurement support (no counterpart in the reference): when enabled, every engine
  * launch on this context is bracketed by a pair of CUDA events on the context stream and

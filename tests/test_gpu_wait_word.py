@@ -1,0 +1,61 @@
+"""A bounded device-side wait that runs out is reported by the call it happened in (-m gpu).
+
+The kernels that wait (bulk copies, grid barriers) set the context's pinned error word when
+a wait runs out, and what they leave behind is not a result.  Here the host sets the word,
+as such a kernel would, and no kernel misbehaves.
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from gpu_util import need_gpu
+import hsps_b200 as H
+from hsps_b200 import _abi
+from hsps_b200 import problems as P
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _gpu():
+    need_gpu()
+
+
+@pytest.fixture
+def system():
+    """(matrix on a context of its own, the context's word, a right-hand side)"""
+    ctx = H.Context(0)
+    w = C.POINTER(C.c_int32)()
+    assert H.lib().hamlss_ctx_wait_word(ctx.h, C.byref(w)) == 0 and w[0] == 0
+    A = H.SparseMatrix(400, 400, *P.poisson_2d(20), ctx=ctx)
+    return A, w, P.rhs(400, 1)
+
+
+@pytest.mark.parametrize("make", [lambda: H.ILUPreconditioner(), lambda: H.JacobiPreconditioner(),
+                                  lambda: H.AMGPreconditioner()], ids=["ilu", "jacobi", "amg"])
+def test_setup_reports_its_own_wait(system, make):
+    A, w, b = system
+    M = make()
+    w[0] = 1
+    with pytest.raises(H.HamlssError) as e:
+        M.setup(A)
+    assert e.value.code == _abi.ERR_TIMEOUT and w[0] == 0
+    assert M.h is None and not M.is_ready()
+    A.spmv(b)                                  # the next call is not blamed
+    M.setup(A)
+    assert np.isfinite(M.apply(b)).all()
+
+
+def test_failed_setup_leaves_no_word(system):
+    A, w, b = system
+    v = A.values().copy()
+    v[0] = 0.0                                 # a_00: no Jacobi
+    A.set_values(v)
+    w[0] = 1
+    with pytest.raises(H.HamlssError) as e:
+        H.JacobiPreconditioner().setup(A)
+    assert e.value.code == _abi.ERR_TIMEOUT and w[0] == 0
+    with pytest.raises(H.HamlssError) as e:
+        H.JacobiPreconditioner().setup(A)
+    assert e.value.code == _abi.ERR_ZERO_DIAG
