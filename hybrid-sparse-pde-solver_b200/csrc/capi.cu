@@ -368,7 +368,7 @@ int dot_impl(hamlss_ctx* ctx, int32_t n, const double* x, const double* y, doubl
 extern "C" {
 
 int hamlss_spmv(hamlss_ctx* ctx, const hamlss_mat* A, const double* x, double* y, int where) {
-    return guarded([&]() -> int {
+    return on_lane(ctx, "an SpMV gave up waiting for its bulk copies", [&]() -> int {
         if (!ctx || !A || (A->A.n && (!x || !y))) return set_err(HAMLSS_ERR_INVALID, "null argument");
         Ctx& c = ctx->c;
         cudaStream_t s = c.lane.stream;
@@ -398,8 +398,6 @@ int hamlss_spmv(hamlss_ctx* ctx, const hamlss_mat* A, const double* x, double* y
         }
         if (where == HAMLSS_HOST) ws.d[7].download(y, A->A.n, s);
         HAMLSS_CUDA(cudaStreamSynchronize(s));
-        if (lane_take_timeout(c.lane))
-            return set_err(HAMLSS_ERR_TIMEOUT, "an SpMV gave up waiting for its bulk copies");
         return HAMLSS_OK;
     });
 }
@@ -486,7 +484,7 @@ int hamlss_precond_setup(hamlss_ctx* ctx, const hamlss_mat* A, int kind,
 
 int hamlss_precond_apply(hamlss_ctx* ctx, const hamlss_prec* M, const double* r, double* z,
                          int where) {
-    return guarded([&]() -> int {
+    return on_lane(ctx, "a preconditioner kernel gave up a bounded wait", [&]() -> int {
         if (!ctx || !M || !r || !z) return set_err(HAMLSS_ERR_INVALID, "null argument");
         Ctx& c = ctx->c;
         cudaStream_t s = c.lane.stream;
@@ -504,8 +502,6 @@ int hamlss_precond_apply(hamlss_ctx* ctx, const hamlss_prec* M, const double* r,
         M->p->apply(c, c.lane, dr, dz, nullptr);
         if (where == HAMLSS_HOST) ws.d[7].download(z, n, s);
         HAMLSS_CUDA(cudaStreamSynchronize(s));
-        if (lane_take_timeout(c.lane))
-            return set_err(HAMLSS_ERR_TIMEOUT, "a preconditioner kernel gave up waiting for its bulk copies");
         return HAMLSS_OK;
     });
 }
@@ -528,7 +524,7 @@ int hamlss_precond_release(hamlss_prec* M) {
 
 int hamlss_amg_aggregate(hamlss_ctx* ctx, const hamlss_mat* A, double theta, int32_t* agg,
                          int32_t* n_agg) {
-    return guarded([&]() -> int {
+    return on_lane(ctx, "a kernel of the aggregation gave up a bounded wait", [&]() -> int {
         if (!ctx || !A || !agg || !n_agg) return set_err(HAMLSS_ERR_INVALID, "null argument");
         return amg_aggregate_matrix(ctx->c, const_cast<hamlss_mat*>(A), theta, agg, n_agg);
     });
@@ -632,6 +628,8 @@ void fill_stats(Ctx& c, hamlss_mat* Am, int solver, const Prec* P, const SolveRe
     *out = st;
 }
 
+constexpr const char* kSolveWait = "a kernel of the solve gave up a bounded wait";
+
 struct IoVecs {
     const double* b;
     double* x;
@@ -653,7 +651,7 @@ extern "C" {
 int hamlss_solve(hamlss_ctx* ctx, int solver, const hamlss_mat* A, const hamlss_prec* M,
                  const double* b, double* x, int where, const hamlss_params* params,
                  hamlss_stats* stats) {
-    return guarded([&]() -> int {
+    return on_lane(ctx, kSolveWait, [&]() -> int {
         if (!ctx || !A || !b || !x) return set_err(HAMLSS_ERR_INVALID, "null argument");
         if (A->A.n != A->A.m) return set_err(HAMLSS_ERR_SIZE, "solve needs a square matrix");
         if (M && M->p->n != A->A.n)
@@ -682,15 +680,13 @@ int hamlss_solve(hamlss_ctx* ctx, int solver, const hamlss_mat* A, const hamlss_
         HAMLSS_CUDA(cudaStreamSynchronize(s));
         if (r.status != HAMLSS_OK)
             return set_err(r.status, "non-finite values met during the solve");
-        if (lane_take_timeout(c.lane))
-            return set_err(HAMLSS_ERR_TIMEOUT, "a kernel of the solve gave up a bounded wait");
         return HAMLSS_OK;
     });
 }
 
 int hamlss_extract_features(hamlss_ctx* ctx, const hamlss_mat* A, double features[24],
                             int32_t* initial_state) {
-    return guarded([&]() -> int {
+    return on_lane(ctx, "a kernel of the feature extraction gave up a bounded wait", [&]() -> int {
         if (!ctx || !A || !features) return set_err(HAMLSS_ERR_INVALID, "null argument");
         int st = 0;
         int rc = extract_features(ctx->c, const_cast<hamlss_mat*>(A), features, &st);
@@ -704,7 +700,7 @@ int hamlss_solve_adaptive(hamlss_ctx* ctx, const hamlss_mat* A, const double* b,
                           int where, const hamlss_params* params, hamlss_stats* stats,
                           hamlss_escalation* log, int32_t log_cap, int32_t* n_log,
                           int32_t* initial_state) {
-    return guarded([&]() -> int {
+    return on_lane(ctx, kSolveWait, [&]() -> int {
         if (!ctx || !A || !b || !x) return set_err(HAMLSS_ERR_INVALID, "null argument");
         if (A->A.n != A->A.m) return set_err(HAMLSS_ERR_SIZE, "solve needs a square matrix");
         hamlss_params p;
@@ -756,6 +752,9 @@ int hamlss_solve_adaptive(hamlss_ctx* ctx, const hamlss_mat* A, const double* b,
             r = solve_core(c, solver, Am, P.get(), io.b, io.x, p, &lad, &outer);
             double t2 = now_s();
             double e1 = p.record_hw_energy ? nvml_energy_j(c.device) : 0.0;
+            HAMLSS_CUDA(cudaStreamSynchronize(s));
+            // (before the next rung starts from this one's x)
+            if (lane_take_timeout(c.lane)) return set_err(HAMLSS_ERR_TIMEOUT, kSolveWait);
             if (r.status != HAMLSS_OK) return set_err(r.status, "non-finite values met during the solve");
             fill_stats(c, Am, solver, P.get(), r, t2 - t1, outer, e0, e1, io.b, io.x, &last);
             last.setup_time_s = setup + setup;     // stats.setup_time_s counted twice (:350-351)
@@ -778,8 +777,6 @@ int hamlss_solve_adaptive(hamlss_ctx* ctx, const hamlss_mat* A, const double* b,
         if (n_log) *n_log = nlog;
         if (where == HAMLSS_HOST) Am->ws.d[7].download(x, A->A.n, s);
         HAMLSS_CUDA(cudaStreamSynchronize(s));
-        if (lane_take_timeout(c.lane))
-            return set_err(HAMLSS_ERR_TIMEOUT, "a kernel of the solve gave up a bounded wait");
         return HAMLSS_OK;
     });
 }

@@ -24,8 +24,8 @@ def _gpu():
 
 @pytest.fixture
 def system():
-    """(matrix on a context of its own, the context's word, a right-hand side)"""
-    ctx = H.Context(0)
+    """(matrix, its context's word, a right-hand side)"""
+    ctx = H.Context.default()
     w = C.POINTER(C.c_int32)()
     assert H.lib().hamlss_ctx_wait_word(ctx.h, C.byref(w)) == 0 and w[0] == 0
     A = H.SparseMatrix(400, 400, *P.poisson_2d(20), ctx=ctx)
@@ -59,3 +59,48 @@ def test_failed_setup_leaves_no_word(system):
     with pytest.raises(H.HamlssError) as e:
         H.JacobiPreconditioner().setup(A)
     assert e.value.code == _abi.ERR_ZERO_DIAG
+
+
+@pytest.mark.parametrize("precond", ["JACOBI", "ILU", "AMG"])
+def test_nonfinite_solve_with_a_wait(system, precond):
+    # an abandoned kernel's leftovers are often not finite: the wait is what is reported
+    A, w, b = system
+    s, M = H.SolverFactory.make("FGMRES", precond, A, H.SolverParams(drop_tol=0.0))
+    bad = b.copy()
+    bad[3] = np.inf
+    w[0] = 1
+    with pytest.raises(H.HamlssError) as e:
+        s.solve(A, bad, np.zeros(400))
+    assert e.value.code == _abi.ERR_TIMEOUT and w[0] == 0
+    with pytest.raises(H.HamlssError) as e:
+        s.solve(A, bad, np.zeros(400))
+    assert e.value.code == _abi.ERR_NONFINITE
+    A.spmv(b)
+    x = np.zeros(400)
+    assert s.solve(A, b, x)
+
+
+@pytest.mark.parametrize("poison", [False, True])
+def test_adaptive_with_a_wait(system, poison):
+    A, w, b = system
+    b = b.copy()
+    if poison:
+        b[3] = np.inf
+    w[0] = 1
+    with pytest.raises(H.HamlssError) as e:
+        H.AdaptiveSelector(H.SolverParams()).solve(A, b, np.zeros(400))
+    assert e.value.code == _abi.ERR_TIMEOUT and w[0] == 0
+    A.spmv(np.ones(400))
+
+
+def test_every_other_call_takes_its_word(system):
+    A, w, b = system
+    M = H.ILUPreconditioner()
+    M.setup(A)
+    for call in (lambda: A.spmv(b), lambda: M.apply(b), lambda: H.amg_aggregate(A),
+                 lambda: H.AdaptiveSelector().extract_features(A)):
+        w[0] = 1
+        with pytest.raises(H.HamlssError) as e:
+            call()
+        assert e.value.code == _abi.ERR_TIMEOUT and w[0] == 0
+        call()
