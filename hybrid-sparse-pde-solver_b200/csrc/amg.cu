@@ -2719,6 +2719,10 @@ std::unique_ptr<Prec> make_amg(Ctx& ctx, hamlss_mat* A, const hamlss_params& p) 
             at.val.clusterDim.y = at.val.clusterDim.z = 1;
             cfg.attrs = &at;
             cfg.numAttrs = 1;
+            // (fewer blocks where the device holds no cluster of 16: the kernel strides by its grid)
+            int most = 0;
+            if (cudaOccupancyMaxPotentialClusterSize(&most, k_dense_factor, &cfg) != cudaSuccess) cudaGetLastError();
+            cfg.gridDim.x = at.val.clusterDim.x = std::max(1, std::min(kFactorBlocks, most));
             HAMLSS_CUDA(cudaLaunchKernelEx(&cfg, k_dense_factor, nc, W.p, M->Md.p, M->piv.p, M->skip.p));
         }
         phase(M->levels() - 1, "coarse LU");

@@ -298,47 +298,69 @@ struct FinTrip {
 };
 
 template <typename T, bool JAC, int SLOTS, bool CLUSTER, typename Fin>
-void launch_persist_t(Ctx& ctx, const PersistArgs<T>& a, CgState* s, int blocks, size_t smem, const Fin& fin) {
-    auto kern = k_cg_persist<T, JAC, SLOTS, CLUSTER, CgState, Fin>;
-    static DeviceOnce raised;
-    raised(ctx.device, [&] {
-        HAMLSS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPersistSmem));
-        if (CLUSTER) HAMLSS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    });
+struct PersistLaunch {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(a.rows <= 256 ? 256 : 512);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = ctx.lane.stream;
     cudaLaunchAttribute at{};
-    if (CLUSTER) {
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = blocks;
-        at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    } else {
-        at.id = cudaLaunchAttributeCooperative;
-        at.val.cooperative = 1;
-    }
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    HAMLSS_CUDA(cudaLaunchKernelEx(&cfg, kern, a, s, fin));
-}
+    static constexpr auto kern = k_cg_persist<T, JAC, SLOTS, CLUSTER, CgState, Fin>;
 
-template <typename T, bool JAC, bool CLUSTER, typename Fin>
-void launch_persist_c(Ctx& ctx, const PersistArgs<T>& a, CgState* s, int blocks, size_t smem, const Fin& fin) {
-    if (a.rows <= 512) launch_persist_t<T, JAC, 1, CLUSTER>(ctx, a, s, blocks, smem, fin);
-    else if (a.rows <= 1024) launch_persist_t<T, JAC, 2, CLUSTER>(ctx, a, s, blocks, smem, fin);
-    else if (a.rows <= 2048) launch_persist_t<T, JAC, 4, CLUSTER>(ctx, a, s, blocks, smem, fin);
-    else launch_persist_t<T, JAC, kPersistMaxSlots, CLUSTER>(ctx, a, s, blocks, smem, fin);
+    PersistLaunch(Ctx& ctx, int rows, int blocks, size_t smem) {
+        static DeviceOnce raised;
+        raised(ctx.device, [&] {
+            HAMLSS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPersistSmem));
+            if (CLUSTER) HAMLSS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        });
+        cfg.gridDim = dim3(blocks);
+        cfg.blockDim = dim3(rows <= 256 ? 256 : 512);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = ctx.lane.stream;
+        if (CLUSTER) {
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = blocks;
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        } else {
+            at.id = cudaLaunchAttributeCooperative;
+            at.val.cooperative = 1;
+        }
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+    }
+    bool can_run(Ctx& ctx) {
+        int clusters = 0, per_sm = 0;
+        const cudaError_t e = CLUSTER ? cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg)
+                                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                                            &per_sm, kern, (int)cfg.blockDim.x, cfg.dynamicSmemBytes);
+        if (e != cudaSuccess) cudaGetLastError();          // (a shape the device refuses)
+        return e == cudaSuccess && persist_can_run(CLUSTER, (int)cfg.gridDim.x, clusters, per_sm, ctx.sm_count);
+    }
+};
+
+// Calls f with the launch of the matrix's plan.
+template <typename T, bool JAC, typename Fin, typename F>
+void with_persist(Ctx& ctx, const hamlss_mat* A, F&& f) {
+    const int rows = A->persist_rows, blocks = ceil_div(A->A.n, rows);
+    const size_t smem = persist_smem<T>(A->persist_entries, A->persist_window);
+    auto by_rows = [&](auto cluster) {
+        constexpr bool C = decltype(cluster)::value;
+        if (rows <= 512) f(PersistLaunch<T, JAC, 1, C, Fin>(ctx, rows, blocks, smem));
+        else if (rows <= 1024) f(PersistLaunch<T, JAC, 2, C, Fin>(ctx, rows, blocks, smem));
+        else if (rows <= 2048) f(PersistLaunch<T, JAC, 4, C, Fin>(ctx, rows, blocks, smem));
+        else f(PersistLaunch<T, JAC, kPersistMaxSlots, C, Fin>(ctx, rows, blocks, smem));
+    };
+    if (A->persist_cluster) by_rows(std::true_type{});
+    else by_rows(std::false_type{});
 }
 
 // Whether the persistent iteration holds the matrix: its rows a block, their entries and the
 // columns they span fit a block's shared memory (about 500,000 rows of a 5-point grid in
-// FP64).  Otherwise the matrix streams from memory trip by trip and two launches a trip do.
-template <typename T>
+// FP64), and its blocks run at once.  Otherwise the matrix streams from memory trip by trip
+// and two launches a trip do.
+template <typename T, bool JAC, typename Fin>
 bool persist_fits(Ctx& ctx, hamlss_mat* A) {
     ensure_persist_plan(ctx, A);
-    return A->persist_rows > 0 && persist_smem<T>(A->persist_entries, A->persist_window) <= kPersistSmem;
+    if (A->persist_rows <= 0 || persist_smem<T>(A->persist_entries, A->persist_window) > kPersistSmem) return false;
+    bool ok = false;
+    with_persist<T, JAC, Fin>(ctx, A, [&](auto&& launch) { ok = launch.can_run(ctx); });
+    return ok;
 }
 
 // One launch of up to kPersistTrips trips from the state in memory (r, p, x and the
@@ -370,11 +392,10 @@ void launch_persist(Ctx& ctx, hamlss_mat* A, const Csr<T>& Ad, T* x, T* r, T* p,
     a.err = L.err.p;
     a.window = A->persist_window;
     a.entries = A->persist_entries;
-    const int blocks = ceil_div(Ad.n, a.rows);
-    const size_t smem = persist_smem<T>(a.entries, a.window);
     ProfScope ps(L, "cg_trips", csr_bytes(Ad) + (JAC ? 7.0 : 6.0) * sizeof(T) * Ad.n);
-    if (A->persist_cluster) launch_persist_c<T, JAC, true>(ctx, a, s, blocks, smem, fin);
-    else launch_persist_c<T, JAC, false>(ctx, a, s, blocks, smem, fin);
+    with_persist<T, JAC, Fin>(ctx, A, [&](auto&& launch) {
+        HAMLSS_CUDA(cudaLaunchKernelEx(&launch.cfg, launch.kern, a, s, fin));
+    });
 }
 
 template <typename T, bool JAC>
@@ -421,7 +442,7 @@ SolveResult cg_impl(Ctx& ctx, hamlss_mat* A, Prec* M, const T* b, T* x, double t
     restart_seq(true);
     poll(h);
     const bool run = !h.halt && max_iter > 0;
-    const bool persist = run && (JAC || !M) && persist_fits<T>(ctx, A);
+    const bool persist = run && (JAC || !M) && persist_fits<T, JAC, FinTrip<JAC>>(ctx, A);
     T* zp = persist ? wvec<T>(ws, 1, n) : nullptr;     // z of the persistent iteration
     int parity = 0;
     int chunk = std::max(1, check_every);
@@ -713,7 +734,7 @@ SolveResult cg_reliable_impl(Ctx& ctx, hamlss_mat* A, Prec* M, const double* b, 
     restart_seq(true);
     poll(h);
     const bool run = !h.halt && max_iter > 0;
-    const bool persist = run && JAC && persist_fits<float>(ctx, A);
+    const bool persist = run && JAC && persist_fits<float, true, FinTripRU>(ctx, A);
     float* zp = persist ? wvec<float>(ws, 1, n) : nullptr;     // z of the persistent iteration
     int parity = 0;
     int chunk = std::max(1, check_every);

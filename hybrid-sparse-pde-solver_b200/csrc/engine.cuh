@@ -5,6 +5,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "rules.hpp"
 #include "spmv.cuh"
 #include "spmv_stream.cuh"
 
@@ -131,12 +132,9 @@ constexpr double kSkewRatio = 32.0;
 void ensure_row_profile(Ctx& ctx, hamlss_mat* M);
 // Rows a block, and the entries and columns its rows span at most, of the persistent CG
 // (once per matrix; the pattern is fixed).
-constexpr int kPersistMaxRows = 3584;
-constexpr int kPersistClusterBlocks = 16;
 // (us a trip, Jacobi on grids: cluster 3.2 at 4,096 rows, 4.4 at 16,384, 6.7 at 32,761, 9.6 at
 // 48,841; grid 6.5 at 65,536, 8.0 at 160,000, 11.8 at 491,401)
 constexpr int kPersistClusterRows = 28672;
-constexpr int kPersistMaxBlocks = 256;
 constexpr size_t kPersistSmem = 224 * 1024;   // shared memory of a block beside the kernel's own
 // Shared memory of a block: p window, matrix values and 16-bit column offsets.
 template <typename T>

@@ -1,0 +1,42 @@
+"""The host-side rules that choose a kernel's form (csrc/rules.hpp), compiled on the CPU."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "hybrid-sparse-pde-solver_b200", "csrc")
+
+
+@pytest.fixture
+def evaluate(tmp_path):
+    """evaluate(expressions): their values as integers, from a program that includes rules.hpp"""
+
+    def run(exprs):
+        src = tmp_path / "rules.cpp"
+        exe = tmp_path / "rules"
+        lines = "".join(f'    std::printf("%lld\\n", (long long)({e}));\n' for e in exprs)
+        src.write_text('#include <cstdio>\n#include "rules.hpp"\nusing namespace hamlss;\n'
+                       f"int main() {{\n{lines}}}\n")
+        subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", "-I", CSRC, str(src), "-o", str(exe)], check=True)
+        return [int(x) for x in subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout.split()]
+
+    return run
+
+
+def test_persistent_cg_runs_only_where_its_blocks_run_together(evaluate):
+    cases = [
+        # cluster, blocks, active clusters, blocks an SM, SMs -> runs
+        ((1, 16, 8, 0, 148), 1),
+        ((1, 16, 0, 1, 148), 0),          # no GPC with that many SMs free
+        ((1, 17, 8, 1, 148), 0),
+        ((0, 148, 0, 1, 148), 1),
+        ((0, 148, 0, 1, 147), 0),
+        ((0, 148, 0, 0, 148), 0),         # not even one block an SM
+        ((0, 148, 0, 2, 74), 1),
+        ((0, 256, 0, 1, 300), 1),
+        ((0, 257, 0, 1, 300), 0),         # more blocks than sets of partial sums
+        ((0, 0, 0, 1, 148), 0),
+    ]
+    got = evaluate([f"persist_can_run({c[0]}, {c[1]}, {c[2]}, {c[3]}, {c[4]})" for c, _ in cases])
+    assert got == [want for _, want in cases]
