@@ -103,12 +103,19 @@ __global__ void k_jacobi_apply(int n, const T* __restrict__ inv, const T* __rest
         z[i] = (T)__dmul_rn((double)inv[i], (double)r[i]);
 }
 
-__global__ void k_row_len_max(int n, const int* __restrict__ rp, int* mx) {
-    int m = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+// mx[0]: the longest row; mx[1]: the most entries of `group` rows from a multiple of it (group > 0)
+__global__ void k_row_len_max(int n, const int* __restrict__ rp, int group, int* mx) {
+    int m = 0, g = 0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         m = max(m, rp[i + 1] - rp[i]);
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(mx, m);
+        if (group > 0 && i % group == 0) g = max(g, rp[min(n, i + group)] - rp[i]);
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    g = __reduce_max_sync(0xffffffffu, g);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&mx[0], m);
+        atomicMax(&mx[1], g);
+    }
 }
 
 __global__ void k_rows_longer(int n, const int* __restrict__ rp, int len, int* list, int* count) {
@@ -201,14 +208,17 @@ void ensure_row_profile(Ctx& ctx, hamlss_mat* M) {
     M->long_len = INT_MAX;
     if (n == 0) return;
     cudaStream_t s = ctx.lane.stream;
-    DBuf<int> cnt(1);
+    DBuf<int> cnt(2);
     cnt.zero(s);
     const int g = std::min(ceil_div(n, 256), ctx.sm_count * 8);
-    k_row_len_max<<<g, 256, 0, s>>>(n, M->A.rp.p, cnt.p);
+    const int R = prod_rows(ctx.sm_count, M->A.f64());
+    k_row_len_max<<<g, 256, 0, s>>>(n, M->A.rp.p, R, cnt.p);
     HAMLSS_LAUNCH_CHECK();
-    int h = 0;
-    cnt.download(&h, 1, s);
+    int hm[2];
+    cnt.download(hm, 2, s);
     HAMLSS_CUDA(cudaStreamSynchronize(s));
+    int h = hm[0];
+    M->A.uneven = R > 0 && prod_uneven(h, hm[1], M->A.nnz);
     const double avg = (double)M->A.nnz / n;
     if (h <= kSkewRow || h <= kSkewRatio * avg) return;
     const int len = std::max(kSkewRow, (int)std::ceil(kSkewRatio * avg));

@@ -124,7 +124,8 @@ void lane_destroy(Lane& L);
 // The caller has synchronised the lane's stream.  (A bulk-copy SpMV then read the matrix from
 // global memory, so its results stand; a triangular sweep's or persistent iteration's do not.)
 bool lane_take_timeout(const Lane& L);
-// The matrix's row-length profile for hamlss_spmv: when its longest row has more than
+// The matrix's row-length profile: whether neighbouring long rows make it uneven for
+// k_spmv_prod (DevMat::uneven, for every product with it), and for hamlss_spmv: when its longest row has more than
 // kSkewRow entries and more than kSkewRatio times the average, the rows above
 // max(kSkewRow, kSkewRatio x average) are listed (once per matrix; the pattern is fixed).
 constexpr int kSkewRow = 1024;
@@ -150,6 +151,7 @@ struct Csr {
     const int* rp = nullptr;
     const int* ci = nullptr;
     const T* v = nullptr;
+    bool uneven = false;      // long rows next to one another (prod_uneven)
 };
 
 // Owning device CSR (structure + FP64 values, FP32 values on demand).
@@ -159,7 +161,8 @@ struct DevMat {
     DBuf<double> v;
     DBuf<float> v32;
     bool v32_valid = false;
-    Csr<double> f64() const { return Csr<double>{n, m, nnz, rp.p, ci.p, v.p}; }
+    bool uneven = false;      // ensure_row_profile
+    Csr<double> f64() const { return Csr<double>{n, m, nnz, rp.p, ci.p, v.p, uneven}; }
     Csr<float> f32(cudaStream_t s);
 };
 
@@ -216,7 +219,7 @@ bool long_rows_warp(const Csr<T>& A) {
 // four warps an SM would have work.
 template <typename T>
 int prod_rows(int sm_count, const Csr<T>& A) {
-    if (sizeof(T) != 8 || A.n == 0) return 0;
+    if (sizeof(T) != 8 || A.n == 0 || A.uneven) return 0;
     const double avg = (double)A.nnz / A.n;
     if (avg <= 5.5) return 0;
     const int fit = (int)(kProdFill * kProdTile / avg), share = A.n / (4 * sm_count);

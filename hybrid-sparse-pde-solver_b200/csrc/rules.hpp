@@ -21,4 +21,21 @@ inline bool persist_can_run(bool cluster, int blocks, int active_clusters, int b
     return blocks <= kPersistMaxBlocks && (long long)blocks_per_sm * sm_count >= blocks;
 }
 
+// --------------------------------------------------------------- FP64 products (spmv.cuh)
+constexpr int kProdTile = 512;                // products a warp of k_spmv_prod holds
+
+// Whether a matrix of long rows next to one another is left to a lane a row (k_spmv): all
+// entries of the rows that one warp takes (`heaviest`: the most of any warp) go through its
+// tile, and where a tile holds one row's part, one lane adds it while 31 wait.  Cycles of the
+// slowest warp, measured: a tile ~1,500 for its loads and ~12 an addition; a lane a row ~225 an
+// entry.  The rest of the matrix runs beside that warp and prefers k_spmv_prod by about a
+// 200th of a cycle an entry.  A product of 100,000 rows of 10 with 40 neighbouring rows longer,
+// k_spmv_prod / k_spmv: of 100 31 / 31 us, of 300 66 / 48, of 900 184 / 108; with 8 rows of 900
+// 72 / 101.
+inline bool prod_uneven(int longest, long long heaviest, long long nnz) {
+    const long long tiles = (heaviest + kProdTile - 1) / kProdTile;
+    const long long warp = tiles * (1500 + 12LL * std::min(longest, kProdTile));
+    return warp - 225LL * longest > nnz / 200;
+}
+
 }  // namespace hamlss

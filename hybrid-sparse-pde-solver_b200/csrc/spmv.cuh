@@ -249,7 +249,6 @@ k_spmv_rows_seq(const int* __restrict__ rows, int nrows, const int* __restrict__
 // aggregation levels.  Measured, lane a row -> this: 300,007 x 24 ragged 53 -> 36 us, 50,021
 // x 100 107 -> 47 us, an FP64 V-cycle on 1024^2 2.19 -> 0.93 ms.
 constexpr int kProdWarps = 8;
-constexpr int kProdTile = 512;               // products a warp holds
 constexpr double kProdFill = 0.85;           // average share of them its rows take
 constexpr int kProdLoads = 8;                // entries a lane loads at a time
 

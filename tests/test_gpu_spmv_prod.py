@@ -66,3 +66,37 @@ def test_nonfinite_entries_stay_in_their_rows():
     y = H.SparseMatrix(3000, 3000, *A).spmv(x)
     bad = ~np.isfinite(y)
     assert np.array_equal(np.flatnonzero(bad), [0, 700])
+
+
+def grouped(name, rng):
+    """Row lengths with neighbouring long rows, at both sides of the rule that leaves them to
+    a lane a row."""
+    if name == "long_at_the_end":
+        return np.concatenate([np.full(20011, 8), np.full(19, 900)])
+    if name == "long_in_front":
+        return np.concatenate([np.full(50, 900), np.full(20000, 8)])
+    if name == "uneven":                     # long, short and empty rows side by side
+        out = np.full(20000, 7)
+        out[5000:5064] = rng.integers(0, 600, 64)
+        out[9000:9032:2] = 997
+        out[9001:9033:2] = 0
+        return out
+    if name == "few":                        # too few to matter
+        return np.concatenate([np.full(9000, 9), np.full(6, 900), np.full(9000, 9)])
+    return np.concatenate([np.full(3000, 50), np.full(64, 1500), np.full(3000, 50)])   # "wide"
+
+
+@pytest.mark.parametrize("name", ["long_at_the_end", "long_in_front", "uneven", "few", "wide"])
+def test_neighbouring_long_rows_bitwise(name):
+    rng = np.random.default_rng(7)
+    ln = grouped(name, rng)
+    n, m = len(ln), 30000
+    A = from_lengths(ln, m, 11)
+    x = rng.standard_normal(m)
+    y = H.SparseMatrix(n, m, *A).spmv(x)
+    ref = np.zeros(n)
+    prod = A[2] * x[A[1]]
+    for k in range(int(ln.max())):           # column order, every row at once
+        has = ln > k
+        ref[has] = ref[has] + prod[A[0][:-1][has] + k]
+    assert np.array_equal(y, ref)

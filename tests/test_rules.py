@@ -40,3 +40,19 @@ def test_persistent_cg_runs_only_where_its_blocks_run_together(evaluate):
     ]
     got = evaluate([f"persist_can_run({c[0]}, {c[1]}, {c[2]}, {c[3]}, {c[4]})" for c, _ in cases])
     assert got == [want for _, want in cases]
+
+
+def test_uneven_rows_leave_the_product_tiles(evaluate):
+    # 100,000 rows of 10 and some neighbouring longer ones, 32 of them a warp at most
+    cases = [
+        ((10, 320, 1000000), 0),
+        ((100, 3200, 1003528), 0),
+        ((300, 32 * 300, 1011463), 1),
+        ((900, 32 * 900, 1035271), 1),
+        ((900, 8 * 900, 1006996), 0),
+        ((900, 900 + 31 * 10, 1000900), 0),
+        ((3000, 3000, 9000000), 0),                       # a dense matrix: a row a warp
+        ((900, 32 * 900, 300000000), 0),                  # hidden behind the rest of the matrix
+        ((2 ** 31 - 1, 2 ** 31 - 1, 2 ** 31 - 1), 0),
+    ]
+    assert evaluate([f"prod_uneven({a}, {b}LL, {c}LL)" for (a, b, c), _ in cases]) == [w for _, w in cases]
