@@ -118,6 +118,23 @@ __global__ void k_row_len_max(int n, const int* __restrict__ rp, int group, int*
     }
 }
 
+// near[0] += places k that rows i and i + 1 both have, near[1] += those whose columns lie at
+// most kNearColumns apart; every `stride`-th row, the first eight places
+__global__ void k_row_neighbours(int n, int stride, const int* __restrict__ rp, const int* __restrict__ ci, int* near) {
+    int pairs = 0, close = 0;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; (long long)t * stride < n - 1; t += gridDim.x * blockDim.x) {
+        const int i = t * stride, a = rp[i], b = rp[i + 1], len = min(8, min(b - a, rp[i + 2] - b));
+        pairs += max(len, 0);
+        for (int k = 0; k < len; ++k) close += abs(ci[a + k] - ci[b + k]) <= kNearColumns;
+    }
+    pairs = __reduce_add_sync(0xffffffffu, pairs);
+    close = __reduce_add_sync(0xffffffffu, close);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&near[0], pairs);
+        atomicAdd(&near[1], close);
+    }
+}
+
 __global__ void k_rows_longer(int n, const int* __restrict__ rp, int len, int* list, int* count) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         if (rp[i + 1] - rp[i] > len) list[atomicAdd(count, 1)] = i;
@@ -208,16 +225,23 @@ void ensure_row_profile(Ctx& ctx, hamlss_mat* M) {
     M->long_len = INT_MAX;
     if (n == 0) return;
     cudaStream_t s = ctx.lane.stream;
-    DBuf<int> cnt(2);
+    DBuf<int> cnt(4);
     cnt.zero(s);
     const int g = std::min(ceil_div(n, 256), ctx.sm_count * 8);
     const int R = prod_rows(ctx.sm_count, M->A.f64());
     k_row_len_max<<<g, 256, 0, s>>>(n, M->A.rp.p, R, cnt.p);
     HAMLSS_LAUNCH_CHECK();
-    int hm[2];
-    cnt.download(hm, 2, s);
+    if (stream_group(M->A.f64()) == 1) {
+        const int stride = std::max(1, n / kNeighbourRows);
+        k_row_neighbours<<<std::min(ceil_div(n / stride, 256), ctx.sm_count * 8), 256, 0, s>>>(
+            n, stride, M->A.rp.p, M->A.ci.p, cnt.p + 2);
+        HAMLSS_LAUNCH_CHECK();
+    }
+    int hm[4];
+    cnt.download(hm, 4, s);
     HAMLSS_CUDA(cudaStreamSynchronize(s));
     int h = hm[0];
+    M->A.scattered = gathers_scattered(hm[2], hm[3]);
     M->A.uneven = R > 0 && prod_uneven(h, hm[1], M->A.nnz);
     const double avg = (double)M->A.nnz / n;
     if (h <= kSkewRow || h <= kSkewRatio * avg) return;

@@ -124,8 +124,9 @@ void lane_destroy(Lane& L);
 // The caller has synchronised the lane's stream.  (A bulk-copy SpMV then read the matrix from
 // global memory, so its results stand; a triangular sweep's or persistent iteration's do not.)
 bool lane_take_timeout(const Lane& L);
-// The matrix's row-length profile: whether neighbouring long rows make it uneven for
-// k_spmv_prod (DevMat::uneven, for every product with it), and for hamlss_spmv: when its longest row has more than
+// The matrix's row profile: whether neighbouring long rows make it uneven for k_spmv_prod, or
+// neighbouring rows' columns lie apart (DevMat's flags, for every product with it); and for
+// hamlss_spmv: when its longest row has more than
 // kSkewRow entries and more than kSkewRatio times the average, the rows above
 // max(kSkewRow, kSkewRatio x average) are listed (once per matrix; the pattern is fixed).
 constexpr int kSkewRow = 1024;
@@ -152,6 +153,7 @@ struct Csr {
     const int* ci = nullptr;
     const T* v = nullptr;
     bool uneven = false;      // long rows next to one another (prod_uneven)
+    bool scattered = false;   // neighbouring rows' columns lie apart (gathers_scattered)
 };
 
 // Owning device CSR (structure + FP64 values, FP32 values on demand).
@@ -161,8 +163,8 @@ struct DevMat {
     DBuf<double> v;
     DBuf<float> v32;
     bool v32_valid = false;
-    bool uneven = false;      // ensure_row_profile
-    Csr<double> f64() const { return Csr<double>{n, m, nnz, rp.p, ci.p, v.p, uneven}; }
+    bool uneven = false, scattered = false;      // ensure_row_profile
+    Csr<double> f64() const { return Csr<double>{n, m, nnz, rp.p, ci.p, v.p, uneven, scattered}; }
     Csr<float> f32(cudaStream_t s);
 };
 
@@ -244,10 +246,10 @@ int stream_per_sm(K kernel, size_t smem) {
     return std::min(occupancy_blocks(kernel, kStreamThreads, smem), kMaxBlocksPerSm);
 }
 
-template <typename T, int NRED, typename XOp, typename Epi, typename Fin, int G>
+template <typename T, int NRED, typename XOp, typename Epi, typename Fin, int G, bool WIDE = false>
 void launch_spmv_stream(int sm_count, const Lane& L, const Csr<T>& A, const XOp& xop, const Epi& epi,
                         const Fin& fin, const int* gate, int skip_len) {
-    auto kern = k_spmv_stream<T, NRED, XOp, Epi, Fin, G>;
+    auto kern = k_spmv_stream<T, NRED, XOp, Epi, Fin, G, WIDE>;
     constexpr size_t smem = StreamShape<T>::smem_bytes;
     static const int per_sm = stream_per_sm(kern, smem);
     const int tiles = ceil_div(A.n, kStreamThreads / G);
@@ -264,7 +266,12 @@ void launch_spmv(int sm_count, const Lane& L, const Csr<T>& A, const XOp& xop, c
                  double vec_bytes = -1.0, int skip_len = INT_MAX) {
     ProfScope ps(L, name, csr_bytes(A) + (vec_bytes >= 0 ? vec_bytes : 2.0 * sizeof(T) * A.n));
     switch (stream_group(A)) {
-        case 1: return launch_spmv_stream<T, NRED, XOp, Epi, Fin, 1>(sm_count, L, A, xop, epi, fin, gate, skip_len);
+        case 1:
+            if constexpr (sizeof(T) == 8 && NRED == 0)
+                if (A.scattered)
+                    return launch_spmv_stream<T, NRED, XOp, Epi, Fin, 1, true>(sm_count, L, A, xop, epi, fin, gate,
+                                                                               skip_len);
+            return launch_spmv_stream<T, NRED, XOp, Epi, Fin, 1>(sm_count, L, A, xop, epi, fin, gate, skip_len);
         case 2:
             if constexpr (sizeof(T) == 4)
                 return launch_spmv_stream<T, NRED, XOp, Epi, Fin, 2>(sm_count, L, A, xop, epi, fin, gate, skip_len);

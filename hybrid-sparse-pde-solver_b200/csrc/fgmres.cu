@@ -360,7 +360,8 @@ SolveResult fgmres_solve(Ctx& ctx, hamlss_mat* A, Prec* M, const double* b, doub
     const Lane& L = ctx.lane;
     const int sm = ctx.sm_count;
     cudaStream_t st = L.stream;
-    if (prod_rows(sm, A->A.f64())) ensure_row_profile(ctx, A);
+    // (how its products go: only where a product is long against the profile's ~20 us)
+    if (A->A.nnz >= (1 << 17)) ensure_row_profile(ctx, A);
     const long long ld = ((long long)n + 31) / 32 * 32;      // keep every basis vector 256-B aligned
     const bool flex = M != nullptr;
     ws.basis.ensure((size_t)ld * (size_t)(m + 1 + (flex ? m : 0)));

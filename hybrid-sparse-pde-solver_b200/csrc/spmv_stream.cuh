@@ -118,6 +118,15 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned b
 // 21.5 KB x 2 stages, FP64 19.5 KB x 2 stages, five CTAs per SM both.  FP64 on the 2048^2
 // 5-point operator (a product with vectors, device time): 3 stages at three CTAs 76.6 us, 2
 // at four or five 59.5 us (5.6 TB/s) -- more warps to wait for their gathers, not more stages.
+//
+// Registers decide what a row's gathers overlap with.  At five CTAs (48 a thread) a product's
+// gathers go one after another, which costs nothing where neighbouring rows' columns share
+// lines.  Where they do not (Csr::scattered: each gather waits for L2) the form with all of a
+// row's gathers in flight (WIDE, 64 registers, four CTAs) is the better one: the rows of the
+// 2048^2 operator in random order 199 -> 94 us a product, in order 60 -> 64 us.  Products with
+// sums (CG's, whose operand is formed from three vectors) take 64 registers always: 100 trips
+// of CG + Jacobi in random order 68 ms at three stages and CTAs, 129 at five CTAs, 54 here; in
+// order 15.8, 14.3, 14.4 ms.
 // FP32, measured
 // on the 2048^2 hierarchy (V-cycle SpMVs, GB/s): 1536 entries x 3 stages at five CTAs
 // 2456; 3072 x 2 at four 3007; 2560 x 2 at five 3218; 4096 x 2 at three 2800; 3072 x 3 at
@@ -128,6 +137,7 @@ struct StreamShape {
     static constexpr int K = sizeof(T) == 8 ? 1536 : 2560;
     static constexpr int S = 2;
     static constexpr int kMinBlocks = 5;   // CTAs per SM the smem allows
+    static constexpr int kWideBlocks = sizeof(T) == 8 ? 4 : 5;   // with more registers a thread
     static constexpr int kTrMax = kStreamThreads;            // rows per tile with G = 1
     static constexpr size_t rp_bytes = (kTrMax + 4) * 4;
     static constexpr size_t ci_bytes = (K + 4) * 4;
@@ -174,8 +184,9 @@ __device__ __forceinline__ void stream_issue(unsigned char* smem, int s, uint64_
     }
 }
 
-template <typename T, int NRED, typename XOp, typename Epi, typename Fin, int G>
-__global__ void __launch_bounds__(kStreamThreads, StreamShape<T>::kMinBlocks)
+template <typename T, int NRED, typename XOp, typename Epi, typename Fin, int G, bool WIDE = false>
+__global__ void __launch_bounds__(kStreamThreads, NRED > 0 || WIDE ? StreamShape<T>::kWideBlocks
+                                                                   : StreamShape<T>::kMinBlocks)
 k_spmv_stream(int n, const int* __restrict__ rp, const int* __restrict__ ci, const T* __restrict__ v,
               XOp xop, Epi epi, Reducer red, Fin fin, const int* gate, int* err, int skip_len) {
     constexpr int S = StreamShape<T>::S;
@@ -302,11 +313,26 @@ k_spmv_stream(int n, const int* __restrict__ rp, const int* __restrict__ ci, con
                 sum = mul_add<T>(sum, a2, x2);
                 sum = mul_add<T>(sum, a3, x3);
             }
-            for (; k < re; k += G) {
-                T a;
-                int c;
-                entry(k, a, c);
-                sum = mul_add<T>(sum, a, xop_l(c));
+            if constexpr (WIDE) {
+                T a[3];
+                int c[3];
+                double x[3];
+#pragma unroll
+                for (int u = 0; u < 3; ++u)
+                    if (k + u * G < re) entry(k + u * G, a[u], c[u]);
+#pragma unroll
+                for (int u = 0; u < 3; ++u)
+                    if (k + u * G < re) x[u] = xop_l(c[u]);
+#pragma unroll
+                for (int u = 0; u < 3; ++u)
+                    if (k + u * G < re) sum = mul_add<T>(sum, a[u], x[u]);
+            } else {
+                for (; k < re; k += G) {
+                    T a;
+                    int c;
+                    entry(k, a, c);
+                    sum = mul_add<T>(sum, a, xop_l(c));
+                }
             }
         }
         if constexpr (G > 1) {

@@ -56,3 +56,9 @@ def test_uneven_rows_leave_the_product_tiles(evaluate):
         ((2 ** 31 - 1, 2 ** 31 - 1, 2 ** 31 - 1), 0),
     ]
     assert evaluate([f"prod_uneven({a}, {b}LL, {c}LL)" for (a, b, c), _ in cases]) == [w for _, w in cases]
+
+
+def test_scattered_gathers(evaluate):
+    assert evaluate([f"gathers_scattered({p}, {q})" for p, q in
+                     [(0, 0), (320000, 319000), (320000, 160000), (320000, 159999), (320000, 12),
+                      (8 * 65536 * 2, 8 * 65536), (1, 0), (1, 1)]]) == [0, 0, 0, 1, 1, 0, 1, 0]
