@@ -303,14 +303,14 @@ struct PersistLaunch {
     cudaLaunchAttribute at{};
     static constexpr auto kern = k_cg_persist<T, JAC, SLOTS, CLUSTER, CgState, Fin>;
 
-    PersistLaunch(Ctx& ctx, int rows, int blocks, size_t smem) {
+    PersistLaunch(Ctx& ctx, int rows, int window, int blocks, size_t smem) {
         static DeviceOnce raised;
         raised(ctx.device, [&] {
             HAMLSS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPersistSmem));
             if (CLUSTER) HAMLSS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         });
         cfg.gridDim = dim3(blocks);
-        cfg.blockDim = dim3(rows <= 256 ? 256 : 512);
+        cfg.blockDim = dim3(persist_threads(rows, window - rows));
         cfg.dynamicSmemBytes = smem;
         cfg.stream = ctx.lane.stream;
         if (CLUSTER) {
@@ -337,14 +337,14 @@ struct PersistLaunch {
 // Calls f with the launch of the matrix's plan.
 template <typename T, bool JAC, typename Fin, typename F>
 void with_persist(Ctx& ctx, const hamlss_mat* A, F&& f) {
-    const int rows = A->persist_rows, blocks = ceil_div(A->A.n, rows);
+    const int rows = A->persist_rows, window = A->persist_window, blocks = ceil_div(A->A.n, rows);
     const size_t smem = persist_smem<T>(A->persist_entries, A->persist_window);
     auto by_rows = [&](auto cluster) {
         constexpr bool C = decltype(cluster)::value;
-        if (rows <= 512) f(PersistLaunch<T, JAC, 1, C, Fin>(ctx, rows, blocks, smem));
-        else if (rows <= 1024) f(PersistLaunch<T, JAC, 2, C, Fin>(ctx, rows, blocks, smem));
-        else if (rows <= 2048) f(PersistLaunch<T, JAC, 4, C, Fin>(ctx, rows, blocks, smem));
-        else f(PersistLaunch<T, JAC, kPersistMaxSlots, C, Fin>(ctx, rows, blocks, smem));
+        if (rows <= 512) f(PersistLaunch<T, JAC, 1, C, Fin>(ctx, rows, window, blocks, smem));
+        else if (rows <= 1024) f(PersistLaunch<T, JAC, 2, C, Fin>(ctx, rows, window, blocks, smem));
+        else if (rows <= 2048) f(PersistLaunch<T, JAC, 4, C, Fin>(ctx, rows, window, blocks, smem));
+        else f(PersistLaunch<T, JAC, kPersistMaxSlots, C, Fin>(ctx, rows, window, blocks, smem));
     };
     if (A->persist_cluster) by_rows(std::true_type{});
     else by_rows(std::false_type{});

@@ -62,3 +62,9 @@ def test_scattered_gathers(evaluate):
     assert evaluate([f"gathers_scattered({p}, {q})" for p, q in
                      [(0, 0), (320000, 319000), (320000, 160000), (320000, 159999), (320000, 12),
                       (8 * 65536 * 2, 8 * 65536), (1, 0), (1, 1)]]) == [0, 0, 0, 1, 1, 0, 1, 0]
+
+
+def test_persistent_cg_threads(evaluate):
+    assert evaluate([f"persist_threads({r}, {o})" for r, o in
+                     [(256, 0), (256, 4096), (256, 4097), (256, 24000), (288, 0), (3584, 100)]]) == \
+        [256, 256, 512, 512, 512, 512]
