@@ -15,7 +15,7 @@
 //   3. level-ordered copies of L (strictly lower part) and U (diagonal + upper part), so
 //      the rows of one level are contiguous in memory.
 // Apply: forward then backward sweep, each by the kernel its triangle's shape asks for
-// (TriMode below).  The arithmetic per row is the reference's (ilu.cpp:230-237, :249-260),
+// (tri_mode, rules.hpp).  The arithmetic per row is the reference's (ilu.cpp:230-237, :249-260),
 // so z is bit-identical to ILUPreconditioner::apply.
 #include <cooperative_groups.h>
 
@@ -1087,16 +1087,7 @@ void coop_launch(cudaStream_t s, K kernel, int blocks, int threads, Args... args
 }  // namespace
 
 // ---------------------------------------------------------------------- the object
-// Kernel of a triangle's sweep, by its shape:
-//   GRID   more than 4,096 rows a level on average: the whole grid, a grid barrier (~2 us) a
-//          level; one block would spend longer than that on a level's rows
-//   RING   otherwise, rows of at most 16 entries: one block, shared-memory rings
-//          (0.15 to 0.37 us a level)
-//   BLOCK  otherwise (a step of the ring kernel would hold too few rows): one block reading
-//          through the caches (~1.1 us a level)
-enum class TriMode { RING, BLOCK, GRID };
-constexpr int kTriMaxRow = 16;
-
+// (the kernel of a triangle's sweep: tri_mode, rules.hpp)
 struct Triangle {
     int nlev = 0, nnz = 0, max_row = 0, max_width = 0;
     TriMode mode = TriMode::GRID;
@@ -1115,11 +1106,13 @@ inline std::tuple<DBuf<float>&, DBuf<float>&, DBuf<int>&> tri_bufs(Triangle& t, 
 
 // Calls f(std::integral_constant<int, K>) with the entry places a RING triangle's rows get.
 template <typename F>
-void tri_places(const Triangle& t, F&& f) {
-    if (t.max_row <= 2) f(std::integral_constant<int, 2>{});
-    else if (t.max_row <= 4) f(std::integral_constant<int, 4>{});
-    else if (t.max_row <= 8) f(std::integral_constant<int, 8>{});
-    else f(std::integral_constant<int, 16>{});
+void with_places(const Triangle& t, F&& f) {
+    switch (tri_places(t.max_row)) {
+        case 2: return f(std::integral_constant<int, 2>{});
+        case 4: return f(std::integral_constant<int, 4>{});
+        case 8: return f(std::integral_constant<int, 8>{});
+        default: return f(std::integral_constant<int, 16>{});
+    }
 }
 
 template <typename T, int K, TriOp OP>
@@ -1168,7 +1161,7 @@ struct IluPrec : Prec {
     template <typename T, bool DIV>
     void pack(Ctx& ctx, Triangle& t, const int* pos, int* far, int* bad) {
         constexpr TriOp op = DIV ? TriOp::BACKWARD : TriOp::FORWARD;
-        tri_places(t, [&](auto k) {
+        with_places(t, [&](auto k) {
             constexpr int K = decltype(k)::value;
             constexpr int RB = TriShape<T, K, op>::RB;
             const int rows = ceil_div(n, RB) * RB;
@@ -1186,7 +1179,7 @@ struct IluPrec : Prec {
     template <bool DIV>
     void make_steps(Ctx& ctx, Triangle& t) {
         constexpr TriOp op = DIV ? TriOp::BACKWARD : TriOp::FORWARD;
-        tri_places(t, [&](auto k) {
+        with_places(t, [&](auto k) {
             constexpr int K = decltype(k)::value;
             t.step_rows = std::min(TriShape<double, K, op>::max_rows, TriShape<float, K, op>::max_rows);
         });
@@ -1210,7 +1203,7 @@ struct IluPrec : Prec {
         if (t.mode == TriMode::RING) {
             constexpr TriOp op = DIV ? TriOp::BACKWARD : TriOp::FORWARD;
             const TriView<T> F{n, t.nsteps, t.sptr.p, tv.p, tcode.p, tdg.p, nullptr, nullptr, nullptr};
-            tri_places(t, [&](auto k) {
+            with_places(t, [&](auto k) {
                 constexpr int K = decltype(k)::value;
                 launch_tri<T, K, op>(ctx, ln, t.far, t.step_rows, F, rhs, out, gate);
             });
@@ -1489,8 +1482,7 @@ void finish_ilu(Ctx& ctx, IluPrec* P, bool factorise) {
         k_level_sort<<<std::min(t.nlev, ctx.sm_count * 8), 256, 0, s>>>(t.nlev, t.lptr.p, t.ord.p, facts.p + 7 + k);
         k_invert<<<g, 256, 0, s>>>(n, t.ord.p, pos[k].p);
         HAMLSS_LAUNCH_CHECK();
-        const bool wide = (double)n / t.nlev > 4096.0;
-        t.mode = wide ? TriMode::GRID : t.max_row <= kTriMaxRow ? TriMode::RING : TriMode::BLOCK;
+        t.mode = tri_mode(n, t.nlev, hf[5 + k], t.max_row);
     }
     int hw[2];
     HAMLSS_CUDA(cudaMemcpyAsync(hw, facts.p + 7, sizeof(hw), cudaMemcpyDeviceToHost, s));

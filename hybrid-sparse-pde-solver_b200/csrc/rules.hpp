@@ -54,4 +54,38 @@ constexpr int kNearColumns = 8;
 constexpr int kNeighbourRows = 65536;         // rows looked at, about
 inline bool gathers_scattered(int pairs, int near) { return pairs > 0 && 2LL * near < pairs; }
 
+// ---------------------------------------------------------- triangular sweeps (ilu_sweep.cuh)
+// Kernel of a triangle's sweep:
+//   RING   one block, shared-memory rings, rows of at most 16 entries in 2, 4, 8 or 16 places
+//   BLOCK  one block reading through the caches
+//   GRID   the whole grid, a grid barrier (~2 us) a level
+enum class TriMode { RING, BLOCK, GRID };
+constexpr int kTriMaxRow = 16;
+
+// Entry places of a RING triangle's rows, from its longest row.
+inline int tri_places(int max_row) { return max_row <= 2 ? 2 : max_row <= 4 ? 4 : max_row <= 8 ? 8 : 16; }
+
+// More than 4,096 rows a level on average: GRID (one block spends longer than a grid barrier
+// on a level's rows).  Otherwise RING wherever its rows need 2 or 4 places (1.1 to 2 times
+// BLOCK at every width, 200 to 4,000 rows a level of 1 to 4 entries).  With 8 and 16 places all
+// rows pay for the longest one -- their empty places are copied too, and a step holds 416 or 224
+// rows -- so RING and BLOCK are weighed.  Microseconds, measured: a RING step 0.3 and 0.003 a row
+// (8 places), 0.35 and 0.0087 a row (16); a BLOCK level 0.95 and 0.00065 an entry, 0.0009 where
+// rows have more than 8 on average.  An apply, RING / BLOCK: 8 of 8 places used, 500 rows a level
+// 0.22 / 0.43 ms, 4,000 1.93 / 2.66; 2 of 8, 2,000 a level 0.95 / 0.56; 16 of 16, 500 a level 0.59 /
+// 1.13; 4 of 16, 2,000 a level 2.48 / 0.76; one row of 14 in a 512^2 grid's rows of 2 3.4 / 2.3.
+inline TriMode tri_mode(int n, int nlev, int nnz, int max_row) {
+    if (nlev < 1) return TriMode::BLOCK;
+    const double width = (double)n / nlev;
+    if (width > 4096.0) return TriMode::GRID;
+    if (max_row > kTriMaxRow) return TriMode::BLOCK;
+    const int K = tri_places(max_row);
+    if (K <= 4) return TriMode::RING;
+    const double rows = K == 8 ? 416.0 : 224.0;                        // a step
+    const double steps = nlev * std::max(1.0, width / rows + 0.5);     // (a level's last is partly filled)
+    const double ring = K == 8 ? 0.3 * steps + 0.003 * n : 0.35 * steps + 0.0087 * n;
+    const double block = 0.95 * nlev + (nnz > 8.0 * n ? 0.0009 : 0.00065) * nnz;
+    return ring <= block ? TriMode::RING : TriMode::BLOCK;
+}
+
 }  // namespace hamlss

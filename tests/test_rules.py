@@ -68,3 +68,32 @@ def test_persistent_cg_threads(evaluate):
     assert evaluate([f"persist_threads({r}, {o})" for r, o in
                      [(256, 0), (256, 4096), (256, 4097), (256, 24000), (288, 0), (3584, 100)]]) == \
         [256, 256, 512, 512, 512, 512]
+
+
+def test_sweep_kernel_by_shape(evaluate):
+    ring, block, grid = evaluate([f"TriMode::{m}" for m in ("RING", "BLOCK", "GRID")])
+    cases = [
+        # rows, levels, entries, longest row
+        ((262144, 1023, 523264, 2), ring),               # 512^2 grid
+        ((262144, 1477, 523276, 14), block),             # ... with one row of 14
+        ((262144, 1456, 523268, 6), ring),               # ... of 6: RING is still the better one
+        ((120000, 60, 480000, 16), block),               # 4 of 16 places used, 2,000 rows a level
+        ((18000, 60, 72000, 16), block),
+        ((30000, 60, 480000, 16), ring),                 # all 16 used
+        ((120000, 60, 240000, 8), block),                # 2 of 8 used
+        ((120000, 60, 480000, 8), block),
+        ((12000, 60, 24000, 8), ring),                   # narrow levels
+        ((18000, 60, 36000, 8), ring),
+        ((240000, 60, 1920000, 8), ring),                # all 8 used
+        ((65536, 1021, 780000, 12), ring),               # 25-point stencil on 256^2
+        ((49152, 765, 340000, 8), ring),                 # three unknowns a node
+        ((240000, 60, 240000, 1), ring),
+        ((240000, 60, 960000, 4), ring),
+        ((30000, 60, 500000, 17), block),
+        ((16384, 2, 32000, 2), grid),
+        ((1, 1, 0, 0), ring),
+        ((0, 0, 0, 0), block),
+    ]
+    got = evaluate([f"tri_mode({n}, {lv}, {nz}, {mr})" for (n, lv, nz, mr), _ in cases])
+    assert got == [want for _, want in cases]
+    assert evaluate([f"tri_places({k})" for k in (0, 1, 2, 3, 4, 5, 8, 9, 16)]) == [2, 2, 2, 4, 4, 8, 8, 16, 16]
