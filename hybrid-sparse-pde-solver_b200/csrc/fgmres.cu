@@ -211,6 +211,53 @@ k_mdot(int n, int nv, const double* __restrict__ V, long long ld, double* w,
     }
 }
 
+// The same with a thread an entry, for few vectors: each entry's chain over the vectors is
+// short then, w is read once instead of by every warp that has a vector, and no warp is without
+// one.  4 M entries, an average of the three modes, this / k_mdot: 1 vector 27 / 45 us, up to 4 41 /
+// 55, up to 8 52 / 62, up to 10 65 / 68, up to 16 102 / 83; 1 M entries 14 / 18, 15 / 19, 18 / 20; 260,000
+// 12.4 / 13.4, 12.8 / 13.7, 14.3 / 13.9; below that the launch is most of either.
+template <int NV, int MODE, typename Fin>
+__global__ void __launch_bounds__(256)
+k_mdot_few(int n, int nv, const double* __restrict__ V, long long ld, double* w,
+           const double* __restrict__ hprev, Reducer red, Fin fin, const int* gate) {
+    constexpr int NR = MODE == 2 ? 1 : NV;
+    __shared__ double hp[NV];
+    __shared__ double rsh[8 * NR];
+    if (gate && *(volatile const int*)gate) return;
+    if (MODE >= 1) {
+        for (int k = threadIdx.x; k < NV; k += blockDim.x) hp[k] = k < nv ? hprev[k] : 0.0;
+        __syncthreads();
+    }
+    double acc[NR];
+#pragma unroll
+    for (int k = 0; k < NR; ++k) acc[k] = 0.0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        double wi = w[i];
+        if (MODE >= 1) {
+#pragma unroll
+            for (int k = 0; k < NV; ++k)
+                if (k < nv) wi -= hp[k] * __ldg(&V[k * ld + i]);
+            w[i] = wi;
+        }
+        if (MODE <= 1) {
+#pragma unroll
+            for (int k = 0; k < NV; ++k)
+                if (k < nv) acc[k] += __ldg(&V[k * ld + i]) * wi;
+        } else {
+            acc[0] += wi * wi;
+        }
+    }
+    double tot[NR];
+    if (!grid_reduce<NR>(red, acc, rsh, tot)) return;
+    if constexpr (MODE == 2) {
+        fin(tot);
+    } else {
+#pragma unroll
+        for (int k = 0; k < NV; ++k)
+            if (k < nv) fin(k, tot[k]);
+    }
+}
+
 struct FinH1 {                                             // a thread a vector
     GmArrays a;
     int j;
@@ -327,15 +374,19 @@ void launch_mdot_t(Ctx& ctx, int mode, int n, int nv, const double* V, long long
     int blocks = std::max(1, std::min(ceil_div(n, 256), ctx.sm_count * 4));
     L.red_check(blocks, mode == 2 ? 1 : NV);
     ProfScope ps(L, "gmres_mdot", 8.0 * n * (nv + (mode == 0 ? 1 : 2)));
-    if (mode == 0)
-        k_mdot<NV, 0, FinH1><<<blocks, 256, 0, L.stream>>>(n, nv, V, ld, w, hprev, L.red(),
-                                                                FinH1{a, j}, gate);
-    else if (mode == 1)
-        k_mdot<NV, 1, FinH2><<<blocks, 256, 0, L.stream>>>(n, nv, V, ld, w, hprev, L.red(),
-                                                                FinH2{a, j}, gate);
-    else
-        k_mdot<NV, 2, FinNorm><<<blocks, 256, 0, L.stream>>>(n, nv, V, ld, w, hprev, L.red(),
-                                                              FinNorm{s, a, j}, gate);
+    auto launch = [&](auto k0, auto k1, auto k2) {
+        if (mode == 0) k0<<<blocks, 256, 0, L.stream>>>(n, nv, V, ld, w, hprev, L.red(), FinH1{a, j}, gate);
+        else if (mode == 1) k1<<<blocks, 256, 0, L.stream>>>(n, nv, V, ld, w, hprev, L.red(), FinH2{a, j}, gate);
+        else k2<<<blocks, 256, 0, L.stream>>>(n, nv, V, ld, w, hprev, L.red(), FinNorm{s, a, j}, gate);
+    };
+    if constexpr (NV <= 8) {
+        if (mdot_few(n, nv)) {
+            launch(k_mdot_few<NV, 0, FinH1>, k_mdot_few<NV, 1, FinH2>, k_mdot_few<NV, 2, FinNorm>);
+            HAMLSS_LAUNCH_CHECK();
+            return;
+        }
+    }
+    launch(k_mdot<NV, 0, FinH1>, k_mdot<NV, 1, FinH2>, k_mdot<NV, 2, FinNorm>);
     HAMLSS_LAUNCH_CHECK();
 }
 

@@ -88,4 +88,9 @@ inline TriMode tri_mode(int n, int nlev, int nnz, int max_row) {
     return ring <= block ? TriMode::RING : TriMode::BLOCK;
 }
 
+// ------------------------------------------------------------- FGMRES multi-dots (fgmres.cu)
+// A thread an entry (k_mdot_few) where there are few vectors and enough entries that the loads
+// count: the figures stand at the kernel.
+inline bool mdot_few(int n, int nv) { return nv <= 4 ? n >= (1 << 17) : nv <= 8 && n >= (1 << 19); }
+
 }  // namespace hamlss

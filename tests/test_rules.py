@@ -97,3 +97,9 @@ def test_sweep_kernel_by_shape(evaluate):
     got = evaluate([f"tri_mode({n}, {lv}, {nz}, {mr})" for (n, lv, nz, mr), _ in cases])
     assert got == [want for _, want in cases]
     assert evaluate([f"tri_places({k})" for k in (0, 1, 2, 3, 4, 5, 8, 9, 16)]) == [2, 2, 2, 4, 4, 8, 8, 16, 16]
+
+
+def test_multi_dots_of_few_vectors(evaluate):
+    cases = [((131071, 1), 0), ((131072, 1), 1), ((131072, 4), 1), ((131072, 5), 0), ((524287, 8), 0),
+             ((524288, 8), 1), ((4000000, 9), 0), ((1000, 1), 0)]
+    assert evaluate([f"mdot_few({n}, {v})" for (n, v), _ in cases]) == [w for _, w in cases]
