@@ -2406,13 +2406,12 @@ void seq_rows(Ctx& ctx, bool fill, const int* rows, int nrows, int span, const i
 // on near-dense levels whatever their size), else up to kGatherRatio a product, as long as
 // they stay below kGatherMost.  (L2 delivers ~1.4e12 pairs a second; the classes handle ~1e11
 // products.)  false: not taken.
-constexpr long long kGatherDense = 16LL << 20;           // entries of B held dense
 constexpr unsigned long long kGatherPairs = 200ull * 1000 * 1000;
 constexpr unsigned long long kGatherMost = 1000ull * 1000 * 1000;
 constexpr unsigned long long kGatherRatio = 8;
 
 bool spgemm_gather(Ctx& ctx, const Csr<double>& A, const Csr<double>& B, DCsr& C) {
-    if (!A.n || !A.nnz || !B.m || (long long)B.n * B.m > kGatherDense) return false;
+    if (!A.n || !A.nnz || !B.m || (long long)B.n * B.m > ctx.gather_dense) return false;
     // (cheap bounds first: small rows belong to the sequential classes)
     if ((double)A.nnz / A.n < 48.0 && (double)A.nnz * B.m > (double)kGatherPairs) return false;
     cudaStream_t s = ctx.lane.stream;
@@ -2438,7 +2437,7 @@ bool spgemm_gather(Ctx& ctx, const Csr<double>& A, const Csr<double>& B, DCsr& C
     HAMLSS_CUDA(cudaMemcpyAsync(off.p, wspan.p, sizeof(int) * (size_t)A.n, cudaMemcpyDeviceToDevice, s));
     HAMLSS_CUDA(cudaMemsetAsync(off.p + A.n, 0, sizeof(int), s));
     const long long total = exclusive_scan(ctx, off.p, A.n + 1);     // a slot a window column
-    if (total > INT_MAX) return false;
+    if (total > INT_MAX || total > std::max(ctx.gather_dense, (long long)kGatherSlots)) return false;
     DBuf<int> wci(std::max(total, 1LL));
     DBuf<double> wv(std::max(total, 1LL));
     k_spgemm_gather<<<std::min(A.n, ctx.sm_count * 16), kGatherThreads, 0, s>>>(A.n, wlo.p, wspan.p, A.rp, A.ci, A.v,

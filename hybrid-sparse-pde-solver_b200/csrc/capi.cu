@@ -76,6 +76,7 @@ void fgmres_cost(long long n, long long nz, const SolveResult& r, long long* flo
 }  // namespace
 
 namespace hamlss {
+void ctx_gather_dense(hamlss_ctx* ctx, long long entries) { ctx->c.gather_dense = entries; }
 int set_last_error(int code, const std::string& msg) { return set_err(code, msg); }
 }  // namespace hamlss
 

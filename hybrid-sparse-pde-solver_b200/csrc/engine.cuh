@@ -104,8 +104,12 @@ struct Ctx {
     // matrices then allocate nothing large (fresh pool memory of GBs maps slowly)
     DBuf<int> gemm_ci;
     DBuf<double> gemm_v;
+    // entries of a right operand that an AMG setup may hold dense (spgemm_gather)
+    long long gather_dense = kGatherDense;
     std::mutex mu;
 };
+// The server's solve lanes hold less of it, so that a request stays within its estimate.
+void ctx_gather_dense(hamlss_ctx* ctx, long long entries);
 
 // Max co-resident blocks of a kernel (cached per kernel instantiation by the caller).
 template <typename K>

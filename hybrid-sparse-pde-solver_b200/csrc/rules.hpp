@@ -93,4 +93,41 @@ inline TriMode tri_mode(int n, int nlev, int nnz, int max_row) {
 // count: the figures stand at the kernel.
 inline bool mdot_few(int n, int nv) { return nv <= 4 ? n >= (1 << 17) : nv <= 8 && n >= (1 << 19); }
 
+// ----------------------------------------------------------- dense right operands (amg.cu)
+// Entries of a right operand that an AMG setup holds dense, and of the slots beside it, on a
+// context of its own and on a server's solve lane (8 and 12 bytes an entry).
+constexpr long long kGatherDense = 16LL << 20;
+constexpr long long kGatherDenseLane = 2LL << 20;
+constexpr int kGatherSlots = 2 << 20;
+
+// --------------------------------------------------------- the server's estimates (serve.cu)
+// Device footprint of one request while it is admitted on a solve lane (bytes, an upper
+// estimate): CSR (int32 row_ptr + int32 col_idx + FP64 values), its FP32 copy and the diagonal;
+// Krylov workspace (eight FP64 and eight FP32 vectors, the FGMRES basis V and Z of 2m+1
+// vectors); and the larger of
+//   ILU(0)  the factor, L and U in sweep order, FP64 and FP32 -- a ring triangle's rows have the
+//           places of its longest row (at most max_row entries), the others their own entries --,
+//           diagonals with reciprocals, level sets and vectors
+//   AMG     the hierarchy (operators of the coarse levels, P and R) bounded by twice the fine
+//           operator, the dense right operand and its slots, and the coarse elimination's copy
+// (max_row 5, m = 30: FGMRES + ILU(0) on 250^2 holds 50 MB.)
+inline long long footprint_of(long long n, long long nnz, int m, int max_row) {
+    const long long csr = 4 * (n + 1) + 12 * nnz;
+    const long long f32 = 4 * nnz + 8 * n;
+    const long long ws = 8 * 8 * n + 8 * 4 * n + (2LL * m + 1) * 8 * n + 64 * 1024;
+    const long long ring = 2LL * tri_places(std::min(max_row, kTriMaxRow)) * (8 + 4 + 4 + 4) * n;
+    const long long rows = 16 * nnz + 8 * n;
+    const long long ilu = 8 * nnz + std::max(ring, 0LL) + (max_row > 4 ? rows : 0) + 100 * n;
+    const long long amg = 2 * (csr + f32) + 4 * 8 * n + std::min(20 * kGatherDenseLane, 5 * n * n) +
+                          std::min(8LL << 20, 8 * n * n);
+    return csr + f32 + 8 * n + ws + std::max(ilu, amg) + (1 << 20);
+}
+
+// Footprint of a request solved in the batch lane: the block's share of the batch's CSR (FP64 +
+// FP32), the ILU(0) factor while it is made, its entries in level order, level sets, and the
+// per-system vectors (2m + 5 in FP32, four in FP64).
+inline long long footprint_small(long long n, long long nnz, int m) {
+    return 36 * nnz + (8LL * m + 160) * n + 4096;
+}
+
 }  // namespace hamlss

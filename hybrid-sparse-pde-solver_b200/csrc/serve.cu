@@ -46,6 +46,11 @@
 #include <vector>
 
 #include "common.cuh"
+#include "rules.hpp"
+
+namespace hamlss {
+void ctx_gather_dense(hamlss_ctx* ctx, long long entries);     // engine.cuh
+}
 
 namespace {
 
@@ -70,6 +75,7 @@ struct Request {
     const double* b = nullptr;
     double* x = nullptr;
     hamlss_params p{};
+    int32_t max_row = 0;        // entries of the longest row
     int64_t footprint = 0;
     bool small = false;         // goes to the batch lane first
     bool spd_like = false;      // symmetric with a positive diagonal
@@ -82,26 +88,6 @@ struct Request {
     hamlss_stats stats{};
     double t_submit = 0.0, t_done = 0.0;
 };
-
-// Device footprint of one request while it is admitted (bytes, an upper estimate):
-// CSR (int32 row_ptr + int32 col_idx + FP64 values), its FP32 copy and the diagonal;
-// Krylov workspace (eight FP64 and eight FP32 vectors, the FGMRES basis V and Z of
-// 2m+1 vectors); ILU(0) factors plus level-ordered L and U copies; an AMG hierarchy
-// (operators of the coarse levels, P and R) bounded by twice the fine operator.
-int64_t footprint_of(int64_t n, int64_t nnz, int m) {
-    const int64_t csr = 4 * (n + 1) + 12 * nnz;
-    const int64_t f32 = 4 * nnz + 8 * n;
-    const int64_t ws = 8 * 8 * n + 8 * 4 * n + (int64_t)(2 * m + 1) * 8 * n + 64 * 1024;
-    const int64_t ilu = 8 * nnz + 2 * (12 * nnz + 4 * n) + 16 * n;
-    const int64_t amg = 2 * (csr + f32) + 4 * 8 * n;
-    return csr + f32 + 8 * n + ws + std::max(ilu, amg) + (1 << 20);
-}
-
-// Footprint of a request solved in the batch lane: the block's share of the batch's
-// CSR (FP64 + FP32), factors, level sets and per-system vectors.
-int64_t footprint_small(int64_t n, int64_t nnz, int m) {
-    return 4 * (n + 1) + 12 * nnz + 4 * nnz + 8 * nnz + 16 * n + 8 * n * (2 * m + 12) + 4096;
-}
 
 // Symmetric values and a positive diagonal (columns sorted within each row).
 bool spd_like(int n, const int32_t* rp, const int32_t* ci, const double* v) {
@@ -212,7 +198,7 @@ struct hamlss_server {
         --running;
         if (requeue) {
             r->state = St::Queued;
-            r->footprint = footprint_of(r->n, r->nnz, r->p.restart_size);
+            r->footprint = hamlss::footprint_of(r->n, r->nnz, r->p.restart_size, r->max_row);
             big_q.push_front(r);     // escalations go first: they have waited already
         } else {
             r->state = St::Done;
@@ -443,6 +429,7 @@ int hamlss_server_create(const hamlss_server_config* config, hamlss_server** out
             delete s;
             return fail(rc, m);
         }
+        hamlss::ctx_gather_dense(h, hamlss::kGatherDenseLane);
         s->ctxs.push_back(h);
     }
     for (int i = 0; i < c.slots; ++i)
@@ -470,6 +457,8 @@ int hamlss_server_submit(hamlss_server* s, int32_t n, int32_t nnz, const int32_t
     r->x = x;
     if (params) r->p = *params;
     else hamlss_params_default(&r->p);
+    for (int i = 0; i < n; ++i) r->max_row = std::max(r->max_row, row_ptr[i + 1] - row_ptr[i]);
+    const int64_t big = hamlss::footprint_of(n, nnz, r->p.restart_size, r->max_row);
     r->small = s->cfg.batch_max_rows > 0 && n <= s->cfg.batch_max_rows;
     if (r->small) {
         for (int i = 0; i < n; ++i)
@@ -479,11 +468,10 @@ int hamlss_server_submit(hamlss_server* s, int32_t n, int32_t nnz, const int32_t
             if (col_idx[e] < 0 || col_idx[e] >= n)
                 return fail(HAMLSS_ERR_MALFORMED, "column index out of range");
         r->spd_like = spd_like(n, row_ptr, col_idx, values);
-        r->footprint = footprint_small(n, nnz, std::min(r->p.restart_size, kBatchMaxRestart));
+        r->footprint = hamlss::footprint_small(n, nnz, std::min(r->p.restart_size, kBatchMaxRestart));
     } else {
-        r->footprint = footprint_of(n, nnz, r->p.restart_size);
+        r->footprint = big;
     }
-    const int64_t big = footprint_of(n, nnz, r->p.restart_size);
     if (big > s->cfg.hbm_budget_bytes)
         return fail(HAMLSS_ERR_BUDGET, "request needs an estimated " + std::to_string(big) +
                                            " bytes, more than the server's HBM budget");

@@ -103,3 +103,26 @@ def test_multi_dots_of_few_vectors(evaluate):
     cases = [((131071, 1), 0), ((131072, 1), 1), ((131072, 4), 1), ((131072, 5), 0), ((524287, 8), 0),
              ((524288, 8), 1), ((4000000, 9), 0), ((1000, 1), 0)]
     assert evaluate([f"mdot_few({n}, {v})" for (n, v), _ in cases]) == [w for _, w in cases]
+
+
+def test_request_footprint(evaluate):
+    # device bytes that one request held at its peak on a solve lane (n, entries, restart, longest
+    # row, measured on a B200 with the ring sweeps), all below the estimate
+    held = [
+        ((62500, 311512, 30, 18), 67.8e6),      # a grid with one row of 14 lower entries, all rows in 16 places
+        ((60000, 1136184, 30, 19), 98.6e6),
+        ((60000, 1136184, 5, 19), 74.6e6),
+        ((64000, 1643032, 30, 27), 113.8e6),
+        ((62500, 311500, 30, 5), 50.3e6),
+        ((360000, 1797600, 30, 5), 289.5e6),
+    ]
+    got = evaluate([f"footprint_of({n}, {z}, {m}, {r})" for (n, z, m, r), _ in held])
+    assert all(g >= h for g, (_, h) in zip(got, held)), got
+    flat = 20 * (2 << 20) + (8 << 20)          # what an AMG setup may hold besides, whatever n is
+    assert all(g <= 2 * h + flat for g, (_, h) in zip(got, held)), got
+    # the batch lane's arrays, counted from their sizes (restart 1 to 32, five entries a row)
+    got = evaluate([f"footprint_small(1000, 4900, {m})" for m in (1, 32)])
+    for g, m in zip(got, (1, 32)):
+        entries = 4 + 8 + 4 + 8 + 8 + 4        # columns, FP64, FP32, factor, level order, transpose
+        rows = 4 * 4 + 4 * 8 + 4 * (2 * m + 5) + 16 + 4 + 8 + 4 + 8 + 9 * 4
+        assert g >= 4900 * entries + 1000 * rows
