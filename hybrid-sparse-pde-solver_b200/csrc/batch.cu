@@ -19,7 +19,7 @@ namespace {
 
 constexpr double kEps = 2.220446049250313e-16;
 constexpr int kGroup = 8;               // accumulators per multi-dot group
-constexpr int kMaxPhases = kBatchClasses;
+constexpr int kMaxPhases = kBatchGroups;
 
 struct Phase {
     int begin, end, width;              // systems order[begin, end), team width
@@ -164,6 +164,18 @@ __device__ __forceinline__ RowPair rows_ax32(int g0, int g1, bool two, int row0,
     return r;
 }
 
+// Systems of at most kBatchSmall rows: a warp each.  Their entries and vectors sit in L1 and a
+// lane has a few rows, so what counts is the instructions of a row and the barriers of a trip;
+// the pipelined and unrolled forms below, made for loads that wait, take more of both.  (2,000
+// systems of 25 rows, CG / FGMRES + ILU(0): 0.35 / 0.37 ms by 128 threads and the forms below, 0.11 /
+// 0.12 by a warp and those, 0.064 / 0.085 by a warp and these.)
+__device__ __forceinline__ float row_ax32(int g, int row0, const BArgs& a, const float* v) {
+    float s = 0.f;
+    for (int k = __ldg(&a.rp[g]); k < __ldg(&a.rp[g + 1]); ++k)
+        s = __fmaf_rn(__ldg(&a.v32[k]), v[__ldg(&a.ci[k]) - row0], s);
+    return s;
+}
+
 // ---------------------------------------------------------------- inner PCG (FP32)
 struct CgZ {
     const float* R;
@@ -172,6 +184,75 @@ struct CgZ {
         return dinv ? __fmul_rn(__ldg(&dinv[i]), R[i]) : R[i];
     }
 };
+
+// q = A p formed with p = z + beta p_old on the fly (p_old and p in turn in two vectors), the
+// same values as inner_cg's.
+__device__ int inner_cg_small(const Team& T, const BArgs& a, const BProb& P, float* w, double itol, int maxit) {
+    const int n = P.n, r0 = P.row0;
+    float* R = w;
+    float* pold = w + n;
+    float* pnew = w + 2 * (size_t)n;
+    float* Q = w + 3 * (size_t)n;
+    float* D = w + 4 * (size_t)n;
+    const CgZ z{R, P.method == BM_CG_JAC ? a.dinv + r0 : nullptr};
+    double rz = 0.0, rr = 0.0;
+    for (int i = T.lt; i < n; i += T.W) {
+        const float r = R[i];
+        rz += (double)r * (double)z(i);
+        rr += (double)r * (double)r;
+        pold[i] = 0.f;
+    }
+    T.put(rz, 0);
+    T.put(rr, 1);
+    T.finish(2);
+    double rho = T.res[0];
+    const double rn0 = sqrt(T.res[1]);
+    if (!(rn0 > 0.0)) return 0;
+    float beta = 0.f;
+    int it = 0;
+    while (it < maxit) {
+        double pq = 0.0;
+        for (int i = T.lt; i < n; i += T.W) {
+            const int g = r0 + i;
+            float s = 0.f;
+            for (int k = __ldg(&a.rp[g]); k < __ldg(&a.rp[g + 1]); ++k) {
+                const int j = __ldg(&a.ci[k]) - r0;
+                s = __fmaf_rn(__ldg(&a.v32[k]), __fmaf_rn(beta, pold[j], z(j)), s);
+            }
+            const float pi = __fmaf_rn(beta, pold[i], z(i));
+            pnew[i] = pi;
+            Q[i] = s;
+            pq += (double)pi * (double)s;
+        }
+        T.put(pq, 0);
+        T.finish(1);
+        pq = T.res[0];
+        if (!(fabs(pq) > kEps * 1e6 * fabs(rho))) break;        // breakdown or NaN
+        const float af = (float)(rho / pq);
+        rr = 0.0;
+        rz = 0.0;
+        for (int i = T.lt; i < n; i += T.W) {
+            D[i] = __fmaf_rn(af, pnew[i], D[i]);
+            const float r = __fmaf_rn(-af, Q[i], R[i]);
+            R[i] = r;
+            rr += (double)r * (double)r;
+            rz += (double)r * (double)z(i);
+        }
+        T.put(rr, 0);
+        T.put(rz, 1);
+        T.finish(2);
+        ++it;
+        const double rel = sqrt(T.res[0]) / rn0;
+        if (!(rel >= itol)) break;                               // converged or NaN
+        if (!(fabs(rho) > 0.0)) break;
+        beta = (float)(T.res[1] / rho);
+        rho = T.res[1];
+        float* t = pold;
+        pold = pnew;
+        pnew = t;
+    }
+    return it;
+}
 
 __device__ int inner_cg(const Team& T, const BArgs& a, const BProb& P, float* w, double itol,
                         int maxit) {
@@ -343,10 +424,38 @@ __device__ __forceinline__ void bsweep(const Team& T, const int* __restrict__ lp
     }
 }
 
+// The same from the right-hand side b, each level's rows loaded in the level (x in global
+// memory: L1).
+template <bool DIV>
+__device__ __forceinline__ void bsweep_small(const Team& T, const int* __restrict__ lptr, int nlev,
+                                             const int2* __restrict__ info, const int2* __restrict__ ent,
+                                             const float* __restrict__ dg, const float* b, float* x) {
+    for (int l = 0; l < nlev; ++l) {
+        const int e = __ldg(&lptr[l + 1]);
+        for (int t = __ldg(&lptr[l]) + T.lt; t < e; t += T.W) {
+            const int2 in = __ldg(&info[t]);
+            const int end = __ldg(&info[t + 1].y);
+            float s = b[in.x];
+            for (int k = in.y; k < end; ++k) {
+                const int2 en = __ldg(&ent[k]);
+                s = __fmaf_rn(-__int_as_float(en.y), x[en.x], s);
+            }
+            x[in.x] = DIV ? __fdiv_rn(s, __ldg(&dg[t])) : s;
+        }
+        T.sync();
+    }
+}
+
 // z = M^-1 v for the FGMRES systems (Y: work vector, used where the team has no shared one);
 // ends with a team barrier.  Returns where the products A z should gather z from.
+template <bool SMALL>
 __device__ const float* bprec(const Team& T, const BArgs& a, const BProb& P, const float* v, float* z, float* Y) {
     const int n = P.n, r0 = P.row0;
+    if (SMALL && P.method == BM_GM_ILU) {
+        bsweep_small<false>(T, a.lptrL + P.levL, P.nlevL, a.infoL, a.entL, nullptr, v, z);
+        bsweep_small<true>(T, a.lptrU + P.levU, P.nlevU, a.infoU, a.entU, a.dgU, z, z);
+        return z;
+    }
     if (P.method == BM_GM_ILU) {
         float* x = T.vec ? T.vec : Y;
         for (int i = T.lt; i < n; i += T.W) x[i] = v[i];
@@ -383,6 +492,7 @@ __device__ void multi_dot(const Team& T, const float* V, size_t n, int nv, const
 }
 
 // ------------------------------------------------------------- inner FGMRES (FP32)
+template <bool SMALL>
 __device__ int inner_gmres(const Team& T, const BArgs& a, const BProb& P, float* w, double itol,
                            int maxit) {
     const int n = P.n, r0 = P.row0, m = a.m;
@@ -400,7 +510,7 @@ __device__ int inner_gmres(const Team& T, const BArgs& a, const BProb& P, float*
         double bb = 0.0;
         for (int i = T.lt; i < n; i += T.W) {
             float s = R[i];
-            if (beta0 >= 0.0) s -= rows_ax32(r0 + i, 0, false, r0, a, D).s0;
+            if (beta0 >= 0.0) s -= SMALL ? row_ax32(r0 + i, r0, a, D) : rows_ax32(r0 + i, 0, false, r0, a, D).s0;
             V[i] = s;
             bb += (double)s * (double)s;
         }
@@ -421,9 +531,11 @@ __device__ int inner_gmres(const Team& T, const BArgs& a, const BProb& P, float*
         for (int j = 0; j < m && it < maxit; ++j) {
             const float* Vj = V + (size_t)j * nn;
             float* Zj = Z + (size_t)j * nn;
-            const float* zj = bprec(T, a, P, Vj, Zj, Y);
+            const float* zj = bprec<SMALL>(T, a, P, Vj, Zj, Y);
             // w = A z_j ; h = V^T w
-            for (int i = T.lt; i < n; i += 2 * T.W) {
+            if constexpr (SMALL)
+                for (int i = T.lt; i < n; i += T.W) Wv[i] = row_ax32(r0 + i, r0, a, zj);
+            else for (int i = T.lt; i < n; i += 2 * T.W) {
                 const RowPair s = rows_ax32(r0 + i, r0 + i + T.W, i + T.W < n, r0, a, zj);
                 Wv[i] = s.s0;
                 if (i + T.W < n) Wv[i + T.W] = s.s1;
@@ -508,6 +620,7 @@ __device__ int inner_gmres(const Team& T, const BArgs& a, const BProb& P, float*
 }
 
 // ------------------------------------------------------ one system: FP64 refinement
+template <bool SMALL>
 __device__ void solve_one(const Team& T, const BArgs& a, int k) {
     const BProb P = a.prob[k];
     const int n = P.n, r0 = P.row0;
@@ -545,8 +658,9 @@ __device__ void solve_one(const Team& T, const BArgs& a, int k) {
         }
         T.sync();
         const double itol = fmax(a.inner_tol, 0.5 * a.tol / rel);
-        const int its = cg ? inner_cg(T, a, P, w, itol, a.max_iter - total)
-                           : inner_gmres(T, a, P, w, itol, a.max_iter - total);
+        const int left = a.max_iter - total;
+        const int its = !cg ? inner_gmres<SMALL>(T, a, P, w, itol, left)
+                        : SMALL ? inner_cg_small(T, a, P, w, itol, left) : inner_cg(T, a, P, w, itol, left);
         total += its;
         for (int i = T.lt; i < n; i += T.W) a.x[r0 + i] += rn * (double)D[i];
         T.sync();
@@ -566,6 +680,7 @@ __device__ void solve_one(const Team& T, const BArgs& a, int k) {
     T.sync();
 }
 
+template <bool SMALL>
 __global__ void __launch_bounds__(kBatchThreads, 1) k_batch_solve(BArgs a) {
     extern __shared__ double smem[];
     for (int p = 0; p < a.nphase; ++p) {
@@ -578,7 +693,7 @@ __global__ void __launch_bounds__(kBatchThreads, 1) k_batch_solve(BArgs a) {
             const int q = *T.slot;
             T.sync();
             if (q >= cnt) break;
-            solve_one(T, a, a.order[a.ph[p].begin + q]);
+            solve_one<SMALL>(T, a, a.order[a.ph[p].begin + q]);
         }
         __syncthreads();
     }
@@ -696,6 +811,8 @@ __global__ void k_batch_pack(int rows, const int* __restrict__ ord, const int* _
         if (!FILL) first[t] = o;
     }
 }
+
+int batch_group(const BProb& P) { return hamlss::batch_group(P.n, P.method == BM_CG_JAC || P.method == BM_CG_NONE); }
 
 int klass_of(int n) {
     if (n <= 1024) return 0;
@@ -895,12 +1012,12 @@ std::unique_ptr<Batch> batch_create(Ctx& ctx, hamlss_ctx* h, int count, const in
     std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) {
         const BProb& a = B->hprob[x];
         const BProb& b = B->hprob[y];
-        if (a.klass != b.klass) return a.klass > b.klass;
+        if (batch_group(a) != batch_group(b)) return batch_group(a) > batch_group(b);
         return a.n > b.n;
     });
     B->order.ensure(count);
     B->order.upload(ord.data(), count, s);
-    B->tickets.ensure(kMaxPhases);
+    B->tickets.ensure(2 * kMaxPhases);
     B->r64.ensure(N);
     B->xb.ensure(N);
     B->bb.ensure(N);
@@ -913,25 +1030,31 @@ std::unique_ptr<Batch> batch_create(Ctx& ctx, hamlss_ctx* h, int count, const in
 
 double batch_run(Ctx& ctx, Batch& B, const double* b, double* x, unsigned class_mask) {
     cudaStream_t s = ctx.lane.stream;
-    BArgs a{};
-    // phases in schedule order (classes descending), each a contiguous run of `order`
+    BArgs a{}, small{};
+    // phases in schedule order (groups descending), each a contiguous run of `order`; the
+    // systems of group 0 go to a launch of their own
     int pos = 0;
-    a.nphase = 0;
-    std::vector<int> per(kBatchClasses, 0);
-    for (const auto& P : B.hprob) per[P.klass]++;
+    a.nphase = small.nphase = 0;
+    std::vector<int> per(kBatchGroups, 0);
+    for (const auto& P : B.hprob) per[batch_group(P)]++;
     size_t team_bytes = 0, vec_bytes = 0;
-    for (int c = kBatchClasses - 1; c >= 0; --c) {
-        if (!per[c]) continue;
+    for (int g = kBatchGroups - 1; g >= 0; --g) {
+        if (!per[g]) continue;
+        const int c = batch_group_class(g), W = batch_group_width(g, B.width[c]);
         if (class_mask & (1u << c)) {
-            const int teams = kBatchThreads / B.width[c];
-            const int vec = sizeof(float) * (size_t)teams * kBatchVec[c] <= kBatchVecBytes ? kBatchVec[c] : 0;
-            a.ph[a.nphase++] = Phase{pos, pos + per[c], B.width[c], vec};
-            team_bytes = std::max(team_bytes, batch_team_smem(B.width[c], B.m));
-            vec_bytes = std::max(vec_bytes, sizeof(float) * (size_t)teams * vec);
+            if (g == 0) {
+                small.ph[small.nphase++] = Phase{pos, pos + per[g], W, 0};
+            } else {
+                const int teams = kBatchThreads / W;
+                const int vec = sizeof(float) * (size_t)teams * kBatchVec[c] <= kBatchVecBytes ? kBatchVec[c] : 0;
+                a.ph[a.nphase++] = Phase{pos, pos + per[g], W, vec};
+                team_bytes = std::max(team_bytes, batch_team_smem(W, B.m));
+                vec_bytes = std::max(vec_bytes, sizeof(float) * (size_t)teams * vec);
+            }
         }
-        pos += per[c];
+        pos += per[g];
     }
-    if (a.nphase == 0) return 0.0;
+    if (a.nphase + small.nphase == 0) return 0.0;
     a.order = B.order.p;
     a.tickets = B.tickets.p;
     a.prob = B.prob.p;
@@ -958,23 +1081,36 @@ double batch_run(Ctx& ctx, Batch& B, const double* b, double* x, unsigned class_
     a.max_iter = B.params.max_iter;
     a.max_outer = B.params.ir_max_outer;
     a.m = B.m;
-    a.vec_at = (int)team_bytes;
-    const size_t smem = team_bytes + vec_bytes;
     static DeviceOnce raised;            // the device's opt-in maximum, so no call lowers it
     raised(ctx.device, [&] {
         int optin = 0;
         HAMLSS_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx.device));
-        HAMLSS_CUDA(cudaFuncSetAttribute(k_batch_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+        for (auto f : {k_batch_solve<false>, k_batch_solve<true>})
+            HAMLSS_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     });
-    int per_sm = occupancy_blocks(k_batch_solve, kBatchThreads, smem);
-    const int blocks = std::max(1, per_sm * ctx.sm_count);
-    HAMLSS_CUDA(cudaMemsetAsync(B.tickets.p, 0, sizeof(int) * kMaxPhases, s));
+    HAMLSS_CUDA(cudaMemsetAsync(B.tickets.p, 0, sizeof(int) * 2 * kMaxPhases, s));
     // algorithmic bytes of one launch are not a fixed figure (iteration counts differ per
     // system); the profiler records the launch with 0 bytes
     ProfScope ps(ctx.lane, "batch_solve", 0.0);
     HAMLSS_CUDA(cudaEventRecord(B.e0, s));
-    k_batch_solve<<<blocks, kBatchThreads, smem, s>>>(a);
-    HAMLSS_LAUNCH_CHECK();
+    auto launch = [&](auto kern, BArgs& k, size_t teams, size_t vecs, int most) {
+        k.vec_at = (int)teams;
+        const size_t smem = teams + vecs;
+        const int blocks = std::max(1, std::min(most, occupancy_blocks(kern, kBatchThreads, smem) * ctx.sm_count));
+        kern<<<blocks, kBatchThreads, smem, s>>>(k);
+        HAMLSS_LAUNCH_CHECK();
+    };
+    if (a.nphase) launch(k_batch_solve<false>, a, team_bytes, vec_bytes, INT_MAX);
+    if (small.nphase) {
+        const Phase ph = small.ph[0];
+        const int nphase = small.nphase;
+        small = a;
+        small.nphase = nphase;
+        small.ph[0] = ph;
+        small.tickets = B.tickets.p + kMaxPhases;
+        launch(k_batch_solve<true>, small, batch_team_smem(ph.width, B.m), 0,
+               ceil_div(ph.end - ph.begin, kBatchThreads / ph.width));
+    }
     HAMLSS_CUDA(cudaEventRecord(B.e1, s));
     HAMLSS_CUDA(cudaEventSynchronize(B.e1));
     float ms = 0.f;

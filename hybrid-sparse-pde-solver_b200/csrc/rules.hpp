@@ -130,4 +130,25 @@ inline long long footprint_small(long long n, long long nnz, int m) {
     return 36 * nnz + (8LL * m + 160) * n + 4096;
 }
 
+// ------------------------------------------------------------------ batched solves (batch.cu)
+constexpr int kBatchSmall = 100;              // rows a warp solves by itself
+constexpr int kBatchGroups = 6;
+// Scheduling group of a system: the size classes (n <= 1,024, 4,096, 16,384, larger) are groups 2
+// to 5; of the first class, systems of at most kBatchSmall rows are group 0 and the next ones, up
+// to 200 rows (CG) or 640 (FGMRES), group 1, with narrower teams.  A width depends on the system
+// alone, never on the batch, so that a system's result does not either.  Device time, ms, at 32 /
+// 64 / 128 threads: CG, 121 rows, 40 systems 0.42 / 0.23 / 0.20, 2,000 0.48 / 0.47 / 0.77; 256 rows
+// 0.88 / 0.49 / 0.32, 1.01 / 0.99 / 1.22; FGMRES + ILU(0), 256 rows 0.37 / 0.30 / 0.26, 0.47 / 0.59 /
+// 0.95; 400 rows 0.52 / 0.39 / 0.34, 0.81 / 0.87 / 1.29; 1,024 rows 1.2 / 0.73 / 0.58, 1.9 / 2.0 / 2.4.
+inline int batch_group(int n, bool cg) {
+    if (n <= kBatchSmall) return 0;
+    if (n <= (cg ? 200 : 640)) return 1;
+    return n <= 1024 ? 2 : n <= 4096 ? 3 : n <= 16384 ? 4 : 5;
+}
+inline int batch_group_class(int group) { return std::max(0, group - 2); }
+// (`width`: of the group's size class)
+inline int batch_group_width(int group, int width) {
+    return group == 0 ? 32 : group == 1 ? std::min(width, 64) : width;
+}
+
 }  // namespace hamlss

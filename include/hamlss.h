@@ -313,8 +313,9 @@ int hamlss_batch_create(hamlss_ctx* ctx, int32_t count, const int32_t* row_off,
 int hamlss_batch_solve(hamlss_ctx* ctx, hamlss_batch* B, const double* b, double* x, int where,
                        hamlss_batch_result* results, hamlss_stats* total);
 /* Team width (threads per system: 32, 64, 128, 256 or 512) of the four size classes
- * n <= 1024, <= 4096, <= 16384 and larger.  Results depend on the width only through the
- * order of the dot-product sums. */
+ * n <= 1024, <= 4096, <= 16384 and larger.  (Systems of at most 100 rows take 32 threads, CG
+ * systems up to 200 and FGMRES systems up to 640 at most 64, whatever the first class has.)
+ * Results depend on the width only through the order of the dot-product sums. */
 int hamlss_batch_set_widths(hamlss_batch* B, const int32_t widths[4]);
 int hamlss_batch_get_widths(const hamlss_batch* B, int32_t widths[4]);
 /* Time every width for every size class present (solves of the batch itself, x0 = 0, on

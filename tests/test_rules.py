@@ -126,3 +126,13 @@ def test_request_footprint(evaluate):
         entries = 4 + 8 + 4 + 8 + 8 + 4        # columns, FP64, FP32, factor, level order, transpose
         rows = 4 * 4 + 4 * 8 + 4 * (2 * m + 5) + 16 + 4 + 8 + 4 + 8 + 9 * 4
         assert g >= 4900 * entries + 1000 * rows
+
+
+def test_batch_groups(evaluate):
+    sizes = [1, 100, 101, 200, 201, 640, 641, 1024, 1025, 4096, 4097, 16384, 16385]
+    cg, gm = [0, 0, 1, 1, 2, 2, 2, 2, 3, 3, 4, 4, 5], [0, 0, 1, 1, 1, 1, 2, 2, 3, 3, 4, 4, 5]
+    assert evaluate([f"batch_group({n}, true)" for n in sizes]) == cg
+    assert evaluate([f"batch_group({n}, false)" for n in sizes]) == gm
+    assert evaluate([f"batch_group_class({g})" for g in range(6)]) == [0, 0, 0, 1, 2, 3]
+    assert evaluate([f"batch_group_width({g}, {w})" for w in (32, 128, 512) for g in (0, 1, 2, 5)]) == \
+        [32, 32, 32, 32, 32, 64, 128, 128, 32, 64, 512, 512]
