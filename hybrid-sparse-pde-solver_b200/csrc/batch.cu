@@ -965,8 +965,10 @@ std::unique_ptr<Batch> batch_create(Ctx& ctx, hamlss_ctx* h, int count, const in
         k_level_bucket<false><<<g, 256, 0, s>>>(N, prow.p, B->prob.p, lvL.p, lvU.p, B->lptrL.p, B->lptrU.p,
                                                 nullptr, nullptr);
         HAMLSS_LAUNCH_CHECK();
-        long long rowsL = exclusive_scan(ctx, B->lptrL.p, (int)tl + 1);
-        exclusive_scan(ctx, B->lptrU.p, (int)tu + 1);
+        scan_in_place(ctx, B->lptrL.p, (int)tl + 1);
+        scan_in_place(ctx, B->lptrU.p, (int)tu + 1);
+        long long rowsL = 0;
+        for (int k : sys) rowsL += B->hprob[k].n;
         DBuf<int> lordL(std::max<long long>(rowsL, 1)), lordU(std::max<long long>(rowsL, 1));
         DBuf<int> fL(tl + 1), fU(tu + 1);
         HAMLSS_CUDA(cudaMemcpyAsync(fL.p, B->lptrL.p, sizeof(int) * (tl + 1), cudaMemcpyDeviceToDevice, s));
@@ -987,22 +989,27 @@ std::unique_ptr<Batch> batch_create(Ctx& ctx, hamlss_ctx* h, int count, const in
         HAMLSS_LAUNCH_CHECK();
         // the factors in level order
         const int rows = (int)rowsL;
-        DBuf<int> first(rows + 1);
+        DBuf<int> firstL(rows + 1), firstU(rows + 1);
+        DBuf<long long> totals(2);
         B->infoL.ensure(rows + 1);
         B->infoU.ensure(rows + 1);
         B->dgU.ensure(std::max(rows, 1));
         k_batch_pack<true, false><<<g, 256, 0, s>>>(rows, lordL.p, prow.p, B->prob.p, B->rp.p, B->ci.p, lu64.p,
-                                                    first.p, nullptr, nullptr, nullptr);
-        HAMLSS_LAUNCH_CHECK();
-        B->entL.ensure(std::max(exclusive_scan(ctx, first.p, rows + 1), 1LL));
-        k_batch_pack<true, true><<<g, 256, 0, s>>>(rows, lordL.p, prow.p, B->prob.p, B->rp.p, B->ci.p, lu64.p,
-                                                   first.p, B->infoL.p, B->entL.p, nullptr);
+                                                    firstL.p, nullptr, nullptr, nullptr);
         k_batch_pack<false, false><<<g, 256, 0, s>>>(rows, lordU.p, prow.p, B->prob.p, B->rp.p, B->ci.p, lu64.p,
-                                                     first.p, nullptr, nullptr, nullptr);
+                                                     firstU.p, nullptr, nullptr, nullptr);
         HAMLSS_LAUNCH_CHECK();
-        B->entU.ensure(std::max(exclusive_scan(ctx, first.p, rows + 1), 1LL));
+        scan_in_place(ctx, firstL.p, rows + 1, totals.p);
+        scan_in_place(ctx, firstU.p, rows + 1, totals.p + 1);
+        long long ht[2];
+        totals.download(ht, 2, s);
+        HAMLSS_CUDA(cudaStreamSynchronize(s));
+        B->entL.ensure(std::max(ht[0], 1LL));
+        B->entU.ensure(std::max(ht[1], 1LL));
+        k_batch_pack<true, true><<<g, 256, 0, s>>>(rows, lordL.p, prow.p, B->prob.p, B->rp.p, B->ci.p, lu64.p,
+                                                   firstL.p, B->infoL.p, B->entL.p, nullptr);
         k_batch_pack<false, true><<<g, 256, 0, s>>>(rows, lordU.p, prow.p, B->prob.p, B->rp.p, B->ci.p, lu64.p,
-                                                    first.p, B->infoU.p, B->entU.p, B->dgU.p);
+                                                    firstU.p, B->infoU.p, B->entU.p, B->dgU.p);
         HAMLSS_LAUNCH_CHECK();
         HAMLSS_CUDA(cudaStreamSynchronize(s));
     }

@@ -267,13 +267,26 @@ k_levels_chain(int n, const int* __restrict__ rp, const int* __restrict__ ci, in
     if (tid == 0) nlev[blockIdx.x] = s_max + 1;
 }
 
+// (rows of one level in a warp add once: red-black and other coloured orderings have a few
+// levels of millions of rows, whose counters every thread would queue at)
 __global__ void k_level_hist(int n, const int* __restrict__ level, int* cnt) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) atomicAdd(&cnt[level[i]], 1);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int l = level[i];
+        const unsigned same = __match_any_sync(__activemask(), l);
+        if ((int)(threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&cnt[l], __popc(same));
+    }
 }
 
 __global__ void k_level_place(int n, const int* __restrict__ level, int* fill, int* order) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        order[atomicAdd(&fill[level[i]], 1)] = i;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int l = level[i], lane = threadIdx.x & 31;
+        const unsigned act = __activemask(), same = __match_any_sync(act, l);
+        const int first = __ffs(same) - 1;
+        int at = 0;
+        if (lane == first) at = atomicAdd(&fill[l], __popc(same));
+        at = __shfl_sync(act, at, first);
+        order[at + __popc(same & ((1u << lane) - 1u))] = i;
+    }
 }
 
 // Rows of each level by index (a level of at most kSortRows rows; wider ones keep the order
@@ -550,13 +563,13 @@ __global__ void k_fill_U(int n, const int* __restrict__ order, const int* __rest
 // A triangle in position order with the matrix's own columns and vectors in row order.
 template <typename T>
 struct TriRows {
-    int n, nlev;
-    const int* ord;
-    const int* lptr;
-    const int* rp;
-    const int* ci;
-    const T* v;
-    const T* dg;
+    int n = 0, nlev = 0;
+    const int* ord = nullptr;
+    const int* lptr = nullptr;
+    const int* rp = nullptr;
+    const int* ci = nullptr;
+    const T* v = nullptr;
+    const T* dg = nullptr;
 };
 
 // One sweep by one block for triangles with long rows (ilu_sweep.cuh's rings hold steps of
@@ -662,22 +675,30 @@ k_tri_block(TriRows<T> F, const T* rhs, T* out, const int* gate) {
     }
 }
 
-// The same sweep with the whole grid (cooperative launch) for triangles with wide levels.
+// The same sweep with the whole grid (cooperative launch) for triangles with wide levels: the
+// lower triangle's, the upper one's (nlev = 0: not this one), or one after the other.
 template <typename T, bool DIV>
-__global__ void k_tri_grid(TriRows<T> F, const T* __restrict__ rhs, T* out, const int* gate) {
-    if (gate && *(volatile const int*)gate) return;
+__device__ __forceinline__ void grid_sweep(const TriRows<T>& F, const T* rhs, T* out) {
     cg::grid_group grid = cg::this_grid();
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
     for (int l = 0; l < F.nlev; ++l) {
         const int b = F.lptr[l], e = F.lptr[l + 1];
         for (int t = b + tid; t < e; t += nth) {
             const int i = F.ord[t];
-            T s = rhs[i];
+            T s = __ldcg(&rhs[i]);
             for (int o = F.rp[t]; o < F.rp[t + 1]; ++o) s = sub_mul<T>(s, F.v[o], __ldcg(&out[F.ci[o]]));
             out[i] = DIV ? s / F.dg[t] : s;
         }
         if (l + 1 < F.nlev) grid.sync();
     }
+}
+
+template <typename T>
+__global__ void k_tri_grid(TriRows<T> L, TriRows<T> U, const T* rhs, T* y, T* z, const int* gate) {
+    if (gate && *(volatile const int*)gate) return;
+    grid_sweep<T, false>(L, rhs, y);
+    if (L.nlev && U.nlev) cg::this_grid().sync();
+    grid_sweep<T, true>(U, y, z);
 }
 
 // ------------------------------------------------------------------------- ILUT
@@ -1210,14 +1231,26 @@ struct IluPrec : Prec {
             HAMLSS_LAUNCH_CHECK();
             return;
         }
-        TriRows<T> F{n, t.nlev, t.ord.p, t.lptr.p, t.rp.p, t.ci.p, tv.p, tdg.p};
+        const TriRows<T> F = rows_of<T>(t);
         if (t.mode == TriMode::BLOCK) {
             k_tri_block<T, DIV, 1024><<<1, 1024, 0, ln.stream>>>(F, rhs, out, gate);
             HAMLSS_LAUNCH_CHECK();
+        } else if (DIV) {
+            grid_launch<T>(ctx, ln, TriRows<T>{}, F, nullptr, const_cast<T*>(rhs), out, gate);
         } else {
-            static const int blocks = coop_blocks(ctx, k_tri_grid<T, DIV>, 256);
-            coop_launch(ln.stream, k_tri_grid<T, DIV>, blocks, 256, F, rhs, out, gate);
+            grid_launch<T>(ctx, ln, F, TriRows<T>{}, rhs, out, nullptr, gate);
         }
+    }
+
+    template <typename T>
+    TriRows<T> rows_of(Triangle& t) const {
+        auto [tv, tdg, tcode] = tri_bufs(t, T(0));
+        return TriRows<T>{n, t.nlev, t.ord.p, t.lptr.p, t.rp.p, t.ci.p, tv.p, tdg.p};
+    }
+    template <typename T>
+    void grid_launch(Ctx& ctx, const Lane& ln, TriRows<T> FL, TriRows<T> FU, const T* rhs, T* y, T* z, const int* gate) {
+        static const int blocks = coop_blocks(ctx, k_tri_grid<T>, 256);
+        coop_launch(ln.stream, k_tri_grid<T>, blocks, 256, FL, FU, rhs, y, z, gate);
     }
 
     template <typename T>
@@ -1226,6 +1259,8 @@ struct IluPrec : Prec {
         if (!n) return;
         ProfScope ps(ln, "ilu_sweep", (double)sizeof(T) * (L.nnz + U.nnz + 4.0 * n) + 4.0 * (L.nnz + U.nnz + 4.0 * n));
         const bool lring = L.mode == TriMode::RING, uring = U.mode == TriMode::RING;
+        if (L.mode == TriMode::GRID && U.mode == TriMode::GRID)
+            return grid_launch<T>(ctx, ln, rows_of<T>(L), rows_of<T>(U), r, yb, z, gate);
         if (lring) {
             permute<T, true>(ctx, ln, L.ord.p, r, a, gate);
             sweep<T, false>(ctx, ln, L, a, c, gate);
@@ -1473,7 +1508,7 @@ void finish_ilu(Ctx& ctx, IluPrec* P, bool factorise) {
         HAMLSS_CUDA(cudaMemsetAsync(t.lptr.p, 0, sizeof(int) * (t.nlev + 1), s));
         k_level_hist<<<g, 256, 0, s>>>(n, t.level.p, t.lptr.p);
         HAMLSS_LAUNCH_CHECK();
-        exclusive_scan(ctx, t.lptr.p, t.nlev + 1);
+        scan_in_place(ctx, t.lptr.p, t.nlev + 1);
         DBuf<int> fill(t.nlev + 1);
         HAMLSS_CUDA(cudaMemcpyAsync(fill.p, t.lptr.p, sizeof(int) * (t.nlev + 1), cudaMemcpyDeviceToDevice, s));
         t.ord.ensure(n);
@@ -1484,11 +1519,13 @@ void finish_ilu(Ctx& ctx, IluPrec* P, bool factorise) {
         HAMLSS_LAUNCH_CHECK();
         t.mode = tri_mode(n, t.nlev, hf[5 + k], t.max_row);
     }
-    int hw[2];
-    HAMLSS_CUDA(cudaMemcpyAsync(hw, facts.p + 7, sizeof(hw), cudaMemcpyDeviceToHost, s));
-    HAMLSS_CUDA(cudaStreamSynchronize(s));
-    P->L.max_width = hw[0];
-    P->U.max_width = hw[1];
+    if (P->L.mode == TriMode::RING || P->U.mode == TriMode::RING) {
+        int hw[2];
+        HAMLSS_CUDA(cudaMemcpyAsync(hw, facts.p + 7, sizeof(hw), cudaMemcpyDeviceToHost, s));
+        HAMLSS_CUDA(cudaStreamSynchronize(s));
+        P->L.max_width = hw[0];
+        P->U.max_width = hw[1];
+    }
     if (P->L.mode == TriMode::RING) P->make_steps<false>(ctx, P->L);
     if (P->U.mode == TriMode::RING) P->make_steps<true>(ctx, P->U);
     // factorisation (ILU(0); ILUT arrives factored)
@@ -1544,7 +1581,7 @@ void finish_ilu(Ctx& ctx, IluPrec* P, bool factorise) {
         HAMLSS_CUDA(cudaMemsetAsync(t.rp.p + n, 0, sizeof(int), s));
         k_perm_counts<<<g, 256, 0, s>>>(n, t.ord.p, k == 0 ? lcnt.p : ucnt.p, t.rp.p);
         HAMLSS_LAUNCH_CHECK();
-        exclusive_scan(ctx, t.rp.p, n + 1);
+        scan_in_place(ctx, t.rp.p, n + 1);
         t.ci.ensure(std::max(t.nnz, 1));
         t.v.ensure(std::max(t.nnz, 1));
         if (k == 0) {
@@ -1589,7 +1626,7 @@ void pattern_levels(Ctx& ctx, int n, int nnz, const int* rp, const int* ci, DBuf
     HAMLSS_CUDA(cudaMemsetAsync(trp.p, 0, sizeof(int) * (n + 1), s));
     k_col_count<<<g, 256, 0, s>>>(n, rp, ci, trp.p);
     HAMLSS_LAUNCH_CHECK();
-    exclusive_scan(ctx, trp.p, n + 1);
+    scan_in_place(ctx, trp.p, n + 1);
     HAMLSS_CUDA(cudaMemcpyAsync(fill.p, trp.p, sizeof(int) * n, cudaMemcpyDeviceToDevice, s));
     k_col_fill<<<g, 256, 0, s>>>(n, rp, ci, fill.p, trow.p);
     HAMLSS_LAUNCH_CHECK();

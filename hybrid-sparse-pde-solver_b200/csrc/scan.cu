@@ -63,14 +63,18 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_sums(int* sums, int nb, lon
     if (threadIdx.x == 0) *total = carry;
 }
 
-__global__ void __launch_bounds__(kScanBlock) k_tile_apply(int* a, int count, const int* __restrict__ sums) {
+// sums: the tiles' offsets; null: one tile, whose total goes to *total (if given)
+__global__ void __launch_bounds__(kScanBlock)
+k_tile_apply(int* a, int count, const int* __restrict__ sums, long long* total) {
     __shared__ int sh[32];
     const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
     int v[kScanItems];
     int s = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) { v[k] = (base + k < count) ? a[base + k] : 0; s += v[k]; }
-    int ex = block_exclusive(s, sh, nullptr) + sums[blockIdx.x];
+    int tot;
+    int ex = block_exclusive(s, sh, &tot) + (sums ? sums[blockIdx.x] : 0);
+    if (!sums && total && threadIdx.x == 0) *total = tot;
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
         if (base + k < count) a[base + k] = ex;
@@ -80,17 +84,33 @@ __global__ void __launch_bounds__(kScanBlock) k_tile_apply(int* a, int count, co
 
 }  // namespace
 
+void scan_in_place(Ctx& ctx, int* data, int count, long long* total) {
+    if (count <= 0) return;
+    cudaStream_t s = ctx.lane.stream;
+    const int nb = ceil_div(count, kScanTile);
+    ProfScope ps(ctx.lane, "setup", 8.0 * count);
+    if (nb == 1) {
+        k_tile_apply<<<1, kScanBlock, 0, s>>>(data, count, nullptr, total);
+        HAMLSS_LAUNCH_CHECK();
+        return;
+    }
+    DBuf<int> sums(nb);
+    DBuf<long long> own;
+    if (!total) {
+        own.alloc(1);
+        total = own.p;
+    }
+    k_tile_sums<<<nb, kScanBlock, 0, s>>>(data, count, sums.p);
+    k_scan_sums<<<1, kScanBlock, 0, s>>>(sums.p, nb, total);
+    k_tile_apply<<<nb, kScanBlock, 0, s>>>(data, count, sums.p, nullptr);
+    HAMLSS_LAUNCH_CHECK();
+}
+
 long long exclusive_scan(Ctx& ctx, int* data, int count) {
     if (count <= 0) return 0;
     cudaStream_t s = ctx.lane.stream;
-    const int nb = ceil_div(count, kScanTile);
-    DBuf<int> sums(nb);
     DBuf<long long> total(1);
-    ProfScope ps(ctx.lane, "setup", 8.0 * count);
-    k_tile_sums<<<nb, kScanBlock, 0, s>>>(data, count, sums.p);
-    k_scan_sums<<<1, kScanBlock, 0, s>>>(sums.p, nb, total.p);
-    k_tile_apply<<<nb, kScanBlock, 0, s>>>(data, count, sums.p);
-    HAMLSS_LAUNCH_CHECK();
+    scan_in_place(ctx, data, count, total.p);
     long long h = 0;
     total.download(&h, 1, s);
     HAMLSS_CUDA(cudaStreamSynchronize(s));
