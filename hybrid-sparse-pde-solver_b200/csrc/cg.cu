@@ -282,7 +282,11 @@ void precond_apply<float>(Ctx& ctx, Prec* M, const float* r, float* z, const int
 }
 
 // ------------------------------------------------------------- persistent iteration
-constexpr int kPersistTrips = 4096;       // trips a launch (state is saved between launches)
+// Trips a launch; the state is saved between launches.  The grid form occupies every SM, so other
+// contexts' kernels wait for its launch to end: 1,024 trips, 6 to 12 ms (a launch and its poll cost
+// some 40 us).  A cluster leaves the rest of the chip to them.
+constexpr int kPersistTripsCluster = 4096;
+constexpr int kPersistTripsGrid = 1024;
 
 // finalisers of k_cg_persist: K1's and K2's (without a preconditioner z = r, so K3's sum
 // arrives with K2's)
@@ -363,7 +367,7 @@ bool persist_fits(Ctx& ctx, hamlss_mat* A) {
     return ok;
 }
 
-// One launch of up to kPersistTrips trips from the state in memory (r, p, x and the
+// One launch of trips from the state in memory (r, p, x and the
 // scalars) back to it.
 template <typename T, bool JAC, typename Fin>
 void launch_persist(Ctx& ctx, hamlss_mat* A, const Csr<T>& Ad, T* x, T* r, T* p, T* z, const T* dinv, CgState* s,
@@ -378,7 +382,7 @@ void launch_persist(Ctx& ctx, hamlss_mat* A, const Csr<T>& Ad, T* x, T* r, T* p,
     PersistArgs<T> a;
     a.n = Ad.n;
     a.rows = A->persist_rows;
-    a.max_trips = kPersistTrips;
+    a.max_trips = A->persist_cluster ? kPersistTripsCluster : kPersistTripsGrid;
     a.rp = Ad.rp;
     a.ci = Ad.ci;
     a.v = Ad.v;
