@@ -41,6 +41,7 @@
 #include <climits>
 
 #include "engine.cuh"
+#include "exact_div.hpp"
 
 namespace hamlss {
 
@@ -93,48 +94,6 @@ __device__ __forceinline__ double sub_mul<double>(double s, double a, double b) 
 template <>
 __device__ __forceinline__ float sub_mul<float>(float s, float a, float b) {
     return __fsub_rn(s, __fmul_rn(a, b));
-}
-
-// s / d given r = 1 / d (rounded; 0 when d is not in [2^-kDivExp, 2^kDivExp]): Markstein's
-// correction (IBM J. Res. Dev. 34, 1990) applied twice.  q0 = s r is within 2 ulp, q1 is a
-// faithful quotient, and for a faithful quotient and a correctly rounded reciprocal
-// q1 + r (s - d q1), with the remainder exact in an FMA, is the correctly rounded one -- s / d
-// bit for bit.  Exponents that could under- or overflow on the way, zeros, infinities and
-// NaN take the division.  On the sweep's critical path: 5 dependent operations (~45 cycles)
-// for the division's ~115.
-template <typename T>
-struct DivRange;
-template <>
-struct DivRange<double> {
-    static constexpr int max_exp = 200;
-    static __device__ __forceinline__ bool safe(double s) {
-        return ((unsigned)__double2hiint(s) >> 20 & 0x7ff) - 400u < 1200u;      // 2^-623 .. 2^577
-    }
-};
-template <>
-struct DivRange<float> {
-    static constexpr int max_exp = 30;
-    static __device__ __forceinline__ bool safe(float s) {
-        return (__float_as_uint(s) >> 23 & 0xff) - 70u < 110u;                  // 2^-57 .. 2^53
-    }
-};
-__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-
-template <typename T>
-__device__ __forceinline__ T recip_of(T d) {
-    const T big = (T)ldexp(1.0, DivRange<T>::max_exp), a = d < T(0) ? -d : d;
-    return a >= T(1) / big && a <= big ? T(1) / d : T(0);
-}
-
-template <typename T>
-__device__ __forceinline__ T div_by(T s, T d, T r) {
-    if (DivRange<T>::safe(s) && r != T(0)) {
-        const T q0 = s * r;
-        const T q1 = fma_rn(fma_rn(-d, q0, s), r, q0);
-        return fma_rn(fma_rn(-d, q1, s), r, q1);
-    }
-    return s / d;
 }
 
 template <typename T, int K, int EXTRA>
