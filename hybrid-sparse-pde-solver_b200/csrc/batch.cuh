@@ -21,7 +21,9 @@
 // it to the end, synchronising on a named barrier of its own.  Systems are grouped in
 // size classes, each with its own team width (the "row-scheduling shape"), processed
 // largest class first and, inside a class, longest system first.  The widths come from a
-// measured autotuner (hamlss_batch_autotune) with an on-disk cache, or defaults.
+// measured autotuner (hamlss_batch_autotune) with an on-disk cache, or defaults; small systems
+// of the first class have narrower teams, and the smallest a launch of their own (batch_group,
+// rules.hpp).
 #pragma once
 
 #include "krylov.cuh"

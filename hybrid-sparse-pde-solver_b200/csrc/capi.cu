@@ -689,6 +689,8 @@ int hamlss_extract_features(hamlss_ctx* ctx, const hamlss_mat* A, double feature
                             int32_t* initial_state) {
     return on_lane(ctx, "a kernel of the feature extraction gave up a bounded wait", [&]() -> int {
         if (!ctx || !A || !features) return set_err(HAMLSS_ERR_INVALID, "null argument");
+        HAMLSS_CUDA(cudaSetDevice(ctx->c.device));
+        AllocScope scope(ctx->c.lane.stream);
         int st = 0;
         int rc = extract_features(ctx->c, const_cast<hamlss_mat*>(A), features, &st);
         if (initial_state) *initial_state = st;

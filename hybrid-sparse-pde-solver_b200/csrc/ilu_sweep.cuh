@@ -35,7 +35,7 @@
 // rows lie before the current step (the step's barrier tells the producer).  Waits on the
 // copies are bounded (~1 s): a thread whose wait ran out sets the lane's error word and only
 // keeps to the barriers from then on; the producer issues no more copies and lets those in
-// flight land, and the host reports HAMLSS_ERR_TIMEOUT.
+// flight land, and the host reports HAMLSS_ERR_TIMEOUT from the call (setup, apply or solve).
 #pragma once
 
 #include <climits>
