@@ -118,7 +118,7 @@ struct BodyScaleV0 {
 // 27.4 / 37.9 / 20.2, against 15.0 / 17.9 / 14.6 and 8.9 / 11.0 / 11.0 here.  Now bound by
 // the vectors' loads from L2 and the sums' latency.
 template <int NV, int MODE, typename Fin>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 k_mdot(int n, int nv, const double* __restrict__ V, long long ld, double* w,
        const double* __restrict__ hprev, Reducer red, Fin fin, const int* gate) {
     constexpr int PER = (NV + 7) / 8;              // vectors a warp
@@ -213,11 +213,11 @@ k_mdot(int n, int nv, const double* __restrict__ V, long long ld, double* w,
 
 // The same with a thread an entry, for few vectors: each entry's chain over the vectors is
 // short then, w is read once instead of by every warp that has a vector, and no warp is without
-// one.  4 M entries, an average of the three modes, this / k_mdot: 1 vector 27 / 45 us, up to 4 41 /
-// 55, up to 8 52 / 62, up to 10 65 / 68, up to 16 102 / 83; 1 M entries 14 / 18, 15 / 19, 18 / 20; 260,000
-// 12.4 / 13.4, 12.8 / 13.7, 14.3 / 13.9; below that the launch is most of either.
+// one.  An average of the three modes, this / k_mdot, us: 4 M entries, 1 vector 24 / 36, up to 4
+// 33 / 44, up to 8 46 / 51; 1 M entries 14 / 16, 15 / 17, 18 / 19; 260,000 no difference.  (Both with
+// four blocks an SM: the finaliser's registers left room for three, of a grid of four.)
 template <int NV, int MODE, typename Fin>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 k_mdot_few(int n, int nv, const double* __restrict__ V, long long ld, double* w,
            const double* __restrict__ hprev, Reducer red, Fin fin, const int* gate) {
     constexpr int NR = MODE == 2 ? 1 : NV;

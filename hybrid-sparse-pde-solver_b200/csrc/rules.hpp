@@ -91,7 +91,7 @@ inline TriMode tri_mode(int n, int nlev, int nnz, int max_row) {
 // ------------------------------------------------------------- FGMRES multi-dots (fgmres.cu)
 // A thread an entry (k_mdot_few) where there are few vectors and enough entries that the loads
 // count: the figures stand at the kernel.
-inline bool mdot_few(int n, int nv) { return nv <= 4 ? n >= (1 << 17) : nv <= 8 && n >= (1 << 19); }
+inline bool mdot_few(int n, int nv) { return nv <= 8 && n >= (1 << 19); }
 
 // ----------------------------------------------------------- dense right operands (amg.cu)
 // Entries of a right operand that an AMG setup holds dense, and of the slots beside it, on a

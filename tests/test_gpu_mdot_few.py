@@ -1,6 +1,6 @@
-"""FGMRES' multi-dots of few vectors at the sizes where a thread an entry takes over (131,072
-entries up to 4 vectors, 524,288 up to 8), both sides of each (-m gpu).  The yardstick and its
-bound are test_gpu_mdot.py's."""
+"""FGMRES' multi-dots of few vectors at the sizes where a thread an entry takes over (524,288
+entries, up to 8 vectors), both sides of each, and below (-m gpu).  The yardstick and its bound
+are test_gpu_mdot.py's."""
 import numpy as np
 import pytest
 

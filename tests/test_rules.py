@@ -100,8 +100,8 @@ def test_sweep_kernel_by_shape(evaluate):
 
 
 def test_multi_dots_of_few_vectors(evaluate):
-    cases = [((131071, 1), 0), ((131072, 1), 1), ((131072, 4), 1), ((131072, 5), 0), ((524287, 8), 0),
-             ((524288, 8), 1), ((4000000, 9), 0), ((1000, 1), 0)]
+    cases = [((524287, 1), 0), ((524287, 8), 0), ((524288, 1), 1), ((524288, 8), 1), ((524288, 9), 0),
+             ((4000000, 9), 0), ((1000, 1), 0)]
     assert evaluate([f"mdot_few({n}, {v})" for (n, v), _ in cases]) == [w for _, w in cases]
 
 
