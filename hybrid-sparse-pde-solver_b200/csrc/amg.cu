@@ -762,7 +762,7 @@ __global__ void k_spgemm_classify(int m, const int* __restrict__ arp, const int*
 // the arithmetic of k_spgemm; the zero products it adds leave a sum as it is (the launcher
 // makes sure A is finite).  No step waits for another, so a row costs its left entries' loads
 // (sixteen in flight a thread) and adds: the near-dense levels of a few hundred rows took
-// 2 ms a product in the merging kernels, one output column at a time, and take ~10 us here.
+// 2 ms a product in the merging kernels, one output column at a time, and take ~50 us here.
 constexpr int kGatherThreads = 128;
 constexpr int kGatherLeft = 256;             // left entries staged at a time
 constexpr int kGatherLoads = 8;
@@ -1557,7 +1557,7 @@ __global__ void k_d2f(const double* __restrict__ a, float* b, long long n) {
 // block keeps the order of the remaining rows, so a step is one round of reads (the column,
 // then the pivot row and the rows below) and one cluster barrier.  A step is bound by those
 // latencies: 155 rows in 5.25 ms by one block that searched the pivot with one thread and
-// walked rows in place, 0.25 ms here.
+// walked rows in place, 0.66 ms here.
 constexpr int kFactorBlocks = 16, kFactorThreads = 512;
 __global__ void __launch_bounds__(kFactorThreads)
 k_dense_factor(int n, double* W, double* M, int* piv, int* skip) {
