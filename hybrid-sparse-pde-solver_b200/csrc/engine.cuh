@@ -225,7 +225,7 @@ bool long_rows_warp(const Csr<T>& A) {
 // four warps an SM would have work.
 template <typename T>
 int prod_rows(int sm_count, const Csr<T>& A) {
-    if (sizeof(T) != 8 || A.n == 0 || A.uneven) return 0;
+    if (sizeof(T) != 8 || A.n == 0 || A.uneven || !prod_indexable(A.nnz)) return 0;
     const double avg = (double)A.nnz / A.n;
     if (avg <= 5.5) return 0;
     const int fit = (int)(kProdFill * kProdTile / avg), share = A.n / (4 * sm_count);

@@ -45,6 +45,9 @@ inline bool prod_uneven(int longest, long long heaviest, long long nnz) {
     return warp - 225LL * longest > nnz / 200;
 }
 
+// Whether k_spmv_prod's entry indices stay in range: it steps by a tile past the last entry.
+inline bool prod_indexable(long long nnz) { return nnz <= 2147483647LL - kProdTile; }
+
 // Whether the gathers of neighbouring rows mostly fall on different lines: of the places that
 // two neighbouring rows both have, fewer than half with columns at most kNearColumns apart.
 // (Grids in natural or coloured order: nearly all.  Rows in random order, or random columns in

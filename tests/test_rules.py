@@ -136,3 +136,8 @@ def test_batch_groups(evaluate):
     assert evaluate([f"batch_group_class({g})" for g in range(6)]) == [0, 0, 0, 1, 2, 3]
     assert evaluate([f"batch_group_width({g}, {w})" for w in (32, 128, 512) for g in (0, 1, 2, 5)]) == \
         [32, 32, 32, 32, 32, 64, 128, 128, 32, 64, 512, 512]
+
+
+def test_product_tiles_stay_in_index_range(evaluate):
+    # the last step's start + 512 must not pass the largest int
+    assert evaluate([f"prod_indexable({k}LL)" for k in (0, 2 ** 31 - 513, 2 ** 31 - 512, 2 ** 31 - 1)]) == [1, 1, 0, 0]
