@@ -120,9 +120,10 @@ inline long long footprint_of(long long n, long long nnz, int m, int max_row) {
     const long long ws = 8 * 8 * n + 8 * 4 * n + (2LL * m + 1) * 8 * n + 64 * 1024;
     const long long ring = 2LL * tri_places(std::min(max_row, kTriMaxRow)) * (8 + 4 + 4 + 4) * n;
     const long long rows = 16 * nnz + 8 * n;
-    const long long ilu = 8 * nnz + std::max(ring, 0LL) + (max_row > 4 ? rows : 0) + 100 * n;
-    const long long amg = 2 * (csr + f32) + 4 * 8 * n + std::min(20 * kGatherDenseLane, 5 * n * n) +
-                          std::min(8LL << 20, 8 * n * n);
+    const long long ilu = 8 * nnz + ring + (max_row > 4 ? rows : 0) + 100 * n;
+    const long long small = std::min(n, 100000LL), square = small * small;      // (larger: the caps)
+    const long long amg = 2 * (csr + f32) + 4 * 8 * n + std::min(20 * kGatherDenseLane, 5 * square) +
+                          std::min(8LL << 20, 8 * square);
     return csr + f32 + 8 * n + ws + std::max(ilu, amg) + (1 << 20);
 }
 

@@ -457,7 +457,8 @@ int hamlss_server_submit(hamlss_server* s, int32_t n, int32_t nnz, const int32_t
     r->x = x;
     if (params) r->p = *params;
     else hamlss_params_default(&r->p);
-    for (int i = 0; i < n; ++i) r->max_row = std::max(r->max_row, row_ptr[i + 1] - row_ptr[i]);
+    for (int i = 0; i < n; ++i)          // (row_ptr is validated on the device: any values here)
+        r->max_row = (int32_t)std::max<int64_t>(r->max_row, std::min<int64_t>((int64_t)row_ptr[i + 1] - row_ptr[i], nnz));
     const int64_t big = hamlss::footprint_of(n, nnz, r->p.restart_size, r->max_row);
     r->small = s->cfg.batch_max_rows > 0 && n <= s->cfg.batch_max_rows;
     if (r->small) {

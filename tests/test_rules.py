@@ -120,6 +120,9 @@ def test_request_footprint(evaluate):
     assert all(g >= h for g, (_, h) in zip(got, held)), got
     flat = 20 * (2 << 20) + (8 << 20)          # what an AMG setup may hold besides, whatever n is
     assert all(g <= 2 * h + flat for g, (_, h) in zip(got, held)), got
+    # any size the interface takes gives a sum in range, growing with it
+    big = evaluate([f"footprint_of({n}LL, {5 * n}LL, 30, 5)" for n in (10 ** 5, 10 ** 6, 10 ** 8, 2 ** 31 - 1)])
+    assert big == sorted(big) and big[0] > 0 and big[3] > 1000 * (2 ** 31 - 1)
     # the batch lane's arrays, counted from their sizes (restart 1 to 32, five entries a row)
     got = evaluate([f"footprint_small(1000, 4900, {m})" for m in (1, 32)])
     for g, m in zip(got, (1, 32)):
